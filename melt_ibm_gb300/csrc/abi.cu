@@ -363,7 +363,7 @@ static uint64_t step_key(Ctx* c) {
     mix(b);
   }
   mix((uint64_t)c->precision); mix((uint64_t)c->nproj); mix(c->lag_gen); mix(c->q32 ? 1 : 0);
-  mix(c->tune_gen); mix(c->diag_on ? 1 : 0);
+  mix(c->tune_gen); mix(c->diag_on ? 1 : 0); mix(c->tri_geo ? 1 : 0);
   return h;
 }
 
@@ -476,7 +476,7 @@ static int autotune(Ctx* c) {
   TuneResult r;
   for (int d = 0; d < 3; ++d) {
     std::vector<int> cand = tri_chunk_candidates(c, d);
-    r.m[d] = tri_chunk(c, d);
+    r.m[d] = tri_chunk_used(c, d);
     r.ms_m[d] = -1.f;
     for (int m : cand) {
       float ms = tri_time_direction(c, d, m, f32, 5);
@@ -933,7 +933,7 @@ int mibm_autotune_(void) {
 
 int mibm_autotune_get_(int* out) {
   Ctx* c = current(); if (!ready(c)) return MIBM_ESTATE;
-  for (int d = 0; d < 3; ++d) out[d] = tri_chunk(c, d);
+  for (int d = 0; d < 3; ++d) out[d] = tri_chunk_used(c, d);
   out[3] = c->tune_by;
   return MIBM_OK;
 }

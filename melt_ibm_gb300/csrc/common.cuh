@@ -200,6 +200,7 @@ struct Ctx {
   bool profiling = false;                 // per-kernel event profiling on (no graphs then)
   // shapes chosen by the autotuner (tune.cu); -1 / 8 = the default rules
   int tune_m[3] = {-1, -1, -1};           // line-solve chunk length per direction
+  bool tri_geo = false;                   // FP64 step: every line solve takes the geo_* kernels (tridiag.cu)
   int tune_by = 2;                        // block height of the explicit-term kernels (32 x 2 threads: the
                                           // autotuner's choice at 48^3, 128^3 and 256^3)
   uint64_t tune_gen = 0;
@@ -356,7 +357,8 @@ void hit_free(Ctx* c);
 // autotuner support (tridiag.cu, stencil.cu)
 float tri_time_direction(Ctx* c, int dir, int m, bool f32, int reps);
 std::vector<int> tri_chunk_candidates(Ctx* c, int dir);
-int tri_chunk(Ctx* c, int dir);
+int tri_chunk_used(Ctx* c, int dir);
+bool tri_keep_order(Ctx* c);
 float stencil_time_by(Ctx* c, const StepParams* dp, int by, int reps);
 // restart regrid (interp.cu): host arrays in, host array out
 void k_interp_restart(Ctx* c, double* arrold, double* arrnew, int n1o, int n2o, int n3o, int intvar, int kstarto,

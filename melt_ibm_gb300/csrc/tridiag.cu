@@ -15,7 +15,28 @@
 //             x_i = x_n s_i + f_i
 // = 4 FP64 operations per element, one read and one write of the line.
 //
-// Main path (chunked solves): a line of n cells is cut into G chunks of M
+// FP64 lines (geo_* kernels): the system is circulant, so it factors exactly
+// into two first-order recurrences with one constant,
+//   (1+2G) - G (S + S^-1) = (G/rho) (1 - rho S^-1) (1 - rho S),
+//   rho = 2G / (1 + 2G + sqrt(1 + 4G)),  rho/G = (1 - rho)^2:
+//   y_i = r_i + rho y_{i-1},  x_i = y_i + rho x_{i+1},  scaled by (1-rho)^2,
+// 2 FP64 operations per element instead of the Thomas sweep's 4, with no
+// factor tables to read.  A line of n cells is cut into G chunks of M cells,
+// one thread each; a chunk sweeps from a zero entry and adds rho^{i+1} y_in
+// afterwards, y_in = sum_m rho^{mM} C_{h-1-m} / (1 - rho^n) over the end
+// values C of the chunks before it (periodic: the closure is the wrap of
+// that index).  Powers of rho below 2^-60 are dropped: of the fix-up only the
+// first F cells of a chunk and of the sum only K terms remain, F = 5..10 and
+// K = 1 at the time steps the CFL condition allows (rho = 3e-4 .. 2e-2); with
+// F = M and K = G the same kernel solves any G > -1/4.  The x and y solves of
+// a step leave their scale to the z solve, whose addition into the field
+// becomes an FMA.  Against 80-bit solutions the error is at the rounding of
+// the result at every G from 1e-6 to 1e5 (1e-16 .. 1e-14 relative); the Thomas
+// sweep is there up to G = 2 and loses accuracy above (1e-15 at 6.5, 5e-15 at
+// 40, 4e-12 at 1e5), as its closure cancels.
+//
+// Chunked Thomas solves (FP32, and FP64 where tri_keep_order says why the
+// order is kept): a line of n cells is cut into G chunks of M
 // cells and each thread keeps one chunk in registers.  The two recurrences
 // are linear, so a chunk runs them from a zero entry value and corrects
 // afterwards with its true entry value times a factor that depends on the
@@ -37,6 +58,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -124,7 +146,11 @@ void tri_build_table(int n, double betadx, std::vector<double>& t) { build_table
 
 static size_t slot_len(int nmax);
 static void fill_slot(int n, int m, double betadx, double* out);
+static void fill_geo(int n, int m, double betadx, double scale, double* out);
+static bool geo_ok(double betadx);
+static double geo_scale(double betadx);
 int tri_chunk(Ctx* c, int dir);
+static int geo_chunk(Ctx* c, int dir);
 
 // Device table cache: small ring of slots, refilled when (n, betadx) changes.
 struct TriCache {
@@ -149,12 +175,14 @@ static CtxTri* tri_of(Ctx* c) {
   return t;
 }
 
-// Returns a device pointer to the table of (n, betadx).  The table is
-// written to a pinned slot and copied on the context stream, so the value is
-// stream-ordered with the solve that uses it.
-static const double* table_for(Ctx* c, int dir, double betadx) {
+// Returns a device pointer to the FP64 table of (n, betadx) for the drop-in
+// solves (geo: the constants of the geo_* kernels, each direction with its own
+// scale; else the Thomas factors).  The table is written to a pinned slot and
+// copied on the context stream, so the value is stream-ordered with the solve
+// that uses it.
+static const double* table_for(Ctx* c, int dir, double betadx, bool geo) {
   const int n = dir == 0 ? c->g.n1m : (dir == 1 ? c->g.n2m : c->g.n3m);
-  const int m = tri_chunk(c, dir);
+  const int m = geo ? -geo_chunk(c, dir) : tri_chunk(c, dir);     // the cache key of the slot
   TriCache& tc = tri_of(c)->cache;
   int nmax = std::max(c->g.n1m, c->g.n3m);
   if (!tc.dev) {
@@ -163,7 +191,7 @@ static const double* table_for(Ctx* c, int dir, double betadx) {
     if (!cuda_ok(c, cudaMalloc(&tc.dev, sizeof(double) * tc.len * tc.slots), "tri table")) return nullptr;
     if (!cuda_ok(c, cudaMallocHost(&tc.pinned, sizeof(double) * tc.len * tc.slots), "tri table")) return nullptr;
     tc.n.assign(tc.slots, -1);
-    tc.m.assign(tc.slots, -1);
+    tc.m.assign(tc.slots, 0);
     tc.bd.assign(tc.slots, -1.0);
   }
   for (int s = 0; s < tc.slots; ++s)
@@ -172,7 +200,8 @@ static const double* table_for(Ctx* c, int dir, double betadx) {
   tc.next = (tc.next + 1) % tc.slots;
   // a slot may still be read by an in-flight kernel: order the refill on the stream
   cudaStreamSynchronize(c->stream);
-  fill_slot(n, m, betadx, tc.pinned + (size_t)s * tc.len);
+  if (geo) fill_geo(n, -m, betadx, geo_scale(betadx), tc.pinned + (size_t)s * tc.len);
+  else fill_slot(n, m, betadx, tc.pinned + (size_t)s * tc.len);
   cudaMemcpyAsync(tc.dev + (size_t)s * tc.len, tc.pinned + (size_t)s * tc.len, sizeof(double) * tc.len,
                   cudaMemcpyHostToDevice, c->stream);
   tc.n[s] = n;
@@ -373,6 +402,15 @@ static bool chunk_ok(int m) {
   return false;
 }
 
+// chunk lengths of the geo_* kernels
+static const int kGeoM[] = {2, 3, 4, 6, 8, 12, 16, 18, 24, 32};
+
+static bool geo_chunk_ok(int m) {
+  for (int v : kGeoM)
+    if (v == m) return true;
+  return false;
+}
+
 // lanes a line occupies in the x-line kernel: G = n/M rounded up to a power
 // of two (shuffle segments); a warp solves 32/that lines
 __host__ __device__ constexpr int line_lanes(int G) {
@@ -401,6 +439,8 @@ int tri_chunk_line(int n) {
   }
   return best_wide ? best_wide : best;
 }
+
+constexpr int kGeoRowThreads = 128;   // threads of a geo_x_kernel block
 
 // y/z blocks: up to 32 chunks (warps) of M <= 8 cells, or 16 chunks of the
 // longer M (register budget of a 1024- or 512-thread block)
@@ -525,27 +565,115 @@ static TriLayout tri_layout(int n, int m) {
   return L;
 }
 
-static bool chunk_feasible(int n, int m, bool line) {
-  if (!chunk_ok(m) || n % m != 0) return false;
+static bool chunk_feasible(int n, int m, bool line, bool geo) {
+  if (!(geo ? geo_chunk_ok(m) : chunk_ok(m)) || n % m != 0) return false;
   return line ? n / m <= 32 : n / m <= col_max_chunks(m);
 }
+
+static int line_len(Ctx* c, int dir) { return dir == 0 ? c->g.n1m : (dir == 1 ? c->g.n2m : c->g.n3m); }
 
 // chunk length of direction dir (0 x, 1 y, 2 z) for context c: the
 // autotuner's choice when one is set and feasible, else the default rule
 int tri_chunk(Ctx* c, int dir) {
-  const int n = dir == 0 ? c->g.n1m : (dir == 1 ? c->g.n2m : c->g.n3m);
-  int m = c->tune_m[dir];
-  if (m > 0 && chunk_feasible(n, m, dir == 0)) return m;
+  const int n = line_len(c, dir), m = c->tune_m[dir];
+  if (m > 0 && chunk_feasible(n, m, dir == 0, false)) return m;
   return dir == 0 ? tri_chunk_line(n) : tri_chunk_col(n);
 }
 
-// candidate chunk lengths of direction dir (for the autotuner)
+// geo_* chunks: a chunk costs 2 M + 2 F operations with F independent of M, so
+// long ones do least, as long as there are threads enough.  y/z: 24 before 32
+// before 16, at least four chunks (measured y / z us per solve, u, v, w and T
+// averaged: 192^3 24: 87 / 115, 16: 91 / 118, 32: 95 / 121; 256^3 32: 201 / 246,
+// 16: 202 / 262; 96^3 24: 17 / 21, 16: 18.4 / 22; within 5% at 48-64).
+// x: 16 (256^3 196, 32: 221; 128^3 35, 8: 42, 32: 44), but 8 or 6 where 16 leaves
+// fewer than 100 blocks for a field (48^3 10.8 against 12.9); odd ones last,
+// they load 8 bytes at a time.
+static int geo_chunk_line(int n, int lines) {
+  static const int pref[] = {16, 12, 8, 6, 4, 2, 3};
+  int found = 0;
+  for (int m : pref) {
+    if (n % m != 0 || n / m > 32) continue;
+    if (m > 8 || !found) found = found ? found : m;
+    if ((size_t)lines * (n / found) >= 100 * kGeoRowThreads) return found;
+    if (m <= 8) return m;
+  }
+  return found;
+}
+static int geo_chunk_col(int n) {
+  static const int pref[] = {24, 32, 16, 18, 12, 8, 6, 4, 3, 2};
+  for (int m : pref)
+    if (n % m == 0 && n / m >= 4 && n / m <= col_max_chunks(m)) return m;
+  return 0;
+}
+
+// the same for the geo_* kernels (0: none)
+static int geo_chunk(Ctx* c, int dir) {
+  const int n = line_len(c, dir), m = c->tune_m[dir];
+  if (m > 0 && chunk_feasible(n, m, dir == 0, true)) return m;
+  return dir == 0 ? geo_chunk_line(n, c->g.n2m * c->g.n3m) : geo_chunk_col(n);
+}
+
+// Whether the FP64 step of context c keeps the Thomas sweep's order of
+// operations.  The literal MLS of a body that melts without moving turns a
+// last-bit difference of a vertex coordinate into about 1e-8 of the heat flux
+// on fine grids (the condition number of its moment matrix grows as (n/L)^2),
+// and the front integrates it: after 9 steps from identical inputs another
+// order of the line solves alone moves the pressure at single cells by 1e-9
+// (96^3), 6e-9 (144^3), 1e-8 (192^3) and 1.5e-7 (256^3) of its rms.  Fine grids
+// therefore keep it, so that their runs reproduce those of earlier builds.
+constexpr int kOrderCells = 160;
+bool tri_keep_order(Ctx* c) {
+  return c->I(MIBM_I_IMLSFOR) == 1 && c->I(MIBM_I_IMELT) == 1 && c->I(MIBM_I_IMLSSTR) != 1 && c->maxnf > 0 &&
+         std::max(c->g.n1m, c->g.n3m) > kOrderCells;
+}
+
+// chunk length in use by the form the context runs
+int tri_chunk_used(Ctx* c, int dir) {
+  const int m = c->precision == 0 && !tri_keep_order(c) ? geo_chunk(c, dir) : 0;
+  return m ? m : tri_chunk(c, dir);
+}
+
+// candidate chunk lengths of direction dir for that form (for the autotuner)
 std::vector<int> tri_chunk_candidates(Ctx* c, int dir) {
-  const int n = dir == 0 ? c->g.n1m : (dir == 1 ? c->g.n2m : c->g.n3m);
+  const bool geo = c->precision == 0 && !tri_keep_order(c);
   std::vector<int> out;
-  for (int m : kChunkM)
-    if (chunk_feasible(n, m, dir == 0)) out.push_back(m);
+  for (int m : kGeoM)
+    if (chunk_feasible(line_len(c, dir), m, dir == 0, geo)) out.push_back(m);
   return out;
+}
+
+// Constants of the geo_* kernels for (n, M, G = betadx): rho, the scale the
+// kernel applies, F and K (see the top of the file; the thresholds drop
+// relative 2^-60), then rho^(i+1) for i < M and rho^(mM) / (1 - rho^n) for
+// m < n/M.  The powers are formed in extended precision from the rounded rho,
+// so that every path round the line uses the same constant.
+constexpr int kGeoPow = 4;                     // offsets within the slot
+constexpr int kGeoMul = kGeoPow + 32;
+constexpr int kGeoLen = kGeoMul + 32;
+static bool geo_ok(double betadx) { return betadx > -0.24 && betadx < 1e12; }
+static double geo_rho(double betadx) {
+  return 2.0 * betadx / (1.0 + 2.0 * betadx + std::sqrt(1.0 + 4.0 * betadx));
+}
+static double geo_scale(double betadx) {
+  const double d = 1.0 - geo_rho(betadx);
+  return d * d;
+}
+static void fill_geo(int n, int m, double betadx, double scale, double* out) {
+  const int G = n / m;
+  const double rho = geo_rho(betadx);
+  const double bits = rho == 0.0 ? 1e9 : -std::log2(std::fabs(rho));    // per cell
+  out[0] = rho;
+  out[1] = scale;
+  out[2] = (double)std::min((double)m, std::ceil(60.0 / bits));
+  out[3] = (double)std::min((double)G, std::ceil(60.0 / (bits * m)));
+  long double p = 1.0L, rn = 1.0L;
+  for (int i = 0; i < m; ++i) { p *= (long double)rho; out[kGeoPow + i] = (double)p; }
+  for (int h = 0; h < G; ++h) rn *= p;
+  p = 1.0L / (1.0L - rn);
+  for (int h = 0; h < G; ++h) {
+    out[kGeoMul + h] = (double)p;
+    for (int i = 0; i < m; ++i) p *= (long double)rho;
+  }
 }
 
 // fills one slot (base + the extended table of chunk m) for (n, betadx)
@@ -788,6 +916,197 @@ __global__ void __launch_bounds__(32 * col_max_chunks(M)) solve_cc_kernel(Grid g
 }
 
 // ---------------------------------------------------------------------
+// FP64 lines (constants T of fill_geo; the method is at the top of the file)
+// ---------------------------------------------------------------------
+// entry value of chunk h from the end values E of the chunks before it
+// (dir = -1) or the start values of those after it (dir = +1), K terms
+template <typename Ends>
+__device__ __forceinline__ double geo_entry(const double* __restrict__ T, int K, int G, int h, int dir, Ends E) {
+  double v = 0.0;
+  int src = h;
+  for (int m = 0; m < K; ++m) {
+    src += dir;
+    src = src < 0 ? G - 1 : (src == G ? 0 : src);
+    v = T[kGeoMul + m] * E(src) + v;
+  }
+  return v;
+}
+// r[first + d*i] += rho^(i+1) v for the F cells the entry value still reaches
+template <int M, bool FWD>
+__device__ __forceinline__ void geo_fix(const double* __restrict__ T, int F, double v, double (&r)[M]) {
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    if (i % 2 == 0 && i >= F) break;               // uniform over the grid
+    double& e = r[FWD ? i : M - 1 - i];
+    e = T[kGeoPow + i] * v + e;
+  }
+}
+
+// x-lines: a block holds as many rows as its threads have chunks (thread t:
+// chunk t % G of row t / G), staged through shared memory so that global
+// loads and stores are whole rows; chunk h of a row starts at h * CS, CS = M + 2
+// for M = 0 mod 4, which spreads the 16-byte reads of eight lanes over all banks.
+// Bound by the FP64 pipe (2 + 2F/M operations per element): 256^3, mean of the
+// u, v, w launch and the T launch, 196 us against 357 us with the Thomas
+// factors (five operations per element and shuffle scans); 128^3 35 against 60.
+__host__ __device__ constexpr int geo_cs(int m) { return m % 2 ? m : (m % 4 == 2 ? m : m + 2); }
+template <int M, bool SCALE>
+__global__ void __launch_bounds__(kGeoRowThreads) geo_x_kernel(Grid g, double* __restrict__ rhs,
+                                                               const double* __restrict__ T, int nfield,
+                                                               unsigned magic) {
+  extern __shared__ __align__(16) double geo_sm[];
+  __shared__ double sC[kGeoRowThreads], sD[kGeoRowThreads];
+  constexpr int CS = geo_cs(M), V = M % 2 ? 1 : 2;
+  const int n = g.n1m, G = n / M, R = kGeoRowThreads / G, RS = G * CS;
+  const int per = g.n2m * g.n3m, lines = per * nfield, row0 = blockIdx.x * R;
+  const int nv = n / V;
+  auto row_ptr = [&](int r) {
+    const int line = row0 + r, f = line / per, l = line - f * per;
+    return rhs + (size_t)f * g.cells + cidx(g, 0, l % g.n2m, l / g.n2m);
+  };
+  const int rows = min(R, lines - row0), total = rows * nv;
+  // the block's rows as one run of V-wide pieces, eight of a thread in flight;
+  // piece / nv as a multiply by magic = 2^32 / nv rounded up (exact below 2^16)
+  auto move = [&](auto body) {
+    for (int p0 = threadIdx.x; p0 < total; p0 += 8 * kGeoRowThreads) body(p0);
+  };
+  auto piece = [&](int p, double*& at_g, int& at_s) {
+    const int r = (int)__umulhi((unsigned)p, magic), e = (p - r * nv) * V;
+    at_g = row_ptr(r) + e;
+    at_s = r * RS + (e / M) * CS + e % M;
+    return MIBM_IDX_OK((size_t)(at_g - rhs) % g.cells + V - 1, g.cells);
+  };
+  typedef typename std::conditional<V == 2, double2, double>::type Vec;
+  move([&](int p0) {
+    Vec t[8];
+    int at[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int p = p0 + u * kGeoRowThreads;
+      double* src;
+      at[u] = -1;
+      if (p < total && piece(p, src, at[u])) t[u] = *reinterpret_cast<const Vec*>(src);
+      else at[u] = -1;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (at[u] >= 0) *reinterpret_cast<Vec*>(geo_sm + at[u]) = t[u];
+  });
+  __syncthreads();
+  const int row = threadIdx.x / G, h = threadIdx.x - row * G;
+  const bool act = row < rows;
+  const double rho = T[0], scale = T[1];
+  const int F = (int)T[2], K = (int)T[3];
+  double* mine = geo_sm + (act ? row * RS + h * CS : 0);
+  double r[M];
+#pragma unroll
+  for (int i = 0; i < M / V; ++i) {
+    if constexpr (V == 2) {
+      const double2 t = reinterpret_cast<const double2*>(mine)[i];
+      r[2 * i] = t.x; r[2 * i + 1] = t.y;
+    } else {
+      r[i] = mine[i];
+    }
+  }
+#pragma unroll
+  for (int i = 1; i < M; ++i) r[i] = rho * r[i - 1] + r[i];
+  sC[threadIdx.x] = r[M - 1];
+  __syncthreads();
+  const int seg = act ? row * G : 0;
+  const double y_in = geo_entry(T, K, G, h, -1, [&](int s) { return sC[seg + s]; });
+  geo_fix<M, true>(T, F, y_in, r);
+#pragma unroll
+  for (int i = M - 2; i >= 0; --i) r[i] = rho * r[i + 1] + r[i];
+  sD[threadIdx.x] = r[0];
+  __syncthreads();
+  const double x_in = geo_entry(T, K, G, h, 1, [&](int s) { return sD[seg + s]; });
+  geo_fix<M, false>(T, F, x_in, r);
+  if (act) {
+#pragma unroll
+    for (int i = 0; i < M / V; ++i) {
+      if constexpr (V == 2) {
+        double2 t = make_double2(r[2 * i], r[2 * i + 1]);
+        if (SCALE) { t.x *= scale; t.y *= scale; }
+        reinterpret_cast<double2*>(mine)[i] = t;
+      } else {
+        mine[i] = SCALE ? r[i] * scale : r[i];
+      }
+    }
+  }
+  __syncthreads();
+  move([&](int p0) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int p = p0 + u * kGeoRowThreads;
+      double* dst;
+      int at;
+      if (p < total && piece(p, dst, at)) *reinterpret_cast<Vec*>(dst) = *reinterpret_cast<const Vec*>(geo_sm + at);
+    }
+  });
+}
+
+// y- and z-lines: block = 32 adjacent i (lanes) x G chunks (warps) of one
+// plane k (y-lines) or one row j (z-lines); a z solve adds scale * x to q
+// (solxk.f90:44-50), with write_rhs also leaving scale * x in rhs.
+// The field is read after the solve, in batches, rather than held in registers
+// beside the line: that leaves room for the other blocks of the SM (256^3, z:
+// 246 against 290 us).  FP64-bound: 256^3 y 385 -> 201 us, z 497 -> 246 us per
+// solve (mean of the u, v, w and the T launch); 128^3 54 -> 33 and 71 -> 39 us.
+template <int M, bool ZL, bool SCALE>
+__global__ void __launch_bounds__(32 * col_max_chunks(M), M == 16 ? 2 : 1) geo_col_kernel(Grid g, double* __restrict__ rhs_base,
+                                                                         const double* __restrict__ T, QSet qs,
+                                                                         int write_rhs) {
+  __shared__ double sC[kColMaxChunks][32];
+  __shared__ double sD[kColMaxChunks][32];
+  const int n = ZL ? g.n3m : g.n2m, G = n / M;
+  const int lane = threadIdx.x, w = threadIdx.y;
+  const int x = blockIdx.x * 32 + lane;
+  const bool act0 = x < g.n1m;
+  const int planes = ZL ? g.n2m : g.n3m;
+  const int f = blockIdx.y / planes, pl = blockIdx.y - f * planes;
+  const int stride = ZL ? (int)g.plane : g.P;
+  const size_t first = (ZL ? cidx(g, act0 ? x : 0, pl, 0) : cidx(g, act0 ? x : 0, 0, pl)) + (size_t)(w * M) * stride;
+  double* __restrict__ rp = rhs_base + (size_t)f * g.cells + first;
+  const bool act = act0 && MIBM_IDX_OK(first + (size_t)(M - 1) * stride, g.cells);
+  double r[M];
+#pragma unroll
+  for (int i = 0; i < M; ++i) r[i] = act ? rp[i * stride] : 0.0;
+  const double rho = T[0], scale = T[1];
+  const int F = (int)T[2], K = (int)T[3];
+#pragma unroll
+  for (int i = 1; i < M; ++i) r[i] = rho * r[i - 1] + r[i];
+  sC[w][lane] = r[M - 1];
+  __syncthreads();
+  const double y_in = geo_entry(T, K, G, w, -1, [&](int s) { return sC[s][lane]; });
+  geo_fix<M, true>(T, F, y_in, r);
+#pragma unroll
+  for (int i = M - 2; i >= 0; --i) r[i] = rho * r[i + 1] + r[i];
+  sD[w][lane] = r[0];
+  __syncthreads();
+  const double x_in = geo_entry(T, K, G, w, 1, [&](int s) { return sD[s][lane]; });
+  geo_fix<M, false>(T, F, x_in, r);
+  if (!act) return;
+  if constexpr (ZL) {
+    double* __restrict__ qp = (f == 0 ? qs.p[0] : (f == 1 ? qs.p[1] : qs.p[2])) + first;
+    constexpr int B = M % 8 == 0 ? 8 : (M % 6 == 0 ? 6 : M);
+#pragma unroll
+    for (int i0 = 0; i0 < M; i0 += B) {
+      double qb[B];
+#pragma unroll
+      for (int u = 0; u < B; ++u) qb[u] = qp[(i0 + u) * stride];
+#pragma unroll
+      for (int u = 0; u < B; ++u) {
+        if (write_rhs) rp[(i0 + u) * stride] = scale * r[i0 + u];
+        qp[(i0 + u) * stride] = scale * r[i0 + u] + qb[u];
+      }
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < M; ++i) rp[i * stride] = SCALE ? scale * r[i] : r[i];
+  }
+}
+
+// ---------------------------------------------------------------------
 // y- and z-lines in FP32 with the lines staged by bulk tensor copies
 // ---------------------------------------------------------------------
 // The same arithmetic as solve_cc_kernel<float, M, ZL>, bit for bit, in a
@@ -962,20 +1281,38 @@ static StepTables* steptab_of(Ctx* c) {
 bool tri_step_fill(Ctx* c, const double betadx[3][2][3], bool f32) {
   StepTables* st = steptab_of(c);
   int nmax = std::max(c->g.n1m, c->g.n3m);
+  const size_t cap = slot_len(nmax);
   if (!st->dev) {
-    st->len = (int)slot_len(nmax);
-    size_t bytes = sizeof(double) * 18 * (size_t)st->len;
+    size_t bytes = sizeof(double) * 18 * cap;
     if (!cuda_ok(c, cudaMalloc(&st->dev, bytes), "step tables")) return false;
     if (!cuda_ok(c, cudaMalloc(&st->devf, bytes / 2), "step tables")) return false;
     if (!cuda_ok(c, cudaMallocHost(&st->pinned, bytes + bytes / 2), "step tables")) return false;
   }
   const int n[3] = {c->g.n1m, c->g.n2m, c->g.n3m};
+  c->tri_geo = !f32 && !tri_keep_order(c);
+  for (int d = 0; d < 3; ++d) c->tri_geo = c->tri_geo && geo_chunk(c, d) != 0;
+  for (int ns = 0; ns < 3; ++ns)
+    for (int f = 0; f < 2; ++f)
+      for (int d = 0; d < 3; ++d) c->tri_geo = c->tri_geo && geo_ok(betadx[ns][f][d]);
+  st->len = (int)(c->tri_geo ? kGeoLen : cap);
+  if (c->tri_geo) {     // the three directions' scales meet in the z solve
+    for (int ns = 0; ns < 3; ++ns)
+      for (int f = 0; f < 2; ++f) {
+        double scale = 1.0;
+        for (int d = 0; d < 3; ++d) {
+          scale *= geo_scale(betadx[ns][f][d]);
+          fill_geo(n[d], geo_chunk(c, d), betadx[ns][f][d], scale,
+                   st->pinned + (size_t)((ns * 2 + f) * 3 + d) * st->len);
+        }
+      }
+    return true;
+  }
   for (int ns = 0; ns < 3; ++ns)
     for (int f = 0; f < 2; ++f)
       for (int d = 0; d < 3; ++d)
         fill_slot(n[d], tri_chunk(c, d), betadx[ns][f][d], st->pinned + (size_t)((ns * 2 + f) * 3 + d) * st->len);
   if (f32) {
-    float* hf = (float*)(st->pinned + 18 * (size_t)st->len);
+    float* hf = (float*)(st->pinned + 18 * cap);
     for (size_t q = 0; q < 18 * (size_t)st->len; ++q) hf[q] = (float)st->pinned[q];
   }
   return true;
@@ -986,7 +1323,7 @@ const double* tri_step_enqueue(Ctx* c, bool f32, int* len_out, const float** f32
   StepTables* st = steptab_of(c);
   if (!st->dev) return nullptr;
   if (f32) {
-    float* hf = (float*)(st->pinned + 18 * (size_t)st->len);
+    float* hf = (float*)(st->pinned + 18 * slot_len(std::max(c->g.n1m, c->g.n3m)));
     cudaMemcpyAsync(st->devf, hf, sizeof(float) * 18 * (size_t)st->len, cudaMemcpyHostToDevice, c->stream);
     if (f32_out) *f32_out = st->devf;
   } else {
@@ -1014,6 +1351,14 @@ static bool smem_ok(Ctx* c, const void* fn, size_t bytes) {
     return cuda_ok(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "smem attr");
   return true;
 }
+
+#define MIBM_GEO_CASES(M_, CALL) \
+  switch (M_) {                       \
+    case 18: CALL(18); break;         \
+    case 24: CALL(24); break;         \
+    case 32: CALL(32); break;         \
+    default: MIBM_CHUNK_CASES(M_, CALL) \
+  }
 
 #define MIBM_CHUNK_CASES(M_, CALL) \
   switch (M_) {                       \
@@ -1210,6 +1555,49 @@ static void solve_z_launch(Ctx* c, V* rhs, const V* T, const QSet& q, int nfield
   MIBM_LAUNCH_CHECK(c, name);
 }
 
+// The geo_* solves; own_scale: x and y lines apply their own scale
+// (drop-in solves), else the z solve's constants hold the product of the three
+static bool geo_x_launch(Ctx* c, double* rhs, const double* T, int nfield, bool own_scale) {
+  const int m = geo_chunk(c, 0);
+  if (!m) return false;
+  const int G = c->g.n1m / m, R = kGeoRowThreads / G;
+  const size_t sm = (size_t)R * G * geo_cs(m) * sizeof(double);
+  const unsigned blocks = div_up((size_t)c->g.n2m * c->g.n3m * nfield, R);
+  {
+    MIBM_PROF(c, "solve_x");
+    const unsigned nv = c->g.n1m / (m % 2 ? 1 : 2), magic = (unsigned)((0x100000000ull + nv - 1) / nv);
+#define GX(M)                                                                                                 \
+  if (own_scale) geo_x_kernel<M, true><<<blocks, kGeoRowThreads, sm, c->stream>>>(c->g, rhs, T, nfield, magic); \
+  else geo_x_kernel<M, false><<<blocks, kGeoRowThreads, sm, c->stream>>>(c->g, rhs, T, nfield, magic)
+    MIBM_GEO_CASES(m, GX)
+#undef GX
+  }
+  ++c->launches;
+  MIBM_LAUNCH_CHECK(c, "solve_x");
+  return true;
+}
+
+template <bool ZL>
+static bool geo_col_launch(Ctx* c, double* rhs, const double* T, const QSet& q, int nfield, int write_rhs,
+                           bool own_scale) {
+  const int n = ZL ? c->g.n3m : c->g.n2m, m = geo_chunk(c, ZL ? 2 : 1);
+  if (!m) return false;
+  const char* name = ZL ? "solve_z" : "solve_y";
+  dim3 block(32, n / m);
+  dim3 grid(div_up(c->g.n1m, 32), (ZL ? c->g.n2m : c->g.n3m) * nfield);
+  {
+    MIBM_PROF(c, name);
+#define GC(M)                                                                                                  \
+  if (own_scale || ZL) geo_col_kernel<M, ZL, true><<<grid, block, 0, c->stream>>>(c->g, rhs, T, q, write_rhs); \
+  else geo_col_kernel<M, false, false><<<grid, block, 0, c->stream>>>(c->g, rhs, T, q, write_rhs)
+    MIBM_GEO_CASES(m, GC)
+#undef GC
+  }
+  ++c->launches;
+  MIBM_LAUNCH_CHECK(c, name);
+  return true;
+}
+
 static QSet qset(double* const* q, int nfield) {
   QSet s{};
   for (int f = 0; f < nfield && f < 3; ++f) s.p[f] = q[f];
@@ -1217,13 +1605,15 @@ static QSet qset(double* const* q, int nfield) {
 }
 
 void k_solve_x_T(Ctx* c, double* rhs, const double* T, int nfield) {
-  solve_x_launch<double>(c, rhs, T, "solve_x", nfield);
+  if (!c->tri_geo || !geo_x_launch(c, rhs, T, nfield, false)) solve_x_launch<double>(c, rhs, T, "solve_x", nfield);
 }
 void k_solve_y_T(Ctx* c, double* rhs, const double* T, int nfield) {
-  solve_y_launch<double>(c, rhs, T, "solve_y", nfield);
+  if (!c->tri_geo || !geo_col_launch<false>(c, rhs, T, QSet{}, nfield, 0, false))
+    solve_y_launch<double>(c, rhs, T, "solve_y", nfield);
 }
 void k_solve_z_T(Ctx* c, double* rhs, const double* T, double* const* q, int nfield, int write_rhs) {
-  solve_z_launch<double>(c, rhs, T, qset(q, nfield), nfield, write_rhs, nullptr, "solve_z");
+  if (!c->tri_geo || !geo_col_launch<true>(c, rhs, T, qset(q, nfield), nfield, write_rhs, true))
+    solve_z_launch<double>(c, rhs, T, qset(q, nfield), nfield, write_rhs, nullptr, "solve_z");
 }
 void k_solve_x_f32(Ctx* c, float* rhs, const float* T, int nfield) {
   solve_x_launch<float>(c, rhs, T, "solve_x_f32", nfield);
@@ -1235,19 +1625,29 @@ void k_solve_z_f32(Ctx* c, float* rhs, const float* T, double* const* q, int nfi
   solve_z_launch<float>(c, rhs, T, qset(q, nfield), nfield, 0, mirror, "solve_z_f32");
 }
 
+// the drop-in solves: the geo_* kernels wherever they cover the system
 void k_solve_x(Ctx* c, double* rhs, double betadx) {
-  const double* T = table_for(c, 0, betadx);
-  if (T) k_solve_x_T(c, rhs, T, 1);
+  const bool geo = geo_ok(betadx) && geo_chunk(c, 0);
+  const double* T = table_for(c, 0, betadx, geo);
+  if (!T) return;
+  if (geo) geo_x_launch(c, rhs, T, 1, true);
+  else solve_x_launch<double>(c, rhs, T, "solve_x", 1);
 }
 
 void k_solve_y(Ctx* c, double* rhs, double betadx) {
-  const double* T = table_for(c, 1, betadx);
-  if (T) k_solve_y_T(c, rhs, T, 1);
+  const bool geo = geo_ok(betadx) && geo_chunk(c, 1);
+  const double* T = table_for(c, 1, betadx, geo);
+  if (!T) return;
+  if (geo) geo_col_launch<false>(c, rhs, T, QSet{}, 1, 0, true);
+  else solve_y_launch<double>(c, rhs, T, "solve_y", 1);
 }
 
 void k_solve_z(Ctx* c, double* rhs, double betadx, double* q) {
-  const double* T = table_for(c, 2, betadx);
-  if (T) k_solve_z_T(c, rhs, T, &q, 1, 1);
+  const bool geo = geo_ok(betadx) && geo_chunk(c, 2);
+  const double* T = table_for(c, 2, betadx, geo);
+  if (!T) return;
+  if (geo) geo_col_launch<true>(c, rhs, T, qset(&q, 1), 1, 1, true);
+  else solve_z_launch<double>(c, rhs, T, qset(&q, 1), 1, 1, nullptr, "solve_z");
 }
 
 // ---------------------------------------------------------------------
@@ -1260,7 +1660,10 @@ float tri_time_direction(Ctx* c, int dir, int m, bool f32, int reps) {
   const int saved = c->tune_m[dir];
   c->tune_m[dir] = m;
   std::vector<double> slot(slot_len(std::max(c->g.n1m, c->g.n3m)), 0.0);
-  fill_slot(n, m, 0.9, slot.data());
+  // (the geo_* kernels' cost depends on betadx: a value of the steps' range)
+  const bool geo = !f32 && !tri_keep_order(c) && geo_chunk(c, dir) == m;
+  if (geo) fill_geo(n, m, 0.01, geo_scale(0.01), slot.data());
+  else fill_slot(n, m, 0.9, slot.data());
   std::vector<float> slotf(slot.begin(), slot.end());
   void* tab = nullptr;
   void* rhs = nullptr;
@@ -1287,7 +1690,10 @@ float tri_time_direction(Ctx* c, int dir, int m, bool f32, int reps) {
       } else {
         double* r = (double*)rhs;
         const double* T = (const double*)tab;
-        if (dir == 0) solve_x_launch<double>(c, r, T, "tune", 1);
+        if (geo && dir == 0) geo_x_launch(c, r, T, 1, false);
+        else if (geo && dir == 1) geo_col_launch<false>(c, r, T, QSet{}, 1, 0, false);
+        else if (geo) geo_col_launch<true>(c, r, T, qset(&q, 1), 1, 0, true);
+        else if (dir == 0) solve_x_launch<double>(c, r, T, "tune", 1);
         else if (dir == 1) solve_y_launch<double>(c, r, T, "tune", 1);
         else solve_z_launch<double>(c, r, T, qset(&q, 1), 1, 0, nullptr, "tune");
       }
