@@ -12,10 +12,10 @@
 //   genSDF.f90:120-365, tagCells.f90:85-111 narrow-band tagging
 //   pencil_rayTag.f90:37-460                initial full tagging
 //
-// Determinism: no floating-point atomics anywhere.  Force spreading is an
-// atomics-free sorted scatter: the 27 cage cells of every triangle are keyed
-// by cell index and stably radix-sorted once per geometry (the key order
-// depends only on the mesh), then each unique cell sums its contributions in
+// Determinism: no floating-point atomics anywhere.  Force spreading gathers:
+// the 27 cage cells of every triangle are grouped by cell once per geometry
+// (the scatter plan below; integer atomics only, and its finished order
+// depends only on the mesh), then each touched cell sums its contributions in
 // triangle order -- the reference's summation order.  Face->vertex sums use
 // a vertex->face adjacency list in ascending face order.  The narrow band
 // takes the minimum distance with 64-bit integer atomicMin on the
@@ -456,16 +456,25 @@ __global__ void force_coef_kernel(Grid g, int nf, ForceArgs F, double tmelt, dou
 }
 
 // ---------------------------------------------------------------------
-// Stable LSD radix sort of (key, value) pairs, 8-bit digits.
+// Scatter plan: the entries grouped by cell, without a sort of the entries.
 // ---------------------------------------------------------------------
-constexpr int kSortChunk = 4096;
-
 // The four cage sets (x, y, z staggered, cell-centred) are merged into one
 // plan: entry e = comp*27*nf + 27*t + slot, key = comp*cells + cage cell
-// (4*cells, after every cell, for ghost faces).  The plan depends only on the cage centres
-// (pind) and the ghost flags; `plan_check` compares them with the values the
-// plan was built from and every kernel of the rebuild returns at once when
-// nothing changed, so a rebuild costs nothing on a stationary cage.
+// (ghost faces have no entries).  A run is the entries of one key, in triangle
+// order; runs are numbered in key order.  The keys touched are marked in a
+// bitmap of 4*cells bits; a scan of its population counts numbers the runs in
+// key order; each entry then takes a slot of its run with one atomic, runs
+// take storage from a cursor, and a warp per run puts its few tens of entries
+// into triangle order by rank.  The slots and the storage depend on the order
+// of the atomics, the finished runs do not.  Eight launches, each a few
+// microseconds: this chain is on the step's critical path at small and
+// moderate grids.  A radix sort of all entries by key in its place took 3 or 4
+// passes of five launches and five more for the run heads (5120 faces on
+// 128^3: PLAN_FIGS).
+// The plan depends only on the cage centres (pind) and the ghost flags;
+// `plan_check` compares them with the values the plan was built from and
+// every kernel of the rebuild returns at once when nothing changed, so a
+// rebuild costs nothing on a stationary cage.
 __global__ void plan_check_kernel(int nf, const int* __restrict__ pind, const int* __restrict__ ghost,
                                   const int* __restrict__ saved, int* __restrict__ dirty,
                                   const StepParams* __restrict__ pp) {
@@ -479,159 +488,184 @@ __global__ void plan_check_kernel(int nf, const int* __restrict__ pind, const in
   if (diff) atomicOr(dirty, 1);
 }
 
-__global__ void plan_commit_kernel(int nf, const int* __restrict__ pind, const int* __restrict__ ghost,
-                                   int* __restrict__ saved, const int* __restrict__ dirty) {
-  if (!*dirty) return;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nf) return;
-  for (int q = 0; q < 6; ++q) saved[7 * (size_t)t + q] = pind[6 * t + q];
-  saved[7 * (size_t)t + 6] = ghost[t];
-}
-
-__global__ void plan_keys_kernel(Grid g, int nf, const int* __restrict__ pind, const int* __restrict__ ghost,
-                                 const int* __restrict__ dirty, int* __restrict__ key, int* __restrict__ src) {
-  if (!*dirty) return;
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  int per = 27 * nf;
-  if (e >= 4 * per) return;
-  int comp = e / per, r = e % per, t = r / 27, sl = r % 27;
-  if (ghost[t]) { key[e] = (int)(4 * g.cells); src[e] = e; return; }   // sorts after every cell
+// key of entry e, or -1 for a ghost face
+__device__ __forceinline__ int plan_key(const Grid& g, int nf, const int* __restrict__ pind,
+                                        const int* __restrict__ ghost, int e) {
+  const int per = 27 * nf, comp = e / per, r = e - comp * per, t = r / 27, sl = r - 27 * t;
+  if (ghost[t]) return -1;
   int i0, j0, k0;
   cage_center(comp, pind + 6 * t, i0, j0, k0);
-  key[e] = (int)((size_t)comp * g.cells + cage_cell(g, i0, j0, k0, sl));
-  src[e] = e;
+  return (int)((size_t)comp * g.cells + cage_cell(g, i0, j0, k0, sl));
 }
 
-__global__ void radix_hist_kernel(const int* __restrict__ key, int n, int shift, int nblk,
-                                  const int* __restrict__ dirty, int* __restrict__ hist) {
+__global__ void __launch_bounds__(256) plan_mark_kernel(Grid g, int nf, const int* __restrict__ pind,
+                                                        const int* __restrict__ ghost, const int* __restrict__ dirty,
+                                                        unsigned* __restrict__ bitmap) {
   if (!*dirty) return;
-  __shared__ int h[256];
-  for (int d = threadIdx.x; d < 256; d += blockDim.x) h[d] = 0;
-  __syncthreads();
-  int b = blockIdx.x;
-  int end = min(n, (b + 1) * kSortChunk);
-  for (int e = b * kSortChunk + threadIdx.x; e < end; e += blockDim.x) atomicAdd(&h[(key[e] >> shift) & 255], 1);
-  __syncthreads();
-  for (int d = threadIdx.x; d < 256; d += blockDim.x) hist[d * nblk + b] = h[d];
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 108 * nf) return;
+  const int key = plan_key(g, nf, pind, ghost, e);
+  if (key < 0) return;
+  const unsigned bit = 1u << (key & 31);
+  if (!(bitmap[key >> 5] & bit)) atomicOr(bitmap + (key >> 5), bit);   // a stale 0 only repeats the atomic
 }
 
-// exclusive scan of one tile of 1024 ints in place (warp-shuffle scans,
-// then a scan of the 32 warp totals); the tile total goes to tsum[tile]
-__device__ __forceinline__ int block_exclusive_scan(int v, int* wsum, int& total) {
+// Bitmap scan in tiles of 4096 words (256 threads x 16 words): the tiles'
+// population counts, then (plan_runs_kernel) each tile's base from those of
+// the tiles before it, the run number at the start of every marked word, and
+// the runs' keys with their counts reset.
+constexpr int kPlanTile = 4096;
+__device__ __forceinline__ int plan_words(const unsigned* __restrict__ bitmap, int words, int w0, unsigned (&v)[16]) {
+  int n = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint4 u = make_uint4(0, 0, 0, 0);
+    if (w0 + 4 * q < words) u = reinterpret_cast<const uint4*>(bitmap + w0)[q];   // padded to a multiple of 4
+    v[4 * q] = u.x; v[4 * q + 1] = u.y; v[4 * q + 2] = u.z; v[4 * q + 3] = u.w;
+    n += __popc(u.x) + __popc(u.y) + __popc(u.z) + __popc(u.w);
+  }
+  return n;
+}
+
+// exclusive scan of one value per thread of a 256-thread block, and the total
+__device__ __forceinline__ int block_scan(int v, int* wsum, int& total) {
   const unsigned FULL = 0xffffffffu;
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int x = v;
   for (int off = 1; off < 32; off <<= 1) {
-    int u = __shfl_up_sync(FULL, x, off);
+    const int u = __shfl_up_sync(FULL, x, off);
     if (lane >= off) x += u;
   }
   if (lane == 31) wsum[w] = x;
   __syncthreads();
-  if (w == 0) {
-    int y = (lane < (int)(blockDim.x >> 5)) ? wsum[lane] : 0;
-    for (int off = 1; off < 32; off <<= 1) {
-      int u = __shfl_up_sync(FULL, y, off);
-      if (lane >= off) y += u;
-    }
-    wsum[lane] = y;                         // inclusive warp totals
+  int base = 0;
+  total = 0;
+  for (int q = 0; q < 8; ++q) {
+    if (q < w) base += wsum[q];
+    total += wsum[q];
   }
   __syncthreads();
-  total = wsum[(blockDim.x >> 5) - 1];
-  return x - v + (w > 0 ? wsum[w - 1] : 0);
+  return base + x - v;
 }
 
-__global__ void scan_tile_kernel(int* __restrict__ a, int m, int* __restrict__ tsum, const int* __restrict__ dirty) {
+__global__ void __launch_bounds__(256) plan_count_kernel(const unsigned* __restrict__ bitmap, int words,
+                                                         const int* __restrict__ dirty, int* __restrict__ tsum) {
   if (!*dirty) return;
-  __shared__ int wsum[32];
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  int v = (idx < m) ? a[idx] : 0;
+  __shared__ int wsum[8];
+  unsigned v[16];
   int total;
-  int ex = block_exclusive_scan(v, wsum, total);
-  if (idx < m) a[idx] = ex;
+  block_scan(plan_words(bitmap, words, blockIdx.x * kPlanTile + 16 * threadIdx.x, v), wsum, total);
   if (threadIdx.x == 0) tsum[blockIdx.x] = total;
 }
 
-__global__ void scan_add_kernel(int* __restrict__ a, int m, const int* __restrict__ tsum, const int* __restrict__ dirty) {
+__global__ void __launch_bounds__(256) plan_runs_kernel(const unsigned* __restrict__ bitmap, int words,
+                                                        const int* __restrict__ dirty, const int* __restrict__ tsum,
+                                                        int* __restrict__ wpre, int* __restrict__ run_key,
+                                                        int* __restrict__ run_cnt, int* __restrict__ nruns) {
   if (!*dirty) return;
-  int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx < m && blockIdx.x > 0) a[idx] += tsum[blockIdx.x];
-}
-
-// exclusive scan of m ints by one block of 1024 threads: coalesced tiles
-// of 1024, warp-shuffle scans inside a tile, a running carry across tiles
-// (used on the tile totals of the multi-block scan)
-__global__ void scan_kernel(int* __restrict__ a, int m, const int* __restrict__ dirty) {
-  if (!*dirty) return;
-  __shared__ int wsum[32];
-  __shared__ int carry;
-  const unsigned FULL = 0xffffffffu;
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int base = 0; base < m; base += blockDim.x) {
-    int idx = base + threadIdx.x;
-    int v = (idx < m) ? a[idx] : 0;
-    int x = v;
-    for (int off = 1; off < 32; off <<= 1) {
-      int u = __shfl_up_sync(FULL, x, off);
-      if (lane >= off) x += u;
+  __shared__ int wsum[8];
+  int before = 0, base;
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += 256) before += tsum[b];
+  block_scan(before, wsum, base);
+  unsigned v[16];
+  const int w0 = blockIdx.x * kPlanTile + 16 * threadIdx.x;
+  int total, at = block_scan(plan_words(bitmap, words, w0, v), wsum, total) + base;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    unsigned m = v[q];
+    if (!m) continue;
+    wpre[w0 + q] = at;
+    for (; m; m &= m - 1) {
+      run_key[at] = 32 * (w0 + q) + __ffs(m) - 1;
+      run_cnt[at] = 0;
+      ++at;
     }
-    if (lane == 31) wsum[w] = x;
-    __syncthreads();
-    if (w == 0) {
-      int y = wsum[lane];
-      for (int off = 1; off < 32; off <<= 1) {
-        int u = __shfl_up_sync(FULL, y, off);
-        if (lane >= off) y += u;
-      }
-      wsum[lane] = y;                       // inclusive warp totals
-    }
-    __syncthreads();
-    int incl = x + (w > 0 ? wsum[w - 1] : 0);
-    if (idx < m) a[idx] = carry + incl - v;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry += incl;
-    __syncthreads();
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    nruns[0] = base + total;
+    nruns[1] = 0;                        // the storage cursor
   }
 }
 
-// stable scatter: chunk order, then warp order, then lane order
-__global__ void radix_scatter_kernel(const int* __restrict__ kin, const int* __restrict__ vin, int* __restrict__ kout,
-                                     int* __restrict__ vout, int n, int shift, int nblk, const int* __restrict__ offs,
-                                     const int* __restrict__ dirty) {
+// a slot of its run for every entry
+__global__ void __launch_bounds__(256) plan_slot_kernel(Grid g, int nf, const int* __restrict__ pind,
+                                                        const int* __restrict__ ghost, const int* __restrict__ dirty,
+                                                        const unsigned* __restrict__ bitmap,
+                                                        const int* __restrict__ wpre, int* __restrict__ run_cnt,
+                                                        int2* __restrict__ slot) {
   if (!*dirty) return;
-  __shared__ int base[256];
-  __shared__ int wcnt[8][256];
-  int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  for (int d = tid; d < 256; d += 256) base[d] = offs[d * nblk + b];
-  __syncthreads();
-  int end = min(n, (b + 1) * kSortChunk);
-  for (int start = b * kSortChunk; start < end; start += 256) {
-    int idx = start + tid;
-    bool valid = idx < end;
-    int key = valid ? kin[idx] : 0;
-    int dig = valid ? ((key >> shift) & 255) : 256;
-    for (int q = tid; q < 8 * 256; q += 256) (&wcnt[0][0])[q] = 0;
-    __syncthreads();
-    unsigned peers = __match_any_sync(0xffffffffu, dig);
-    int rank = __popc(peers & ((1u << lane) - 1u));
-    int leader = __ffs(peers) - 1;
-    if (valid && lane == leader) wcnt[w][dig] = __popc(peers);
-    __syncthreads();
-    if (valid) {
-      int pre = 0;
-      for (int q = 0; q < w; ++q) pre += wcnt[q][dig];
-      int pos = base[dig] + pre + rank;
-      kout[pos] = key;
-      vout[pos] = vin[idx];
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 108 * nf) return;
+  const int key = plan_key(g, nf, pind, ghost, e);
+  int2 s = make_int2(-1, 0);
+  if (key >= 0) {
+    s.x = wpre[key >> 5] + __popc(bitmap[key >> 5] & ((1u << (key & 31)) - 1u));
+    s.y = atomicAdd(run_cnt + s.x, 1);
+  }
+  slot[e] = s;
+}
+
+// storage for every run: a warp of runs takes its total from the cursor
+__global__ void __launch_bounds__(256) plan_store_kernel(const int* __restrict__ dirty, const int* __restrict__ run_cnt,
+                                                         int* __restrict__ run_off, int* __restrict__ nruns) {
+  if (!*dirty) return;
+  const unsigned FULL = 0xffffffffu;
+  const int n = nruns[0], lane = threadIdx.x & 31;
+  for (int h0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); h0 < n; h0 += gridDim.x * blockDim.x) {
+    const int h = h0 + lane, v = h < n ? run_cnt[h] : 0;
+    int x = v;
+    for (int off = 1; off < 32; off <<= 1) {
+      const int u = __shfl_up_sync(FULL, x, off);
+      if (lane >= off) x += u;
     }
-    __syncthreads();
-    for (int d = tid; d < 256; d += 256) {
-      int tot = 0;
-      for (int q = 0; q < 8; ++q) tot += wcnt[q][d];
-      base[d] += tot;
+    int base = 0;
+    if (lane == 31) base = atomicAdd(nruns + 1, x);
+    base = __shfl_sync(FULL, base, 31);
+    if (h < n) run_off[h] = base + x - v;
+  }
+}
+
+// entries into their slots; the cage centres the plan was built from
+__global__ void __launch_bounds__(256) plan_place_kernel(int nf, const int* __restrict__ pind,
+                                                         const int* __restrict__ ghost, const int* __restrict__ dirty,
+                                                         const int2* __restrict__ slot, const int* __restrict__ run_off,
+                                                         int* __restrict__ entry, int* __restrict__ saved) {
+  if (!*dirty) return;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 108 * nf) return;
+  const int2 s = slot[e];
+  if (s.x >= 0) entry[run_off[s.x] + s.y] = e;
+  if (e < nf) {
+    for (int q = 0; q < 6; ++q) saved[7 * (size_t)e + q] = pind[6 * e + q];
+    saved[7 * (size_t)e + 6] = ghost[e];
+  }
+}
+
+// a warp per run: the run's entries into triangle order (the rank of an entry
+// is the number of smaller ones), and its word of the bitmap back to zero for
+// the next build
+__global__ void __launch_bounds__(256) plan_order_kernel(const int* __restrict__ dirty, const int* __restrict__ nruns,
+                                                         const int* __restrict__ run_key,
+                                                         const int* __restrict__ run_off,
+                                                         const int* __restrict__ run_cnt,
+                                                         const int* __restrict__ entry, int* __restrict__ src,
+                                                         unsigned* __restrict__ bitmap) {
+  if (!*dirty) return;
+  const unsigned FULL = 0xffffffffu;
+  const int n = nruns[0], lane = threadIdx.x & 31, nw = gridDim.x * 8;
+  for (int h = blockIdx.x * 8 + (threadIdx.x >> 5); h < n; h += nw) {
+    const int o = run_off[h], len = run_cnt[h];
+    if (lane == 0) bitmap[run_key[h] >> 5] = 0u;
+    for (int i0 = 0; i0 < len; i0 += 32) {
+      const int v = i0 + lane < len ? entry[o + i0 + lane] : 0;
+      int rank = 0;
+      for (int j0 = 0; j0 < len; j0 += 32) {
+        const int u = j0 + lane < len ? entry[o + j0 + lane] : 0x7fffffff;
+#pragma unroll 8
+        for (int q = 0; q < 32; ++q) rank += __shfl_sync(FULL, u, q) < v;
+      }
+      if (i0 + lane < len) src[o + rank] = v;
     }
-    __syncthreads();
   }
 }
 
@@ -646,31 +680,7 @@ struct ScatterOut {
 
 __device__ __forceinline__ int key_comp(int k, size_t cells) {
   size_t u = (size_t)k;
-  return (u >= cells) + (u >= 2 * cells) + (u >= 3 * cells) + (u >= 4 * cells);   // 4 = ghost face
-}
-
-// Heads of the sorted plan (the first entry of each run of one real key),
-// in key order, built with the plan: flag, exclusive scan, compaction.
-__device__ __forceinline__ bool plan_head(const int* __restrict__ key, int e, size_t cells) {
-  const int k = key[e];
-  return key_comp(k, cells) < 4 && (e == 0 || key[e - 1] != k);
-}
-
-__global__ void head_flag_kernel(int n, size_t cells, const int* __restrict__ key, const int* __restrict__ dirty,
-                                 int* __restrict__ hidx) {
-  if (!*dirty) return;
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < n) hidx[e] = plan_head(key, e, cells) ? 1 : 0;
-}
-
-__global__ void head_compact_kernel(int n, size_t cells, const int* __restrict__ key, const int* __restrict__ hidx,
-                                    const int* __restrict__ dirty, int* __restrict__ heads, int* __restrict__ nheads) {
-  if (!*dirty) return;
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  const bool head = plan_head(key, e, cells);
-  if (head) heads[hidx[e]] = e;
-  if (e == n - 1) *nheads = hidx[e] + (head ? 1 : 0);
+  return (u >= cells) + (u >= 2 * cells) + (u >= 3 * cells);
 }
 
 // One warp per run (a cell of one component): the lanes take every 32nd
@@ -681,26 +691,31 @@ __global__ void head_compact_kernel(int n, size_t cells, const int* __restrict__
 // thread.  With `segval` the run sum is also recorded at the run's index
 // (for the mean force).
 constexpr int kScatterBlocks = 1216;     // 8 blocks of 8 warps per SM on 152 SMs; the warps loop over runs
-__global__ void __launch_bounds__(256) scatter_apply_kernel(int n, int nf, size_t cells, const int* __restrict__ key,
-                                     const int* __restrict__ src, const double* __restrict__ coef, ScatterOut O,
-                                     int comp_lo, int comp_hi, const int* __restrict__ heads,
-                                     const int* __restrict__ nheads, double* __restrict__ segval) {
+struct PlanRuns {
+  const int* n;       // number of runs
+  const int* key;     // per run, ascending: key, first entry in src, entries
+  const int* off;
+  const int* cnt;
+  const int* src;     // entries in triangle order within a run
+};
+__global__ void __launch_bounds__(256) scatter_apply_kernel(int nf, size_t cells, PlanRuns P,
+                                     const double* __restrict__ coef, ScatterOut O, int comp_lo, int comp_hi,
+                                     double* __restrict__ segval) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (blockDim.x >> 5);
-  const int nh = *nheads;
+  const int nh = *P.n;
   const int per = 27 * nf;
   for (int h = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); h < nh; h += nw) {
-    const int e0 = heads[h];
-    const int k = key[e0];
+    const int k = P.key[h];
     const int comp = key_comp(k, cells);
     if (comp < comp_lo || comp >= comp_hi) continue;            // uniform over the warp
-    const int e1 = h + 1 < nh ? heads[h + 1] : n;               // the last run ends before the ghost entries
+    const int e0 = P.off[h], e1 = e0 + P.cnt[h];
     const double* __restrict__ phi = O.phi[comp];
     const double* __restrict__ cf = coef + (size_t)comp * nf;
     double sum = 0.0;
-    for (int q = e0 + lane; q < e1 && key[q] == k; q += 32) {
-      const int sr = src[q] - comp * per;
+    for (int q = e0 + lane; q < e1; q += 32) {
+      const int sr = P.src[q] - comp * per;
       if (!MIBM_IDX_OK(sr, per)) continue;
       sum = fma(cf[sr / 27], phi[sr], sum);
     }
@@ -724,19 +739,18 @@ __global__ void __launch_bounds__(256) scatter_apply_kernel(int n, int nf, size_
 // means divided by the cell count (FP64 at mean3[0..2], an FP32
 // copy for the precision form at float offset 8)
 constexpr int kMeanBlocks = 256;
-__global__ void __launch_bounds__(256) seg_mean_kernel(const int* __restrict__ nheads, const int* __restrict__ heads,
-                                                      size_t cells, const int* __restrict__ key,
+__global__ void __launch_bounds__(256) seg_mean_kernel(PlanRuns P, size_t cells,
                                                       const double* __restrict__ segval, double* __restrict__ part,
                                                       double ncell, double* __restrict__ mean3) {
   const unsigned FULL = 0xffffffffu;
   __shared__ double ws[8][3];
   __shared__ bool last;
-  const int n = *nheads;
+  const int n = *P.n;
   int per = (n + gridDim.x - 1) / gridDim.x;
   int lo = blockIdx.x * per, hi = min(n, lo + per);
   double s[3] = {0, 0, 0};
   for (int h = lo + threadIdx.x; h < hi; h += blockDim.x) {
-    int comp = key_comp(key[heads[h]], cells);
+    int comp = key_comp(P.key[h], cells);
     if (comp < 3) s[comp] += segval[h];
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1931,11 +1945,13 @@ struct LagState {
   int4* face_cell = nullptr;
   float* cm32 = nullptr;
   // merged scatter plan
-  int plan_n = 0, plan_cap = 0, nblk = 0;
-  int *key = nullptr, *src = nullptr, *tmp_key = nullptr, *tmp_src = nullptr, *hist = nullptr;
-  int* tsum = nullptr;   // tile totals of the histogram scan
-  int *hidx = nullptr, *heads = nullptr, *nheads = nullptr, *htsum = nullptr;   // run heads of the plan
-  int *res_key = nullptr, *res_src = nullptr;   // buffers holding the sorted result
+  unsigned* bitmap = nullptr;                    // one bit per key, zero between builds
+  int *wpre = nullptr, *tsum = nullptr;          // run number at each marked word, marked keys per tile of words
+  int plan_words = 0;
+  int2* slot = nullptr;                          // per entry: its run and its slot in it
+  int *run_key = nullptr, *run_cnt = nullptr, *run_off = nullptr;
+  int* nruns = nullptr;                          // [0] runs, [1] storage cursor
+  int *entry = nullptr, *src = nullptr;          // entries by run, then in triangle order
   int* saved = nullptr;                          // 7 ints per face: pind(1:6), ghost
   int* dirty = nullptr;
   double* segval = nullptr;
@@ -2029,26 +2045,28 @@ static bool ensure_lag_buffers(Ctx* c) {
   }
   if (!c->tri_coef)
     if (!cuda_ok(c, cudaMalloc(&c->tri_coef, sizeof(double) * 4 * std::max(1, c->maxnf)), "lag")) return false;
-  if (!s->key) {
-    int n = 4 * 27 * std::max(1, c->maxnf);
-    s->nblk = (n + kSortChunk - 1) / kSortChunk;
-    bool ok = cuda_ok(c, cudaMalloc(&s->key, sizeof(int) * n), "plan") &&
+  if (!s->bitmap) {
+    const size_t n = 108 * (size_t)std::max(1, c->maxnf);
+    // runs: at most one per entry and one per key
+    const size_t runs = std::min(n, 4 * c->g.cells);
+    s->plan_words = (int)(div_up(4 * c->g.cells, 128) * 4);
+    bool ok = cuda_ok(c, cudaMalloc(&s->bitmap, sizeof(unsigned) * (size_t)s->plan_words), "plan") &&
+              cuda_ok(c, cudaMalloc(&s->wpre, sizeof(int) * (size_t)s->plan_words), "plan") &&
+              cuda_ok(c, cudaMalloc(&s->tsum, sizeof(int) * (size_t)div_up(s->plan_words, kPlanTile)), "plan") &&
+              cuda_ok(c, cudaMalloc(&s->slot, sizeof(int2) * n), "plan") &&
+              cuda_ok(c, cudaMalloc(&s->run_key, sizeof(int) * runs), "plan") &&
+              cuda_ok(c, cudaMalloc(&s->run_cnt, sizeof(int) * runs), "plan") &&
+              cuda_ok(c, cudaMalloc(&s->run_off, sizeof(int) * runs), "plan") &&
+              cuda_ok(c, cudaMalloc(&s->nruns, sizeof(int) * 2), "plan") &&
+              cuda_ok(c, cudaMalloc(&s->entry, sizeof(int) * n), "plan") &&
               cuda_ok(c, cudaMalloc(&s->src, sizeof(int) * n), "plan") &&
-              cuda_ok(c, cudaMalloc(&s->tmp_key, sizeof(int) * n), "plan") &&
-              cuda_ok(c, cudaMalloc(&s->tmp_src, sizeof(int) * n), "plan") &&
-              cuda_ok(c, cudaMalloc(&s->hist, sizeof(int) * 256 * (size_t)s->nblk), "plan") &&
-              cuda_ok(c, cudaMalloc(&s->tsum, sizeof(int) * (size_t)div_up(256 * (size_t)s->nblk, 1024)), "plan") &&
               cuda_ok(c, cudaMalloc(&s->saved, sizeof(int) * 7 * (size_t)std::max(1, c->maxnf)), "plan") &&
               cuda_ok(c, cudaMalloc(&s->dirty, sizeof(int)), "plan") &&
-              cuda_ok(c, cudaMalloc(&s->segval, sizeof(double) * n), "plan") &&
-              cuda_ok(c, cudaMalloc(&s->hidx, sizeof(int) * n), "plan") &&
-              cuda_ok(c, cudaMalloc(&s->heads, sizeof(int) * n), "plan") &&
-              cuda_ok(c, cudaMalloc(&s->nheads, sizeof(int)), "plan") &&
-              cuda_ok(c, cudaMalloc(&s->htsum, sizeof(int) * (size_t)div_up(n, 1024)), "plan");
+              cuda_ok(c, cudaMalloc(&s->segval, sizeof(double) * runs), "plan");
     if (!ok) return false;
-    s->plan_n = n;
+    cudaMemsetAsync(s->bitmap, 0, sizeof(unsigned) * (size_t)s->plan_words, c->stream);
     cudaMemsetAsync(s->saved, 0xff, sizeof(int) * 7 * (size_t)std::max(1, c->maxnf), c->stream);
-    cudaMemsetAsync(s->nheads, 0, sizeof(int), c->stream);
+    cudaMemsetAsync(s->nruns, 0, sizeof(int) * 2, c->stream);
   }
   return true;
 }
@@ -2082,46 +2100,31 @@ bool validate_mesh(Ctx* c) {
 // a step (a remesh, which runs without a step graph) is applied now too.
 static void update_plan(Ctx* c, const StepParams* dp) {
   LagState* s = lag_of(c);
-  int nf = c->maxnf, n = s->plan_n;
+  const int nf = c->maxnf, words = s->plan_words;
+  const unsigned eb = div_up(108 * (size_t)nf, 256), tiles = div_up(words, kPlanTile);
   cudaMemsetAsync(s->dirty, s->force_rebuild ? 1 : 0, sizeof(int), c->stream);   // non-zero: dirty
   s->force_rebuild = false;
   const int* pind = M<int>(c, MIBM_M_PIND);
   const int* ghost = M<int>(c, MIBM_M_GHOST_FACE);
   { MIBM_PROF(c, "plan_check");
     plan_check_kernel<<<div_up(nf, 256), 256, 0, c->stream>>>(nf, pind, ghost, s->saved, s->dirty, dp); }
-  { MIBM_PROF(c, "plan_keys");
-    plan_keys_kernel<<<div_up(n, 256), 256, 0, c->stream>>>(c->g, nf, pind, ghost, s->dirty, s->tmp_key, s->tmp_src); }
-  int* kin = s->tmp_key; int* vin = s->tmp_src; int* kout = s->key; int* vout = s->src;
-  int bits = 1;
-  while ((size_t(1) << bits) <= 4 * c->g.cells) ++bits;
-  int passes = (bits + 7) / 8;
-  for (int ps = 0; ps < passes; ++ps) {
-    int shift = 8 * ps;
-    { MIBM_PROF(c, "radix_hist");
-      radix_hist_kernel<<<s->nblk, 256, 0, c->stream>>>(kin, n, shift, s->nblk, s->dirty, s->hist); }
-    { MIBM_PROF(c, "radix_scan");
-      int m = 256 * s->nblk;
-      unsigned tiles = div_up(m, 1024);
-      scan_tile_kernel<<<tiles, 1024, 0, c->stream>>>(s->hist, m, s->tsum, s->dirty);
-      scan_kernel<<<1, 1024, 0, c->stream>>>(s->tsum, (int)tiles, s->dirty);
-      scan_add_kernel<<<tiles, 1024, 0, c->stream>>>(s->hist, m, s->tsum, s->dirty); }
-    { MIBM_PROF(c, "radix_scatter");
-      radix_scatter_kernel<<<s->nblk, 256, 0, c->stream>>>(kin, vin, kout, vout, n, shift, s->nblk, s->hist, s->dirty); }
-    std::swap(kin, kout); std::swap(vin, vout);
-  }
-  s->res_key = kin; s->res_src = vin;         // fixed per grid: the buffers of the last pass
-  { MIBM_PROF(c, "plan_heads");
-    const unsigned tiles = div_up(n, 1024);
-    head_flag_kernel<<<tiles, 1024, 0, c->stream>>>(n, c->g.cells, s->res_key, s->dirty, s->hidx);
-    scan_tile_kernel<<<tiles, 1024, 0, c->stream>>>(s->hidx, n, s->htsum, s->dirty);
-    scan_kernel<<<1, 1024, 0, c->stream>>>(s->htsum, (int)tiles, s->dirty);
-    scan_add_kernel<<<tiles, 1024, 0, c->stream>>>(s->hidx, n, s->htsum, s->dirty);
-    head_compact_kernel<<<tiles, 1024, 0, c->stream>>>(n, c->g.cells, s->res_key, s->hidx, s->dirty, s->heads,
-                                                       s->nheads); }
-  c->launches += 5;
-  { MIBM_PROF(c, "plan_commit");
-    plan_commit_kernel<<<div_up(nf, 256), 256, 0, c->stream>>>(nf, pind, ghost, s->saved, s->dirty); }
-  c->launches += 3 + 5 * passes;
+  { MIBM_PROF(c, "plan_mark");
+    plan_mark_kernel<<<eb, 256, 0, c->stream>>>(c->g, nf, pind, ghost, s->dirty, s->bitmap); }
+  { MIBM_PROF(c, "plan_runs");
+    plan_count_kernel<<<tiles, 256, 0, c->stream>>>(s->bitmap, words, s->dirty, s->tsum);
+    plan_runs_kernel<<<tiles, 256, 0, c->stream>>>(s->bitmap, words, s->dirty, s->tsum, s->wpre, s->run_key,
+                                                   s->run_cnt, s->nruns); }
+  { MIBM_PROF(c, "plan_slot");
+    plan_slot_kernel<<<eb, 256, 0, c->stream>>>(c->g, nf, pind, ghost, s->dirty, s->bitmap, s->wpre, s->run_cnt,
+                                                s->slot); }
+  { MIBM_PROF(c, "plan_store");
+    plan_store_kernel<<<std::min<unsigned>(eb, 304), 256, 0, c->stream>>>(s->dirty, s->run_cnt, s->run_off, s->nruns); }
+  { MIBM_PROF(c, "plan_place");
+    plan_place_kernel<<<eb, 256, 0, c->stream>>>(nf, pind, ghost, s->dirty, s->slot, s->run_off, s->entry, s->saved); }
+  { MIBM_PROF(c, "plan_order");
+    plan_order_kernel<<<std::min<unsigned>(eb, kScatterBlocks), 256, 0, c->stream>>>(
+        s->dirty, s->nruns, s->run_key, s->run_off, s->run_cnt, s->entry, s->src, s->bitmap); }
+  c->launches += 8;
   MIBM_LAUNCH_CHECK(c, "scatter plan");
 }
 
@@ -2151,12 +2154,14 @@ static void force_coefficients(Ctx* c) {
   ++c->launches;
 }
 
+static PlanRuns plan_runs(const LagState* s) { return PlanRuns{s->nruns, s->run_key, s->run_off, s->run_cnt, s->src}; }
+
 static void scatter(Ctx* c, bool into_fields, int lo, int hi, bool record, float* m32 = nullptr) {
   LagState* s = lag_of(c);
   { MIBM_PROF(c, "scatter_apply");
-    scatter_apply_kernel<<<(unsigned)std::min<size_t>(kScatterBlocks, div_up(s->plan_n, 256)), 256, 0, c->stream>>>(
-        s->plan_n, c->maxnf, c->g.cells, s->res_key, s->res_src, c->tri_coef, scatter_out(c, into_fields, m32), lo, hi,
-        s->heads, s->nheads, record ? s->segval : nullptr); }
+    scatter_apply_kernel<<<(unsigned)std::min<size_t>(kScatterBlocks, div_up(108 * (size_t)c->maxnf, 256)), 256, 0,
+                           c->stream>>>(c->maxnf, c->g.cells, plan_runs(s), c->tri_coef,
+                                        scatter_out(c, into_fields, m32), lo, hi, record ? s->segval : nullptr); }
   ++c->launches;
 }
 
@@ -2698,8 +2703,8 @@ const double* lagr_particle_fused(Ctx* c, const StepParams* dp, float* m32, Step
   scatter(c, true, 0, 3, true);
   double ncell = (double)c->g.n1m * (double)c->g.n2m * (double)c->g.n3m;
   { MIBM_PROF(c, "seg_mean");
-    seg_mean_kernel<<<kMeanBlocks, 256, 0, c->stream>>>(s->nheads, s->heads, c->g.cells, s->res_key, s->segval,
-                                                        c->red + kRedPart, ncell, s->mean3); }
+    seg_mean_kernel<<<kMeanBlocks, 256, 0, c->stream>>>(plan_runs(s), c->g.cells, s->segval, c->red + kRedPart, ncell,
+                                                        s->mean3); }
   c->launches += 1;
   // Fork: the rest of particle (heat flux, temperature forcing, Stefan
   // front, motion, geometry) reads and writes none of the buffers of the
@@ -2821,10 +2826,10 @@ void lagr_free(Ctx* c) {
       cudaFree(s->mean3); cudaFree(s->winner); cudaFree(s->dist_buf);
       cudaFree(s->band_ub); cudaFree(s->face4); cudaFree(s->face_cell); cudaFree(s->cm32);
       cudaFree(s->band_list); cudaFree(s->band_count);
-      cudaFree(s->key); cudaFree(s->src); cudaFree(s->tmp_key); cudaFree(s->tmp_src); cudaFree(s->hist);
-      cudaFree(s->tsum);
+      cudaFree(s->bitmap); cudaFree(s->wpre); cudaFree(s->tsum); cudaFree(s->slot);
+      cudaFree(s->run_key); cudaFree(s->run_cnt); cudaFree(s->run_off); cudaFree(s->nruns);
+      cudaFree(s->entry); cudaFree(s->src);
       cudaFree(s->saved); cudaFree(s->dirty); cudaFree(s->segval);
-      cudaFree(s->hidx); cudaFree(s->heads); cudaFree(s->nheads); cudaFree(s->htsum);
       delete s;
       g_lag.erase(g_lag.begin() + q);
       break;
