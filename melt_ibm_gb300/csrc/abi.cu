@@ -164,7 +164,7 @@ static bool tsolve_fork(Ctx* c) { return c->tsolve && !c->profiling && c->precis
 static void tsolve_begin(Ctx* c) {
   if (!tsolve_fork(c)) return;
   cudaEventRecord(c->ev_sfork, c->stream);
-  cudaStreamWaitEvent(c->tsolve, c->ev_sfork, 0);
+  wait_event(c, c->tsolve, c->ev_sfork);
   std::swap(c->stream, c->tsolve);
 }
 
@@ -175,7 +175,7 @@ static void tsolve_end(Ctx* c) {
 }
 
 static void tsolve_join(Ctx* c) {
-  if (tsolve_fork(c)) cudaStreamWaitEvent(c->stream, c->ev_sjoin, 0);
+  if (tsolve_fork(c)) wait_event(c, c->stream, c->ev_sjoin);
 }
 
 // Precision form: FP32 explicit terms, RHS, line solves and FFTs; u, v, w,
@@ -197,25 +197,26 @@ static void step_enqueue_f32(Ctx* c) {
     lagr_join_geom(c);            // the rest of the side branch is waited for before the forcing
     if (!c->prologue_done) { lagr_join(c); lagr_substep_prologue(c, ns); }
     c->prologue_done = false;
-    k_fused_rhs_f32(c, dp, c->ru32, c->rhs32);
     {
-      // T on its own stream, then u, v, w: one launch per direction (they
-      // share the velocity tables)
-      tsolve_begin(c);
-      const float* Tt = tf + (size_t)((ns * 2 + 1) * 3) * tlen;
-      float* r = c->rhs32 + 3 * g.cells;
-      double* qt[1] = {c->df[kStepFid[3]]};
-      k_solve_x_f32(c, r, Tt, 1);
-      k_solve_y_f32(c, r, Tt + tlen, 1);
-      k_solve_z_f32(c, r, Tt + 2 * tlen, qt, 1, t_mirror);
-      tsolve_end(c);
+      // u, v, w (one launch per direction: they share the velocity tables),
+      // then T: its explicit term reads the mirrors, which the velocity solves
+      // leave alone, so a moving body's loads (96 us per substep at 128^3,
+      // 5120 faces) run beside all of its work (50 us there)
+      k_rhs_uvw_f32(c, dp, c->ru32, c->rhs32);
       const float* Tv = tf + (size_t)((ns * 2 + 0) * 3) * tlen;
       double* qv[3] = {c->df[kStepFid[0]], c->df[kStepFid[1]], c->df[kStepFid[2]]};
       k_solve_x_f32(c, c->rhs32, Tv, 3);
       k_solve_y_f32(c, c->rhs32, Tv + tlen, 3);
       k_solve_z_f32(c, c->rhs32, Tv + 2 * tlen, qv, 3, nullptr);
-      lagr_loads_early(c, dp);                  // u, v, w solved: loads beside the forcing's preparation
-      tsolve_join(c);
+      lagr_loads_early(c, dp);                  // u, v, w solved
+      const float* Tt = tf + (size_t)((ns * 2 + 1) * 3) * tlen;
+      float* r = c->rhs32 + 3 * g.cells;
+      double* qt[1] = {c->df[kStepFid[3]]};
+      k_rhs_t_f32(c, dp, c->ru32 + 3 * g.cells, r);
+      k_solve_x_f32(c, r, Tt, 1);
+      k_solve_y_f32(c, r, Tt + tlen, 1);
+      k_solve_z_f32(c, r, Tt + 2 * tlen, qt, 1, t_mirror);
+      lagr_heat_early(c);
     }
     const double* mean3 = lagr_particle_fused(c, dp, c->q32, ns < 2 ? c->dparams + ns + 1 : nullptr, ns + 1);
     if (c->status != MIBM_OK) return;
@@ -266,6 +267,7 @@ static void step_enqueue_f64(Ctx* c) {
       k_solve_x_T(c, r, Tt, 1);
       k_solve_y_T(c, r, Tt + tlen, 1);
       k_solve_z_T(c, r, Tt + 2 * tlen, qt, 1, 0);
+      lagr_heat_early(c);
       tsolve_end(c);
       const double* Tv = tables + (size_t)((ns * 2 + 0) * 3) * tlen;
       double* qv[3] = {c->df[kStepFid[0]], c->df[kStepFid[1]], c->df[kStepFid[2]]};
@@ -364,6 +366,7 @@ static uint64_t step_key(Ctx* c) {
   }
   mix((uint64_t)c->precision); mix((uint64_t)c->nproj); mix(c->lag_gen); mix(c->q32 ? 1 : 0);
   mix(c->tune_gen); mix(c->diag_on ? 1 : 0); mix(c->tri_geo ? 1 : 0);
+  mix(c->linear ? 1 : 0);
   return h;
 }
 
@@ -382,9 +385,27 @@ static void drop_graph(Ctx* c) {
 }
 
 // Capture step_enqueue into a graph; false (and graphs off for this
-// context) if the capture or the instantiation fails.
+// context) if the capture or the instantiation fails.  A linear step (a member
+// of a large batch) has its side streams stand for the main one, so that the
+// forks and joins vanish and the graph is one chain.
 static bool capture_step(Ctx* c, uint64_t key) {
   drop_graph(c);
+  cudaStream_t* const sides[4] = {&c->side, &c->side2, &c->side3, &c->tsolve};
+  cudaStream_t own[4];
+  for (int q = 0; q < 4; ++q) {
+    own[q] = *sides[q];
+    if (c->linear) *sides[q] = c->stream;
+  }
+  c->one_stream = c->linear;
+  struct Restore {
+    Ctx* c;
+    cudaStream_t* const* sides;
+    cudaStream_t* own;
+    ~Restore() {
+      for (int q = 0; q < 4; ++q) *sides[q] = own[q];
+      c->one_stream = false;
+    }
+  } restore{c, sides, own};
   uint64_t gen = c->lag_gen, before = c->launches;
   if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
     cudaGetLastError();
@@ -419,6 +440,7 @@ static bool capture_step(Ctx* c, uint64_t key) {
 // tsch.f90:18-97 on the device.  From the second call on, the device part
 // runs as a captured graph (one launch per step) while its key holds.
 static void tschem(Ctx* c) {
+  c->linear = false;
   if (!step_prepare(c)) return;
   step_head(c);
   if (c->status != MIBM_OK) return;
@@ -586,8 +608,17 @@ static int batch_step(Batch* b, int ntime) {
     }
   }
   drop_failed(cs);
-  // (B) forcing (gcurv.f90:164-170) and the host part of each step
+  // (B) forcing (gcurv.f90:164-170) and the host part of each step.  The device
+  // runs a process's streams (and a graph's branches) on eight hardware
+  // queues; work that shares one waits in line.  A step graph has four
+  // branches most of the time, so from kLinearCases members up each case runs
+  // as one chain and the cases alone overlap (us per case and step of n 48^3
+  // cases as chains / as branching graphs, precision form: n = 3 391 / 375, 4
+  // 334 / 343, 5 293 / 349, 8 226 / 318; FP64 form: 4 484 / 468, 5 424 / 453, 8
+  // 331 / 419).
+  constexpr size_t kLinearCases = 5;
   for (Ctx* c : cs) {
+    c->linear = cs.size() >= kLinearCases;
     if (c->I(MIBM_I_FORCING) == 1) {
       int which = c->I(MIBM_I_WHICH_HIT);
       if (which == 1) k_hit_random_force(c);

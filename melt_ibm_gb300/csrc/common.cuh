@@ -151,7 +151,10 @@ struct Ctx {
   cudaEvent_t ev_lfork = nullptr, ev_ldone = nullptr;   // structural loads on the side stream
   cudaStream_t side2 = nullptr;                         // narrow-band tagging beside the MLS weights and plan
   cudaEvent_t ev_tfork = nullptr, ev_tjoin = nullptr;
-  cudaStream_t side3 = nullptr;                         // MLS weights beside the scatter plan
+  cudaStream_t side3 = nullptr;                         // body sums and MLS weights beside the scatter plan
+  // heat flux and temperature forcing on the tagging's stream
+  cudaEvent_t ev_hfork = nullptr, ev_hflux = nullptr, ev_tscat = nullptr;
+  bool heat_pending = false, tscat_pending = false;
   cudaEvent_t ev_wfork = nullptr, ev_wjoin = nullptr;
   cudaStream_t tsolve = nullptr;                        // the temperature's line solves beside the velocity's
   cudaEvent_t ev_sfork = nullptr, ev_sjoin = nullptr;
@@ -200,6 +203,8 @@ struct Ctx {
   bool profiling = false;                 // per-kernel event profiling on (no graphs then)
   // shapes chosen by the autotuner (tune.cu); -1 / 8 = the default rules
   int tune_m[3] = {-1, -1, -1};           // line-solve chunk length per direction
+  bool linear = false;                    // member of a large batch: the step graph is one chain
+  bool one_stream = false;                // capturing that chain: the side streams stand for the main one
   bool tri_geo = false;                   // FP64 step: every line solve takes the geo_* kernels (tridiag.cu)
   int tune_by = 2;                        // block height of the explicit-term kernels (32 x 2 threads: the
                                           // autotuner's choice at 48^3, 128^3 and 256^3)
@@ -337,7 +342,8 @@ inline void field_host_shape(const Ctx* c, int id, int& ny, int& klo, int& nk) {
 void k_hdnl(Ctx* c, int which, const StepParams* dp);
 void k_invtr_rhs(Ctx* c, int which, const StepParams* dp, double* rhs_out);
 void k_fused_rhs(Ctx* c, const StepParams* dp);
-void k_fused_rhs_f32(Ctx* c, const StepParams* dp, float* ru4, float* rhs4);
+void k_rhs_uvw_f32(Ctx* c, const StepParams* dp, float* ru4, float* rhs4);
+void k_rhs_t_f32(Ctx* c, const StepParams* dp, float* ru, float* rhs);
 void k_updvp_f32(Ctx* c, const StepParams* dp, const float* phi, const double* mean3, bool mirror);
 void k_prcalc_f32(Ctx* c, const StepParams* dp, const float* phi, bool mirror);
 void k_divg_f32(Ctx* c, const StepParams* dp, float* res);
@@ -443,6 +449,7 @@ void lagr_step_readback(Ctx* c);
 void lagr_join(Ctx* c);
 void lagr_join_geom(Ctx* c);
 void lagr_loads_early(Ctx* c, const StepParams* dp);
+void lagr_heat_early(Ctx* c);
 bool lagr_fork_enabled(Ctx* c);
 void lagr_step_host_finish(Ctx* c);
 void lagr_geometry_to_host(Ctx* c);
@@ -450,6 +457,12 @@ void lagr_invalidate(Ctx* c);
 void lagr_topology_changed(Ctx* c);
 bool lagr_remesh_active(Ctx* c);
 void lagr_free(Ctx* c);
+// an event wait between the streams of a context; none where one stream
+// stands for all (an edge to an older node of the same chain would make the
+// graph branch)
+inline void wait_event(Ctx* c, cudaStream_t s, cudaEvent_t ev) {
+  if (!c->one_stream) cudaStreamWaitEvent(s, ev, 0);
+}
 // ctx.cu
 bool ensure_params(Ctx* c);
 bool validate_mesh(Ctx* c);

@@ -324,6 +324,9 @@ void release(Ctx* c) {
   if (c->ev_sjoin) cudaEventDestroy(c->ev_sjoin);
   if (c->ev_wfork) cudaEventDestroy(c->ev_wfork);
   if (c->ev_wjoin) cudaEventDestroy(c->ev_wjoin);
+  if (c->ev_hfork) cudaEventDestroy(c->ev_hfork);
+  if (c->ev_hflux) cudaEventDestroy(c->ev_hflux);
+  if (c->ev_tscat) cudaEventDestroy(c->ev_tscat);
   if (c->ev_tfork) cudaEventDestroy(c->ev_tfork);
   if (c->ev_tjoin) cudaEventDestroy(c->ev_tjoin);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
@@ -368,6 +371,9 @@ int mibm_context_create_(void) {
       !cuda_ok(c, cudaEventCreateWithFlags(&c->ev_sjoin, cudaEventDisableTiming), "event") ||
       !cuda_ok(c, cudaEventCreateWithFlags(&c->ev_wfork, cudaEventDisableTiming), "event") ||
       !cuda_ok(c, cudaEventCreateWithFlags(&c->ev_wjoin, cudaEventDisableTiming), "event") ||
+      !cuda_ok(c, cudaEventCreateWithFlags(&c->ev_hfork, cudaEventDisableTiming), "event") ||
+      !cuda_ok(c, cudaEventCreateWithFlags(&c->ev_hflux, cudaEventDisableTiming), "event") ||
+      !cuda_ok(c, cudaEventCreateWithFlags(&c->ev_tscat, cudaEventDisableTiming), "event") ||
       !cuda_ok(c, cudaEventCreateWithFlags(&c->ev_tfork, cudaEventDisableTiming), "event") ||
       !cuda_ok(c, cudaEventCreateWithFlags(&c->ev_tjoin, cudaEventDisableTiming), "event") ||
       !cuda_ok(c, cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming), "event") ||

@@ -125,22 +125,31 @@ __device__ bool inv4(double* a) {
   return true;
 }
 
+// Blocks of one warp for the kernels over faces, probes and vertices.  Their
+// warps are chains of FP64 instructions, which the warps of an SM share a
+// narrow pipe for, and a body has few of them (1280 faces: 40 to 160 warps):
+// blocks of four warps left most SMs idle beside some with eight warps to run.
+// Blocks of 128 -> 32 threads: mls_weight_sep 69 -> 49 us (5120 faces), 166 ->
+// 146 us (20480), heat_flux_sep 125 -> 104 us (20480), the others unchanged.
+constexpr int kLagBlock = 32;
+
 // ---------------------------------------------------------------------
 // findCentroidIndices / findProbeIndices
 // ---------------------------------------------------------------------
-__global__ void centroid_idx_kernel(LagArgs A, const double* __restrict__ tri_bar, const int* __restrict__ ghost,
-                                    int* __restrict__ pind) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= A.nf || ghost[t]) return;
-  const Grid& g = A.g;
-  double px = tri_bar[3 * t], py = tri_bar[3 * t + 1], pz = tri_bar[3 * t + 2];
+__device__ __forceinline__ void centroid_idx_one(const Grid& g, double px, double py, double pz, int* p) {
   int i1 = ffloor(px * g.dx1) + 1, ist = fnint(px * g.dx1) + 1;
   int j1 = ffloor(py * g.dx2) + 1, jst = fnint(py * g.dx2) + 1;
   int k1 = ffloor(pz * g.dx3) + 1, kst = fnint(pz * g.dx3) + 1;
   k1 = fmod_pos(k1 - 1, g.n3m) + 1;
   kst = fmod_pos(kst - 1, g.n3m) + 1;
-  int* p = pind + 6 * t;
   p[0] = i1; p[1] = j1; p[2] = k1; p[3] = ist; p[4] = jst; p[5] = kst;
+}
+
+__global__ void centroid_idx_kernel(LagArgs A, const double* __restrict__ tri_bar, const int* __restrict__ ghost,
+                                    int* __restrict__ pind) {
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= A.nf || ghost[t]) return;
+  centroid_idx_one(A.g, tri_bar[3 * t], tri_bar[3 * t + 1], tri_bar[3 * t + 2], pind + 6 * t);
 }
 
 __global__ void probe_idx_kernel(LagArgs A, const double* __restrict__ tri_bar, const double* __restrict__ tri_nor,
@@ -469,8 +478,8 @@ __global__ void force_coef_kernel(Grid g, int nf, ForceArgs F, double tmelt, dou
 // of the atomics, the finished runs do not.  Eight launches, each a few
 // microseconds: this chain is on the step's critical path at small and
 // moderate grids.  A radix sort of all entries by key in its place took 3 or 4
-// passes of five launches and five more for the run heads (5120 faces on
-// 128^3: PLAN_FIGS).
+// passes of five launches and five more for the run heads (serial kernel time
+// of the plan, 5120 faces on 128^3: 170 -> 95 us per substep).
 // The plan depends only on the cage centres (pind) and the ghost flags;
 // `plan_check` compares them with the values the plan was built from and
 // every kernel of the rebuild returns at once when nothing changed, so a
@@ -1119,7 +1128,9 @@ __global__ void heat_flux_sep_kernel(LagArgs A, const double* __restrict__ temp,
     double nd = tri_nor[3 * t + d];
     pos[d] = side == 0 ? tri_bar[3 * t + d] + h * nd / s : tri_bar[3 * t + d] - h * nd / s;
   }
-  int pi1 = pind[6 * t + 3 * side + 0], pi2 = pind[6 * t + 3 * side + 1];
+  // pind null (fused step): the probe's cage as probe_idx_kernel finds it
+  const int pi1 = pind ? pind[6 * t + 3 * side + 0] : ffloor(pos[0] * A.g.dx1) + 1;
+  const int pi2 = pind ? pind[6 * t + 3 * side + 1] : ffloor(pos[1] * A.g.dx2) + 1;
   double grad[3];
   if (!probe_grad_sep(A, pos, pi1, pi2, 1, 1, 1, false, temp, grad)) { atomicOr(flag, 1); qout[t] = 0.0; return; }
   double qv = n0 * grad[0] + n1 * grad[1] + n2 * grad[2];
@@ -1160,8 +1171,9 @@ heat_flux_lit_kernel(LagArgs A, const double* __restrict__ temp, const double* _
       const double nd = tri_nor[3 * t + d];
       pos[d] = side == 0 ? tri_bar[3 * t + d] + h * nd / s : tri_bar[3 * t + d] - h * nd / s;
     }
-    pi1 = pind[6 * t + 3 * side + 0];
-    pi2 = pind[6 * t + 3 * side + 1];
+    // pind null (fused step): the probe's cage as probe_idx_kernel finds it
+    pi1 = pind ? pind[6 * t + 3 * side + 0] : ffloor(pos[0] * g.dx1) + 1;
+    pi2 = pind ? pind[6 * t + 3 * side + 1] : ffloor(pos[1] * g.dx2) + 1;
     k1 = ffloor(pos[2] * g.dx3) + 1;
   }
   if (w == 0 && live) {
@@ -1402,21 +1414,45 @@ loads_face_kernel(LagArgs A, const double* __restrict__ pr, const double* __rest
 }
 
 // face -> vertex: qw_v(v) = sum over adjacent faces (ascending) of q_f*(A_f/3/A_v)
-__global__ void face_to_vert_kernel(int nv, const int* __restrict__ adj_off, const int* __restrict__ adj_face,
-                                    const double* __restrict__ sur, const double* __restrict__ avert,
-                                    const double* __restrict__ qf_o, const double* __restrict__ qf_i,
-                                    double* __restrict__ qv_o, double* __restrict__ qv_i) {
-  int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nv) return;
-  double so = 0.0, si = 0.0, av = avert[v];
+__device__ __forceinline__ void vert_flux(int v, const int* __restrict__ adj_off, const int* __restrict__ adj_face,
+                                          const double* __restrict__ sur, const double* __restrict__ avert,
+                                          const double* __restrict__ qf_o, const double* __restrict__ qf_i,
+                                          double& so, double& si) {
+  const double av = avert[v];
+  so = si = 0.0;
   for (int q = adj_off[v]; q < adj_off[v + 1]; ++q) {
     int f = adj_face[q];
     double w = sur[f] / 3.0 / av;
     so = so + qf_o[f] * w;
     si = si + qf_i[f] * w;
   }
+}
+
+__global__ void face_to_vert_kernel(int nv, const int* __restrict__ adj_off, const int* __restrict__ adj_face,
+                                    const double* __restrict__ sur, const double* __restrict__ avert,
+                                    const double* __restrict__ qf_o, const double* __restrict__ qf_i,
+                                    double* __restrict__ qv_o, double* __restrict__ qv_i) {
+  int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= nv) return;
+  double so, si;
+  vert_flux(v, adj_off, adj_face, sur, avert, qf_o, qf_i, so, si);
   qv_o[v] = so;
   qv_i[v] = si;
+}
+
+__device__ __forceinline__ void vert_melt(int v, const int* __restrict__ ghostv, const double* __restrict__ vert_nor,
+                                          double qo, double qi, double cp_over_L, const StepParams* __restrict__ pp,
+                                          double* __restrict__ vmelt, double* __restrict__ vmelt_m1,
+                                          double* __restrict__ xyzv) {
+  double dt = pp->dt, ga = pp->ga, ro = pp->ro;
+  for (int d = 0; d < 3; ++d) vmelt_m1[3 * v + d] = vmelt[3 * v + d];
+  if (ghostv[v]) return;
+  double dq = qi - qo;
+  for (int d = 0; d < 3; ++d) {
+    double vm = cp_over_L * dq * vert_nor[3 * v + d];
+    vmelt[3 * v + d] = vm;
+    xyzv[3 * v + d] = xyzv[3 * v + d] + dt * (ga * vm + ro * vmelt_m1[3 * v + d]);
+  }
 }
 
 __global__ void stefan_kernel(int nv, const int* __restrict__ ghostv, const double* __restrict__ vert_nor,
@@ -1425,15 +1461,24 @@ __global__ void stefan_kernel(int nv, const int* __restrict__ ghostv, const doub
                               double* __restrict__ vmelt_m1, double* __restrict__ xyzv) {
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nv) return;
-  double dt = pp->dt, ga = pp->ga, ro = pp->ro;
-  for (int d = 0; d < 3; ++d) vmelt_m1[3 * v + d] = vmelt[3 * v + d];
-  if (ghostv[v]) return;
-  double dq = qv_i[v] - qv_o[v];
-  for (int d = 0; d < 3; ++d) {
-    double vm = cp_over_L * dq * vert_nor[3 * v + d];
-    vmelt[3 * v + d] = vm;
-    xyzv[3 * v + d] = xyzv[3 * v + d] + dt * (ga * vm + ro * vmelt_m1[3 * v + d]);
-  }
+  vert_melt(v, ghostv, vert_nor, qv_o[v], qv_i[v], cp_over_L, pp, vmelt, vmelt_m1, xyzv);
+}
+
+// face_to_vert_kernel and stefan_kernel for one vertex in one launch (fused step)
+__global__ void melt_vert_kernel(int nv, const int* __restrict__ adj_off, const int* __restrict__ adj_face,
+                                 const double* __restrict__ sur, const double* __restrict__ avert,
+                                 const double* __restrict__ qf_o, const double* __restrict__ qf_i,
+                                 double* __restrict__ qv_o, double* __restrict__ qv_i, const int* __restrict__ ghostv,
+                                 const double* __restrict__ vert_nor, double cp_over_L,
+                                 const StepParams* __restrict__ pp, double* __restrict__ vmelt,
+                                 double* __restrict__ vmelt_m1, double* __restrict__ xyzv) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= nv) return;
+  double so, si;
+  vert_flux(v, adj_off, adj_face, sur, avert, qf_o, qf_i, so, si);
+  qv_o[v] = so;
+  qv_i[v] = si;
+  vert_melt(v, ghostv, vert_nor, so, si, cp_over_L, pp, vmelt, vmelt_m1, xyzv);
 }
 
 // ---------------------------------------------------------------------
@@ -1476,6 +1521,25 @@ __device__ __forceinline__ void face_geom_one(int t, const int* __restrict__ vof
   pp[11] = v * (z1 * y1 + z2 * y2 + z3 * y3 + z4 * y4);
 }
 
+// the narrow band's FP32 centroid and circumradius of face f and the base
+// cell of its 5^3 band (see band_ub_kernel)
+__device__ __forceinline__ void band_prep_one(int f, int nv, const int* __restrict__ vof, const double* __restrict__ x,
+                                              const double pos[3], const Grid& g, float4* __restrict__ face4,
+                                              int4* __restrict__ face_cell) {
+  int vid[3] = {vof[3 * f] - 1, vof[3 * f + 1] - 1, vof[3 * f + 2] - 1};
+  if (!(MIBM_IDX_OK(vid[0], nv) & MIBM_IDX_OK(vid[1], nv) & MIBM_IDX_OK(vid[2], nv))) vid[0] = vid[1] = vid[2] = 0;
+  double r2 = 0.0;
+  for (int v = 0; v < 3; ++v) {
+    const double dx = x[3 * vid[v]] - pos[0], dy = x[3 * vid[v] + 1] - pos[1], dz = x[3 * vid[v] + 2] - pos[2];
+    r2 = fmax(r2, dx * dx + dy * dy + dz * dz);
+  }
+  float R = (float)sqrt(r2);
+  R = R * 1.000001f + 1e-30f;                                        // round the radius up
+  face4[f] = make_float4((float)pos[0], (float)pos[1], (float)pos[2], R);
+  // base cell of the band, as band_kernel derives it (genSDF.f90:151-153)
+  face_cell[f] = make_int4(ffloor(pos[0] * g.dx1) + 1, ffloor(pos[1] * g.dx2) + 1, ffloor(pos[2] * g.dx3) + 1, 0);
+}
+
 // the post-processing of calc_rigidBody_params (RigidAuxRoutines.f90:736-775)
 // from the 12 body sums: [Surface, Volume1, Volume, pos_CM(3), InertTensor(9)]
 __device__ void geom_finish(const double* sm, double dens_ratio, double* __restrict__ out) {
@@ -1496,6 +1560,23 @@ __device__ void geom_finish(const double* sm, double dens_ratio, double* __restr
   for (int q = 0; q < 9; ++q) out[6 + q] = I[q] * dens_ratio;
 }
 
+// What the next substep derives from the faces alone, formed with them (fused
+// step; null pointers: not wanted): the narrow band's bounds (band_prep_one), the cage
+// indices (findCentroidIndices) and whether they differ from the ones the
+// scatter plan was built from, and cfac (initmls.f90:25).  Separate kernels
+// for these were three more launches on the chain between two substeps.
+struct FaceNext {
+  Grid g;
+  int nv;
+  float4* face4;
+  int4* face_cell;
+  int* pind;
+  const int* saved;      // plan_check's
+  int* dirty;
+  double* cfac;
+  double h, celvol;
+};
+
 // One thread per face.  The 12 per-face sums are added over the block (one
 // quantity per warp: four values per lane in thread order, then a shuffle
 // tree) into part[12 * block + q]; the last block to finish (a ticket
@@ -1504,13 +1585,36 @@ __device__ void geom_finish(const double* sm, double dens_ratio, double* __restr
 // lanes) and writes the body's scalars to out.  Each warp's dependent FP64
 // chain is a few additions per quantity: on this part an FP64 warp
 // instruction holds the pipe for about 64 cycles however few lanes run.
+// SUM = false leaves the last block's part to geom_sum_kernel, off the chain
+// to the next substep's tagging, which reads the faces only.
 constexpr int kGeomBlock = 128;
 static_assert(kGeomBlock == 128, "four values per lane in the block sums");
+__device__ void geom_total(const double* __restrict__ part, int blocks, double* tot, double dens_ratio,
+                           double* __restrict__ out) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int q = warp; q < 12; q += kGeomBlock / 32) {
+    double v = 0.0;
+    for (int b = lane; b < blocks; b += 32) v += __ldcg(part + 12 * (size_t)b + q);
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(FULL, v, off);
+    if (lane == 0) tot[q] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) geom_finish(tot, dens_ratio, out);
+}
+
+__global__ void __launch_bounds__(kGeomBlock) geom_sum_kernel(const double* __restrict__ part, int blocks,
+                                                             double dens_ratio, double* __restrict__ out) {
+  __shared__ double tot[12];
+  geom_total(part, blocks, tot, dens_ratio, out);
+}
+
+template <bool SUM>
 __global__ void __launch_bounds__(kGeomBlock)
 face_geom_kernel(int nf, const int* __restrict__ vof, const int* __restrict__ ghost, const double* __restrict__ x,
                  double* __restrict__ sur, double* __restrict__ nor, double* __restrict__ bar,
                  double* __restrict__ part /* 12 per block */, unsigned* __restrict__ ticket, double dens_ratio,
-                 double* __restrict__ out) {
+                 double* __restrict__ out, FaceNext N) {
   const unsigned FULL = 0xffffffffu;
   __shared__ double ws[12][kGeomBlock];
   __shared__ double tot[12];
@@ -1518,7 +1622,26 @@ face_geom_kernel(int nf, const int* __restrict__ vof, const int* __restrict__ gh
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   double pp[12];
   for (int q = 0; q < 12; ++q) pp[q] = 0.0;
-  if (t < nf && !ghost[t]) face_geom_one(t, vof, x, sur, nor, bar, pp);
+  const bool live = t < nf && !ghost[t];
+  if (live) face_geom_one(t, vof, x, sur, nor, bar, pp);
+  if (t < nf) {
+    const double b[3] = {bar[3 * t], bar[3 * t + 1], bar[3 * t + 2]};
+    if (N.face4) band_prep_one(t, N.nv, vof, x, b, N.g, N.face4, N.face_cell);
+    if (N.pind) {
+      const int* sv = N.saved + 7 * (size_t)t;
+      bool diff = sv[6] != ghost[t];
+      if (live) {
+        int p[6];
+        centroid_idx_one(N.g, b[0], b[1], b[2], p);
+        for (int q = 0; q < 6; ++q) {
+          N.pind[6 * t + q] = p[q];
+          diff = diff || sv[q] != p[q];
+        }
+      }
+      if (diff) atomicOr(N.dirty, 1);
+    }
+    if (N.cfac) N.cfac[t] = (sur[t] * N.h) / N.celvol;
+  }
   for (int q = 0; q < 12; ++q) ws[q][threadIdx.x] = pp[q];
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1527,22 +1650,15 @@ face_geom_kernel(int nf, const int* __restrict__ vof, const int* __restrict__ gh
     for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(FULL, v, off);
     if (lane == 0) part[12 * (size_t)blockIdx.x + q] = v;
   }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int q = warp; q < 12; q += kGeomBlock / 32) {
-    double v = 0.0;
-    for (int b = lane; b < (int)gridDim.x; b += 32) v += __ldcg(part + 12 * (size_t)b + q);
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(FULL, v, off);
-    if (lane == 0) tot[q] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    geom_finish(tot, dens_ratio, out);
-    *ticket = 0u;
+  if constexpr (SUM) {
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    geom_total(part, (int)gridDim.x, tot, dens_ratio, out);
+    if (threadIdx.x == 0) *ticket = 0u;
   }
 }
 
@@ -1606,11 +1722,6 @@ __global__ void tri_velocity_kernel(int nf, const int* __restrict__ ghost, const
   vel_tri[3 * t] = vel[0] + c0;
   vel_tri[3 * t + 1] = vel[1] + c1;
   vel_tri[3 * t + 2] = vel[2] + c2;
-}
-
-__global__ void cfac_kernel(int nf, const double* __restrict__ sur, double h, double celvol, double* __restrict__ cfac) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < nf) cfac[t] = (sur[t] * h) / celvol;
 }
 
 // ---------------------------------------------------------------------
@@ -1709,23 +1820,10 @@ __global__ void cm32_kernel(LagArgs A, float* __restrict__ cm32) {
 }
 
 __global__ void band_prep_kernel(TagArgs T, float4* __restrict__ face4, int4* __restrict__ face_cell) {
-  int f = blockIdx.x * blockDim.x + threadIdx.x;
-  const LagArgs& A = T.L;
-  if (f >= A.nf) return;
-  const Grid& g = A.g;
-  double pos[3] = {T.bar[3 * f], T.bar[3 * f + 1], T.bar[3 * f + 2]};
-  double V[3][3];
-  tri_verts(T, f, V[0], V[1], V[2]);
-  double r2 = 0.0;
-  for (int v = 0; v < 3; ++v) {
-    double dx = V[v][0] - pos[0], dy = V[v][1] - pos[1], dz = V[v][2] - pos[2];
-    r2 = fmax(r2, dx * dx + dy * dy + dz * dz);
-  }
-  float R = (float)sqrt(r2);
-  R = R * 1.000001f + 1e-30f;                                        // round the radius up
-  face4[f] = make_float4((float)pos[0], (float)pos[1], (float)pos[2], R);
-  // base cell of the band, as band_kernel derives it (genSDF.f90:151-153)
-  face_cell[f] = make_int4(ffloor(pos[0] * g.dx1) + 1, ffloor(pos[1] * g.dx2) + 1, ffloor(pos[2] * g.dx3) + 1, 0);
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= T.L.nf) return;
+  const double pos[3] = {T.bar[3 * f], T.bar[3 * f + 1], T.bar[3 * f + 2]};
+  band_prep_one(f, T.L.nv, T.vof, T.x, pos, T.L.g, face4, face_cell);
 }
 
 __device__ __forceinline__ float band_center_dist(const float* __restrict__ cm32, int clen, int coff, int ii, int jj,
@@ -1786,13 +1884,10 @@ __global__ void band_ub_kernel(TagArgs T, const float4* __restrict__ face4, cons
 // a cell's minimum nor win it); pass 0: distance (stored) and the minimum
 // per cell, pass 1: the earliest triangle at that distance, pass 2: the
 // winner writes the signed distance and the VOF
-__global__ void band_kernel(TagArgs T, int pass, unsigned long long* __restrict__ sdf_bits, int* __restrict__ winner,
-                            double* __restrict__ vofp, double* __restrict__ dist_buf, const int4* __restrict__ face_cell,
-                            const int* __restrict__ list, const int* __restrict__ count) {
-  long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= *count) return;
-  gid = list[gid];
-  int f = (int)(gid / 125), q = (int)(gid % 125);
+__device__ __forceinline__ void band_pair(const TagArgs& T, int pass, unsigned long long* __restrict__ sdf_bits,
+                                          int* __restrict__ winner, double* __restrict__ vofp,
+                                          double* __restrict__ dist_buf, const int4* __restrict__ face_cell, int gid) {
+  int f = gid / 125, q = gid % 125;
   const LagArgs& A = T.L;
   if (f >= A.nf || T.ghost[f]) return;
   const Grid& g = A.g;
@@ -1830,6 +1925,16 @@ __global__ void band_kernel(TagArgs T, int pass, unsigned long long* __restrict_
   vofp[c0] = vof;
   sdf_bits[c0] = (unsigned long long)__double_as_longlong(sgnd);
 }
+
+constexpr int kBandBlocks = 152 * 24;
+__global__ void band_kernel(TagArgs T, int pass, unsigned long long* __restrict__ sdf_bits, int* __restrict__ winner,
+                            double* __restrict__ vofp, double* __restrict__ dist_buf, const int4* __restrict__ face_cell,
+                            const int* __restrict__ list, const int* __restrict__ count) {
+  const int n = *count;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+    band_pair(T, pass, sdf_bits, winner, vofp, dist_buf, face_cell, list[t]);
+}
+
 
 // initial full tagging: one thread per cell of the bounding box
 __device__ bool ray_tri(const double C[3], const double Q[3], const double V0[3], const double V1[3],
@@ -2067,6 +2172,7 @@ static bool ensure_lag_buffers(Ctx* c) {
     cudaMemsetAsync(s->bitmap, 0, sizeof(unsigned) * (size_t)s->plan_words, c->stream);
     cudaMemsetAsync(s->saved, 0xff, sizeof(int) * 7 * (size_t)std::max(1, c->maxnf), c->stream);
     cudaMemsetAsync(s->nruns, 0, sizeof(int) * 2, c->stream);
+    cudaMemsetAsync(s->dirty, 0, sizeof(int), c->stream);
   }
   return true;
 }
@@ -2094,20 +2200,25 @@ bool validate_mesh(Ctx* c) {
 }
 
 // (Re)build the merged scatter plan when the cage centres changed.
+// checked: the geometry pass of the substep before compared them already
+// (FaceNext; no parameter block carries a request there).
 // dp: inside the fused step, the substep's parameter block, whose
 // force_plan carries a rebuild request (lagr_take_plan_request); nullptr
 // (drop-ins): the pending request is applied now.  A request raised inside
 // a step (a remesh, which runs without a step graph) is applied now too.
-static void update_plan(Ctx* c, const StepParams* dp) {
+static void update_plan(Ctx* c, const StepParams* dp, bool checked) {
   LagState* s = lag_of(c);
   const int nf = c->maxnf, words = s->plan_words;
   const unsigned eb = div_up(108 * (size_t)nf, 256), tiles = div_up(words, kPlanTile);
-  cudaMemsetAsync(s->dirty, s->force_rebuild ? 1 : 0, sizeof(int), c->stream);   // non-zero: dirty
-  s->force_rebuild = false;
   const int* pind = M<int>(c, MIBM_M_PIND);
   const int* ghost = M<int>(c, MIBM_M_GHOST_FACE);
-  { MIBM_PROF(c, "plan_check");
-    plan_check_kernel<<<div_up(nf, 256), 256, 0, c->stream>>>(nf, pind, ghost, s->saved, s->dirty, dp); }
+  if (s->force_rebuild) cudaMemsetAsync(s->dirty, 1, sizeof(int), c->stream);   // non-zero: dirty
+  s->force_rebuild = false;
+  if (!checked) {
+    MIBM_PROF(c, "plan_check");
+    plan_check_kernel<<<div_up(nf, 256), 256, 0, c->stream>>>(nf, pind, ghost, s->saved, s->dirty, dp);
+    ++c->launches;
+  }
   { MIBM_PROF(c, "plan_mark");
     plan_mark_kernel<<<eb, 256, 0, c->stream>>>(c->g, nf, pind, ghost, s->dirty, s->bitmap); }
   { MIBM_PROF(c, "plan_runs");
@@ -2124,7 +2235,8 @@ static void update_plan(Ctx* c, const StepParams* dp) {
   { MIBM_PROF(c, "plan_order");
     plan_order_kernel<<<std::min<unsigned>(eb, kScatterBlocks), 256, 0, c->stream>>>(
         s->dirty, s->nruns, s->run_key, s->run_off, s->run_cnt, s->entry, s->src, s->bitmap); }
-  c->launches += 8;
+  cudaMemsetAsync(s->dirty, 0, sizeof(int), c->stream);
+  c->launches += 7;
   MIBM_LAUNCH_CHECK(c, "scatter plan");
 }
 
@@ -2149,7 +2261,7 @@ static void force_coefficients(Ctx* c) {
   F.vel_tri = M<double>(c, MIBM_M_VEL_TRI); F.cfac = M<double>(c, MIBM_M_CFAC);
   F.pind = M<int>(c, MIBM_M_PIND); F.ghost = M<int>(c, MIBM_M_GHOST_FACE);
   { MIBM_PROF(c, "force_coef");
-    force_coef_kernel<<<div_up(4 * (size_t)c->maxnf, 128), 128, 0, c->stream>>>(c->g, c->maxnf, F, c->S(MIBM_S_TMELT),
+    force_coef_kernel<<<div_up(4 * (size_t)c->maxnf, kLagBlock), kLagBlock, 0, c->stream>>>(c->g, c->maxnf, F, c->S(MIBM_S_TMELT),
                                                                                   c->tri_coef); }
   ++c->launches;
 }
@@ -2171,7 +2283,7 @@ static void scatter(Ctx* c, bool into_fields, int lo, int hi, bool record, float
 void lagr_find_centroid_indices(Ctx* c) {
   if (c->maxnf == 0) return;
   { MIBM_PROF(c, "centroid_idx");
-    centroid_idx_kernel<<<div_up(c->maxnf, 128), 128, 0, c->stream>>>(
+    centroid_idx_kernel<<<div_up(c->maxnf, kLagBlock), kLagBlock, 0, c->stream>>>(
         lag_args(c), M<double>(c, MIBM_M_TRI_BAR), M<int>(c, MIBM_M_GHOST_FACE), M<int>(c, MIBM_M_PIND)); }
   ++c->launches;
   MIBM_LAUNCH_CHECK(c, "findCentroidIndices");
@@ -2180,7 +2292,7 @@ void lagr_find_centroid_indices(Ctx* c) {
 static void mls_weight_launch(Ctx* c) {
   if (c->precision == 1) {
     { MIBM_PROF(c, "mls_weight_sep");
-      mls_weight_sep_kernel<<<div_up(4 * (size_t)c->maxnf, 128), 128, 0, c->stream>>>(
+      mls_weight_sep_kernel<<<div_up(4 * (size_t)c->maxnf, kLagBlock), kLagBlock, 0, c->stream>>>(
           lag_args(c), M<double>(c, MIBM_M_TRI_BAR), M<int>(c, MIBM_M_GHOST_FACE), M<int>(c, MIBM_M_PIND),
           M<double>(c, MIBM_M_PTXAB_Q1), M<double>(c, MIBM_M_PTXAB_Q2), M<double>(c, MIBM_M_PTXAB_Q3),
           M<double>(c, MIBM_M_PTXAB_TEMP), c->dflag); }
@@ -2188,7 +2300,7 @@ static void mls_weight_launch(Ctx* c) {
     return;
   }
   { MIBM_PROF(c, "mls_weight");
-    mls_weight_kernel<<<div_up(4 * (size_t)c->maxnf, 64), 64, 0, c->stream>>>(
+    mls_weight_kernel<<<div_up(4 * (size_t)c->maxnf, kLagBlock), kLagBlock, 0, c->stream>>>(
         lag_args(c), M<double>(c, MIBM_M_TRI_BAR), M<int>(c, MIBM_M_GHOST_FACE), M<int>(c, MIBM_M_PIND),
         M<double>(c, MIBM_M_PTXAB_Q1), M<double>(c, MIBM_M_PTXAB_Q2), M<double>(c, MIBM_M_PTXAB_Q3),
         M<double>(c, MIBM_M_PTXAB_TEMP), c->dflag); }
@@ -2206,7 +2318,7 @@ void lagr_mls_force(Ctx* c, const StepParams*, bool) {
   if (c->maxnf == 0) return;
   if (!ensure_lag_buffers(c)) return;
   force_coefficients(c);
-  update_plan(c, nullptr);
+  update_plan(c, nullptr, false);
   scatter(c, false, 0, 4, false);
   MIBM_LAUNCH_CHECK(c, "mlsForce");
 }
@@ -2230,7 +2342,7 @@ void lagr_tempforce(Ctx* c) { k_tempforce_apply(c); }
 void lagr_find_probe_indices(Ctx* c) {
   if (c->maxnf == 0) return;
   { MIBM_PROF(c, "probe_idx");
-    probe_idx_kernel<<<div_up(c->maxnf, 128), 128, 0, c->stream>>>(
+    probe_idx_kernel<<<div_up(c->maxnf, kLagBlock), kLagBlock, 0, c->stream>>>(
         lag_args(c), M<double>(c, MIBM_M_TRI_BAR), M<double>(c, MIBM_M_TRI_NOR), M<int>(c, MIBM_M_GHOST_FACE),
         c->S(MIBM_S_H_EULERIAN), M<int>(c, MIBM_M_PIND)); }
   ++c->launches;
@@ -2250,38 +2362,56 @@ void lagr_find_probe_indices(Ctx* c) {
 // reference's to it, at a quarter of its FP64 operations.
 static bool literal_mls(Ctx* c) { return c->precision == 0 && c->I(MIBM_I_IMLSSTR) != 1; }
 
-static void heat_flux_launch(Ctx* c) {
+// fused: without the probe indices in pind, and without the face-to-vertex
+// sums (melt_vert_kernel takes them)
+static void heat_flux_launch(Ctx* c, bool fused) {
   LagState* s = lag_of(c);
+  const int* pind = fused ? nullptr : M<int>(c, MIBM_M_PIND);
   { MIBM_PROF(c, "heat_flux");
     if (literal_mls(c))
       heat_flux_lit_kernel<<<div_up(2 * (size_t)c->maxnf, kHfProbes), 4 * kHfProbes, 0, c->stream>>>(
           lag_args(c), c->df[MIBM_F_TEMP], M<double>(c, MIBM_M_TRI_BAR), M<double>(c, MIBM_M_TRI_NOR),
-          M<int>(c, MIBM_M_GHOST_FACE), M<int>(c, MIBM_M_PIND), c->S(MIBM_S_H_EULERIAN), c->S(MIBM_S_PEC),
+          M<int>(c, MIBM_M_GHOST_FACE), pind, c->S(MIBM_S_H_EULERIAN), c->S(MIBM_S_PEC),
           M<double>(c, MIBM_M_QW_O), M<double>(c, MIBM_M_QW_I), c->dflag);
     else
-      heat_flux_sep_kernel<<<div_up(2 * (size_t)c->maxnf, 128), 128, 0, c->stream>>>(
+      heat_flux_sep_kernel<<<div_up(2 * (size_t)c->maxnf, kLagBlock), kLagBlock, 0, c->stream>>>(
           lag_args(c), c->df[MIBM_F_TEMP], M<double>(c, MIBM_M_TRI_BAR), M<double>(c, MIBM_M_TRI_NOR),
-          M<int>(c, MIBM_M_GHOST_FACE), M<int>(c, MIBM_M_PIND), c->S(MIBM_S_H_EULERIAN), c->S(MIBM_S_PEC),
+          M<int>(c, MIBM_M_GHOST_FACE), pind, c->S(MIBM_S_H_EULERIAN), c->S(MIBM_S_PEC),
           M<double>(c, MIBM_M_QW_O), M<double>(c, MIBM_M_QW_I), c->dflag); }
+  ++c->launches;
+  if (fused) return;
   { MIBM_PROF(c, "face_to_vert");
-    face_to_vert_kernel<<<div_up(c->maxnv, 128), 128, 0, c->stream>>>(
+    face_to_vert_kernel<<<div_up(c->maxnv, kLagBlock), kLagBlock, 0, c->stream>>>(
         c->maxnv, s->adj_off, s->adj_face, M<double>(c, MIBM_M_SUR), M<double>(c, MIBM_M_AVERT),
         M<double>(c, MIBM_M_QW_O), M<double>(c, MIBM_M_QW_I), M<double>(c, MIBM_M_QW_OVERT),
         M<double>(c, MIBM_M_QW_IVERT)); }
-  c->launches += 2;
+  ++c->launches;
+}
+
+static void melt_vert_launch(Ctx* c, const StepParams* dp) {
+  LagState* s = lag_of(c);
+  { MIBM_PROF(c, "melt_vert");
+    melt_vert_kernel<<<div_up(c->maxnv, kLagBlock), kLagBlock, 0, c->stream>>>(
+        c->maxnv, s->adj_off, s->adj_face, M<double>(c, MIBM_M_SUR), M<double>(c, MIBM_M_AVERT),
+        M<double>(c, MIBM_M_QW_O), M<double>(c, MIBM_M_QW_I), M<double>(c, MIBM_M_QW_OVERT),
+        M<double>(c, MIBM_M_QW_IVERT), M<int>(c, MIBM_M_GHOST_VERT), M<double>(c, MIBM_M_VERT_NOR),
+        c->S(MIBM_S_CPLIQUID) / c->S(MIBM_S_LATHEAT), dp, M<double>(c, MIBM_M_VMELT), M<double>(c, MIBM_M_VMELT_M1),
+        M<double>(c, MIBM_M_XYZV)); }
+  ++c->launches;
+  s->weights_valid = false;
 }
 
 void lagr_heat_flux(Ctx* c) {
   if (c->maxnf == 0) return;
   if (!ensure_adjacency(c)) return;
-  heat_flux_launch(c);
+  heat_flux_launch(c, false);
   if (MIBM_LAUNCH_CHECK(c, "mls_heatFlux")) check_flag(c, "mls_heatFlux");
 }
 
 void lagr_stefan(Ctx* c, const StepParams* dp) {
   if (c->maxnv == 0) return;
   { MIBM_PROF(c, "stefan");
-    stefan_kernel<<<div_up(c->maxnv, 128), 128, 0, c->stream>>>(
+    stefan_kernel<<<div_up(c->maxnv, kLagBlock), kLagBlock, 0, c->stream>>>(
         c->maxnv, M<int>(c, MIBM_M_GHOST_VERT), M<double>(c, MIBM_M_VERT_NOR), M<double>(c, MIBM_M_QW_OVERT),
         M<double>(c, MIBM_M_QW_IVERT), c->S(MIBM_S_CPLIQUID) / c->S(MIBM_S_LATHEAT), dp, M<double>(c, MIBM_M_VMELT),
         M<double>(c, MIBM_M_VMELT_M1), M<double>(c, MIBM_M_XYZV)); }
@@ -2295,44 +2425,62 @@ void lagr_stefan(Ctx* c, const StepParams* dp) {
 // the Newton-Euler update (particle.f90:108-117: centroids, normals,
 // volume, centre of mass and inertia tensor of the melted body); it also
 // rewrites `sur`, which nothing reads before the full refresh recomputes it.
-// kGeomFaces: the per-face pass alone (areas, normals, centroids and the
-// block sums); kGeomRest: what follows it (vertex areas and normals, the
-// body's sums, edge lengths, skewness, cfac)
-enum GeomPart { kGeomAll, kGeomFaces, kGeomRest };
+static FaceNext face_next(Ctx* c) {
+  FaceNext N{};
+  N.g = c->g;
+  N.nv = c->maxnv;
+  N.h = c->S(MIBM_S_H_EULERIAN);
+  N.celvol = c->S(MIBM_S_CELVOL);
+  return N;
+}
 
-static void geometry_launch(Ctx* c, bool imelt, bool body_only = false, GeomPart part = kGeomAll) {
+static void vert_geom_launch(Ctx* c) {
   LagState* s = lag_of(c);
-  if (part != kGeomRest) {
-    { MIBM_PROF(c, "face_geom");
-      face_geom_kernel<<<div_up(c->maxnf, kGeomBlock), kGeomBlock, 0, c->stream>>>(
-          c->maxnf, M<int>(c, MIBM_M_VERT_OF_FACE), M<int>(c, MIBM_M_GHOST_FACE), M<double>(c, MIBM_M_XYZV),
-          M<double>(c, MIBM_M_SUR), M<double>(c, MIBM_M_TRI_NOR), M<double>(c, MIBM_M_TRI_BAR), s->face_part,
-          s->geom_ticket, c->S(MIBM_S_DENS_RATIO), s->geom_out); }
-    ++c->launches;
-  }
-  if (body_only || part == kGeomFaces) return;
   { MIBM_PROF(c, "vert_geom");
-    vert_geom_kernel<<<div_up(c->maxnv, 128), 128, 0, c->stream>>>(
+    vert_geom_kernel<<<div_up(c->maxnv, kLagBlock), kLagBlock, 0, c->stream>>>(
         c->maxnv, s->adj_off, s->adj_face, M<int>(c, MIBM_M_GHOST_VERT), M<double>(c, MIBM_M_SUR),
         M<double>(c, MIBM_M_TRI_NOR), M<double>(c, MIBM_M_AVERT), M<double>(c, MIBM_M_VERT_NOR)); }
-  c->launches += 1;
-  if (c->maxne > 0) {           // calculate_eLengths, calculate_skewness (particle.f90:173-176)
-    MIBM_PROF(c, "edges");
-    elength_kernel<<<div_up(c->maxne, 128), 128, 0, c->stream>>>(
-        c->maxne, M<int>(c, MIBM_M_VERT_OF_EDGE), M<int>(c, MIBM_M_GHOST_EDGE), M<double>(c, MIBM_M_XYZV), 0.0,
-        M<double>(c, MIBM_M_ELENGTHS), nullptr);
-    skewness_kernel<<<div_up(c->maxnf, 128), 128, 0, c->stream>>>(
-        c->maxnf, M<int>(c, MIBM_M_EDGE_OF_FACE), M<int>(c, MIBM_M_GHOST_FACE), M<double>(c, MIBM_M_ELENGTHS),
-        M<double>(c, MIBM_M_SUR), M<double>(c, MIBM_M_SKEWNESS));
-    c->launches += 2;
-  }
-  if (imelt) {
-    { MIBM_PROF(c, "cfac");
-      cfac_kernel<<<div_up(c->maxnf, 128), 128, 0, c->stream>>>(c->maxnf, M<double>(c, MIBM_M_SUR),
-                                                                c->S(MIBM_S_H_EULERIAN), c->S(MIBM_S_CELVOL),
-                                                                M<double>(c, MIBM_M_CFAC)); }
-    ++c->launches;
-  }
+  ++c->launches;
+}
+
+static void edges_launch(Ctx* c) {   // calculate_eLengths, calculate_skewness (particle.f90:173-176)
+  if (c->maxne <= 0) return;
+  MIBM_PROF(c, "edges");
+  elength_kernel<<<div_up(c->maxne, kLagBlock), kLagBlock, 0, c->stream>>>(
+      c->maxne, M<int>(c, MIBM_M_VERT_OF_EDGE), M<int>(c, MIBM_M_GHOST_EDGE), M<double>(c, MIBM_M_XYZV), 0.0,
+      M<double>(c, MIBM_M_ELENGTHS), nullptr);
+  skewness_kernel<<<div_up(c->maxnf, kLagBlock), kLagBlock, 0, c->stream>>>(
+      c->maxnf, M<int>(c, MIBM_M_EDGE_OF_FACE), M<int>(c, MIBM_M_GHOST_FACE), M<double>(c, MIBM_M_ELENGTHS),
+      M<double>(c, MIBM_M_SUR), M<double>(c, MIBM_M_SKEWNESS));
+  c->launches += 2;
+}
+
+static void face_geom_launch(Ctx* c, const FaceNext& N, bool sum) {
+  LagState* s = lag_of(c);
+  { MIBM_PROF(c, "face_geom");
+    auto kern = sum ? face_geom_kernel<true> : face_geom_kernel<false>;
+    kern<<<div_up(c->maxnf, kGeomBlock), kGeomBlock, 0, c->stream>>>(
+        c->maxnf, M<int>(c, MIBM_M_VERT_OF_FACE), M<int>(c, MIBM_M_GHOST_FACE), M<double>(c, MIBM_M_XYZV),
+        M<double>(c, MIBM_M_SUR), M<double>(c, MIBM_M_TRI_NOR), M<double>(c, MIBM_M_TRI_BAR), s->face_part,
+        s->geom_ticket, c->S(MIBM_S_DENS_RATIO), s->geom_out, N); }
+  ++c->launches;
+}
+
+static void geom_sum_launch(Ctx* c) {
+  LagState* s = lag_of(c);
+  { MIBM_PROF(c, "geom_sum");
+    geom_sum_kernel<<<1, kGeomBlock, 0, c->stream>>>(s->face_part, (int)div_up(c->maxnf, kGeomBlock),
+                                                     c->S(MIBM_S_DENS_RATIO), s->geom_out); }
+  ++c->launches;
+}
+
+static void geometry_launch(Ctx* c, bool imelt, bool body_only = false) {
+  FaceNext N = face_next(c);
+  if (imelt && !body_only) N.cfac = M<double>(c, MIBM_M_CFAC);
+  face_geom_launch(c, N, true);
+  if (body_only) return;
+  vert_geom_launch(c);
+  edges_launch(c);
 }
 
 // Surface, Volume and centre of mass to the registered host scalars
@@ -2401,45 +2549,61 @@ void lagr_geometry_refresh(Ctx* c, bool imelt) {
 // bits) and leaves the signed distances there: no copy pass
 static unsigned long long* sdf_bits_of(Ctx* c) { return reinterpret_cast<unsigned long long*>(c->df[MIBM_F_SDF]); }
 
-void lagr_tag_narrow_band(Ctx* c) {
-  if (c->maxnf == 0) return;
+static bool ensure_band(Ctx* c) {
   LagState* s = lag_of(c);
-  if (!s->winner && !cuda_ok(c, cudaMalloc(&s->winner, sizeof(int) * c->g.cells), "band")) return;
-  unsigned long long* const sdf_bits = sdf_bits_of(c);
-  TagArgs T;
-  T.L = lag_args(c);
+  if (!s->winner && !cuda_ok(c, cudaMalloc(&s->winner, sizeof(int) * c->g.cells), "band")) return false;
   if (!s->dist_buf) {
+    const LagArgs L = lag_args(c);
     bool ok = cuda_ok(c, cudaMalloc(&s->dist_buf, sizeof(double) * 125 * (size_t)c->maxnf), "band") &&
               cuda_ok(c, cudaMalloc(&s->band_ub, sizeof(unsigned) * c->g.cells), "band") &&
               cuda_ok(c, cudaMalloc(&s->band_list, sizeof(int) * 125 * (size_t)c->maxnf), "band") &&
               cuda_ok(c, cudaMalloc(&s->band_count, sizeof(int)), "band") &&
               cuda_ok(c, cudaMalloc(&s->face4, sizeof(float4) * (size_t)c->maxnf), "band") &&
               cuda_ok(c, cudaMalloc(&s->face_cell, sizeof(int4) * (size_t)c->maxnf), "band") &&
-              cuda_ok(c, cudaMalloc(&s->cm32, sizeof(float) * 3 * (size_t)T.L.clen), "band");
-    if (!ok) return;
-    cm32_kernel<<<div_up(T.L.clen, 256), 256, 0, c->stream>>>(T.L, s->cm32);
+              cuda_ok(c, cudaMalloc(&s->cm32, sizeof(float) * 3 * (size_t)L.clen), "band");
+    if (!ok) return false;
+    cm32_kernel<<<div_up(L.clen, 256), 256, 0, c->stream>>>(L, s->cm32);
     ++c->launches;
   }
+  return true;
+}
+
+static void band_reset(Ctx* c) {
+  LagState* s = lag_of(c);
+  { MIBM_PROF(c, "sdf_reset");
+    sdf_reset_kernel<<<div_up(c->g.cells, 256), 256, 0, c->stream>>>(c->g, sdf_bits_of(c), s->winner, s->band_ub); }
+  cudaMemsetAsync(s->band_count, 0, sizeof(int), c->stream);
+  ++c->launches;
+}
+
+// prepped (fused step): band_reset has run on this stream since the last
+// tagging, and the geometry pass has left the faces' bounds (FaceNext)
+static void tag_narrow_band(Ctx* c, bool prepped) {
+  if (c->maxnf == 0 || !ensure_band(c)) return;
+  LagState* s = lag_of(c);
+  unsigned long long* const sdf_bits = sdf_bits_of(c);
+  TagArgs T;
+  T.L = lag_args(c);
   T.x = M<double>(c, MIBM_M_XYZV); T.vof = M<int>(c, MIBM_M_VERT_OF_FACE); T.ghost = M<int>(c, MIBM_M_GHOST_FACE);
   T.bar = M<double>(c, MIBM_M_TRI_BAR); T.nor = M<double>(c, MIBM_M_TRI_NOR);
-  { MIBM_PROF(c, "sdf_reset");
-    sdf_reset_kernel<<<div_up(c->g.cells, 256), 256, 0, c->stream>>>(c->g, sdf_bits, s->winner, s->band_ub); }
+  if (!prepped) band_reset(c);
   size_t nthr = (size_t)c->maxnf * 125;
   { MIBM_PROF(c, "band_bound");
-    band_prep_kernel<<<div_up(c->maxnf, 128), 128, 0, c->stream>>>(T, s->face4, s->face_cell);
+    if (!prepped) band_prep_kernel<<<div_up(c->maxnf, kLagBlock), kLagBlock, 0, c->stream>>>(T, s->face4, s->face_cell);
     band_ub_kernel<<<div_up(nthr, 128), 128, 0, c->stream>>>(T, s->face4, s->face_cell, s->cm32, s->band_ub);
-    cudaMemsetAsync(s->band_count, 0, sizeof(int), c->stream);
     band_select_kernel<<<div_up(nthr, 128), 128, 0, c->stream>>>(T, s->face4, s->face_cell, s->cm32, s->band_ub,
                                                                   s->dist_buf, s->band_list, s->band_count); }
   for (int pass = 0; pass < 3; ++pass) {
     MIBM_PROF(c, "band");
-    band_kernel<<<div_up(nthr, 128), 128, 0, c->stream>>>(T, pass, sdf_bits, s->winner, c->df[MIBM_F_VOFP],
+    band_kernel<<<(unsigned)std::min<size_t>(div_up(nthr, kLagBlock), kBandBlocks), kLagBlock, 0, c->stream>>>(T, pass, sdf_bits, s->winner, c->df[MIBM_F_VOFP],
                                                            s->dist_buf, s->face_cell, s->band_list, s->band_count);
   }
-  c->launches += 7;
+  c->launches += prepped ? 5 : 6;
   k_interp_vof(c);
   MIBM_LAUNCH_CHECK(c, "narrowBandTagging");
 }
+
+void lagr_tag_narrow_band(Ctx* c) { tag_narrow_band(c, false); }
 
 void lagr_tag_initial(Ctx* c) {
   if (c->maxnf == 0) return;
@@ -2498,7 +2662,7 @@ static bool remesh_check(Ctx* c) {
   if (!s->rm_flag && !cuda_ok(c, cudaMalloc(&s->rm_flag, sizeof(int)), "remesh")) return false;
   cudaMemsetAsync(s->rm_flag, 0, sizeof(int), c->stream);
   { MIBM_PROF(c, "edges");
-    elength_kernel<<<div_up(c->maxne, 128), 128, 0, c->stream>>>(
+    elength_kernel<<<div_up(c->maxne, kLagBlock), kLagBlock, 0, c->stream>>>(
         c->maxne, M<int>(c, MIBM_M_VERT_OF_EDGE), M<int>(c, MIBM_M_GHOST_EDGE), M<double>(c, MIBM_M_XYZV),
         c->S(MIBM_S_E_THRESH), M<double>(c, MIBM_M_ELENGTHS), s->rm_flag); }
   ++c->launches;
@@ -2612,7 +2776,10 @@ void lagr_particle(Ctx* c, const StepParams* dp) {
 // final once that substep's particle is done): for substeps 1 and 2, and for
 // substep 0 of the next step (slot 3: no parameter block, the host's plan
 // rebuild requests invalidate it instead).
-void lagr_substep_prologue(Ctx* c, int slot) {
+// prepped: the geometry pass has left the cage indices and the band's bounds,
+// and band_reset has run on the tagging's stream (lagr_particle_fused, whose
+// geometry refresh is finished here)
+static void substep_prologue(Ctx* c, int slot, bool prepped) {
   if (c->I(MIBM_I_IMLSFOR) != 1 || c->maxnf == 0) return;
   // the tagging (VOF fields) and the cage indices, weights and plan read the
   // same geometry and write disjoint buffers: the tagging goes to a stream of
@@ -2621,27 +2788,27 @@ void lagr_substep_prologue(Ctx* c, int slot) {
   c->geom_join_tag = split;
   if (split) {
     cudaEventRecord(c->ev_tfork, c->stream);
-    cudaStreamWaitEvent(c->side2, c->ev_tfork, 0);
+    wait_event(c, c->side2, c->ev_tfork);
     std::swap(c->stream, c->side2);
-    lagr_tag_narrow_band(c);
+    tag_narrow_band(c, prepped);
     cudaEventRecord(c->ev_tjoin, c->stream);
     std::swap(c->stream, c->side2);
   } else if (!c->I(MIBM_I_STATIONARY)) {
     lagr_tag_narrow_band(c);
   }
   if (!ensure_adjacency(c) || !ensure_lag_buffers(c)) {
-    if (split) cudaStreamWaitEvent(c->stream, c->ev_tjoin, 0);
+    if (split) wait_event(c, c->stream, c->ev_tjoin);
     return;
   }
   LagState* s = lag_of(c);
   bool stationary = c->I(MIBM_I_STATIONARY) != 0;
-  lagr_find_centroid_indices(c);
+  if (!prepped) lagr_find_centroid_indices(c);
   // the MLS weights and the scatter plan both read the cage indices and
   // nothing the other writes: the weights go to a third stream
   const bool wsplit = split && c->side3;
   if (wsplit) {
     cudaEventRecord(c->ev_wfork, c->stream);
-    cudaStreamWaitEvent(c->side3, c->ev_wfork, 0);
+    wait_event(c, c->side3, c->ev_wfork);
     std::swap(c->stream, c->side3);
   }
   if (!(stationary && s->weights_valid)) {
@@ -2653,10 +2820,16 @@ void lagr_substep_prologue(Ctx* c, int slot) {
     cudaEventRecord(c->ev_wjoin, c->stream);
     std::swap(c->stream, c->side3);
   }
-  update_plan(c, slot < 3 ? c->dparams + slot : nullptr);
-  if (wsplit) cudaStreamWaitEvent(c->stream, c->ev_wjoin, 0);
-  if (split) cudaStreamWaitEvent(c->stream, c->ev_tjoin, 0);
+  update_plan(c, slot < 3 ? c->dparams + slot : nullptr, prepped);
+  if (prepped) {                 // the rest of the geometry refresh: nothing of the next substep's chain needs it
+    vert_geom_launch(c);
+    edges_launch(c);
+  }
+  if (wsplit) wait_event(c, c->stream, c->ev_wjoin);
+  if (split) wait_event(c, c->stream, c->ev_tjoin);
 }
+
+void lagr_substep_prologue(Ctx* c, int slot) { substep_prologue(c, slot, false); }
 
 // The side stream takes the second half of particle (and the work that
 // follows it) unless the host's remesher may be needed mid-way or kernels
@@ -2676,12 +2849,30 @@ void lagr_loads_early(Ctx* c, const StepParams* dp) {
   if (!lagr_fork_enabled(c)) return;
   if (!ensure_adjacency(c) || !ensure_lag_buffers(c)) return;
   cudaEventRecord(c->ev_lfork, c->stream);
-  cudaStreamWaitEvent(c->side, c->ev_lfork, 0);
+  wait_event(c, c->side, c->ev_lfork);
   std::swap(c->stream, c->side);
   struct_loads_launch(c, dp, false);
   cudaEventRecord(c->ev_ldone, c->stream);
   std::swap(c->stream, c->side);
   c->loads_pending = true;
+}
+
+// The heat flux reads the solved temperature (before the temperature forcing)
+// and the geometry, nothing of the velocity forcing: the fused step starts it
+// on the tagging's stream, idle at this point, once T is solved (called with
+// the context's stream the one that solves T).  Same conditions as above.
+void lagr_heat_early(Ctx* c) {
+  c->heat_pending = false;
+  if (c->I(MIBM_I_IMLSFOR) != 1 || c->maxnf == 0 || c->I(MIBM_I_IMELT) != 1) return;
+  if (!lagr_fork_enabled(c) || !c->side2) return;
+  if (!ensure_adjacency(c) || !ensure_lag_buffers(c)) return;
+  cudaEventRecord(c->ev_hfork, c->stream);
+  wait_event(c, c->side2, c->ev_hfork);
+  std::swap(c->stream, c->side2);
+  heat_flux_launch(c, true);
+  cudaEventRecord(c->ev_hflux, c->stream);
+  std::swap(c->stream, c->side2);
+  c->heat_pending = true;
 }
 
 const double* lagr_particle_fused(Ctx* c, const StepParams* dp, float* m32, StepParams* next,
@@ -2694,7 +2885,7 @@ const double* lagr_particle_fused(Ctx* c, const StepParams* dp, float* m32, Step
   bool str = c->I(MIBM_I_IMLSSTR) == 1;
   if (str) {                                 // reads the unforced u, v, w and p
     if (c->loads_pending) {
-      cudaStreamWaitEvent(c->stream, c->ev_ldone, 0);
+      wait_event(c, c->stream, c->ev_ldone);
       c->loads_pending = false;
     } else {
       struct_loads_launch(c, dp, false);
@@ -2714,34 +2905,61 @@ const double* lagr_particle_fused(Ctx* c, const StepParams* dp, float* m32, Step
   const bool fork = lagr_fork_enabled(c);
   if (fork) {
     cudaEventRecord(c->ev_fork, c->stream);
-    cudaStreamWaitEvent(c->side, c->ev_fork, 0);
+    wait_event(c, c->side, c->ev_fork);
     std::swap(c->stream, c->side);
   }
+  const bool next_here = fork && next_prologue >= 0 && c->side3;     // the next substep's geometry work follows
+  const bool tag_next = next_here && c->side2 && !c->I(MIBM_I_STATIONARY) && ensure_band(c);
   bool imelt = c->I(MIBM_I_IMELT) == 1;
-  if (imelt) {
-    lagr_find_probe_indices(c);
-    heat_flux_launch(c);
+  if (imelt && !c->heat_pending) heat_flux_launch(c, true);
+  // the temperature forcing (after the heat flux, which reads the unforced
+  // temperature) and the reset of the narrow band need nothing of what
+  // follows here: they go to the tagging's stream, off the chain to the next
+  // substep
+  const bool tside = fork && c->side2;
+  if (tside) {
+    if (!c->heat_pending) cudaEventRecord(c->ev_hfork, c->stream);
+    wait_event(c, c->side2, c->heat_pending ? c->ev_fork : c->ev_hfork);
+    std::swap(c->stream, c->side2);
   }
   scatter(c, true, 3, 4, false, m32);
-  if (imelt) lagr_stefan(c, dp);
+  if (tside) {
+    if (tag_next) band_reset(c);
+    cudaEventRecord(c->ev_tscat, c->stream);
+    std::swap(c->stream, c->side2);
+    c->tscat_pending = true;
+  }
+  if (c->heat_pending) {
+    wait_event(c, c->stream, c->ev_hflux);
+    c->heat_pending = false;
+  }
+  if (imelt) melt_vert_launch(c, dp);
   if (str) motion_launch(c, dp);
   bool remeshed = !fork && lagr_remesh_active(c) && remesh_check(c);
-  if (c->status == MIBM_OK && fork && next_prologue >= 0 && c->side3) {
+  if (c->status == MIBM_OK && next_here) {
     // the next substep's geometry-only work needs the new face centroids and
     // normals alone: it starts after the per-face pass, while a third stream
-    // finishes the refresh and publishes the moved body (ev_pub)
-    geometry_launch(c, imelt, false, kGeomFaces);
+    // finishes the body's sums and publishes the moved body (ev_pub)
+    FaceNext N = face_next(c);
+    N.pind = M<int>(c, MIBM_M_PIND);
+    N.saved = s->saved;
+    N.dirty = s->dirty;
+    if (tag_next) { N.face4 = s->face4; N.face_cell = s->face_cell; }
+    if (imelt) N.cfac = M<double>(c, MIBM_M_CFAC);
+    face_geom_launch(c, N, false);
     cudaEventRecord(c->ev_gfork, c->stream);
-    cudaStreamWaitEvent(c->side3, c->ev_gfork, 0);
+    wait_event(c, c->side3, c->ev_gfork);
     std::swap(c->stream, c->side3);
-    geometry_launch(c, imelt, false, kGeomRest);
+    geom_sum_launch(c);
     if (str) k_rigid_publish(c, s->geom_out, next);
     cudaEventRecord(c->ev_pub, c->stream);
     std::swap(c->stream, c->side3);
     c->geom_join_tag = false;
-    lagr_substep_prologue(c, next_prologue);
+    // the temperature forcing reads the plan and the weights of this substep
+    if (tside) wait_event(c, c->stream, c->ev_tscat);
+    substep_prologue(c, next_prologue, true);
     c->prologue_done = true;
-    cudaStreamWaitEvent(c->stream, c->ev_pub, 0);     // the full join covers the refresh
+    wait_event(c, c->stream, c->ev_pub);     // the full join covers the body's sums
     MIBM_LAUNCH_CHECK(c, "particle");
   } else if (c->status == MIBM_OK) {
     geometry_launch(c, imelt);
@@ -2753,6 +2971,7 @@ const double* lagr_particle_fused(Ctx* c, const StepParams* dp, float* m32, Step
     if (str) k_rigid_publish(c, s->geom_out, next);
     if (fork) cudaEventRecord(c->ev_pub, c->stream);
     c->geom_join_tag = false;
+    if (tside) wait_event(c, c->stream, c->ev_tscat);
     if (fork && next_prologue >= 0) {
       lagr_substep_prologue(c, next_prologue);
       c->prologue_done = true;
@@ -2770,8 +2989,12 @@ const double* lagr_particle_fused(Ctx* c, const StepParams* dp, float* m32, Step
 
 // the main stream waits for the side-stream half of the last particle
 void lagr_join(Ctx* c) {
+  if (c->tscat_pending) {
+    wait_event(c, c->stream, c->ev_tscat);
+    c->tscat_pending = false;
+  }
   if (!c->join_pending) return;
-  cudaStreamWaitEvent(c->stream, c->ev_join, 0);
+  wait_event(c, c->stream, c->ev_join);
   c->join_pending = false;
   c->geom_join_pending = false;
 }
@@ -2780,9 +3003,13 @@ void lagr_join(Ctx* c) {
 // from the side branch: the moved body (published state, geometry) and,
 // when the tagging ran on its own stream, the VOF fields
 void lagr_join_geom(Ctx* c) {
+  if (c->tscat_pending) {          // the forced temperature
+    wait_event(c, c->stream, c->ev_tscat);
+    c->tscat_pending = false;
+  }
   if (!c->geom_join_pending) return;
-  cudaStreamWaitEvent(c->stream, c->ev_pub, 0);
-  if (c->geom_join_tag) cudaStreamWaitEvent(c->stream, c->ev_tjoin, 0);
+  wait_event(c, c->stream, c->ev_pub);
+  if (c->geom_join_tag) wait_event(c, c->stream, c->ev_tjoin);
   c->geom_join_pending = false;
 }
 

@@ -322,13 +322,13 @@ void k_update_xyz(Ctx* c, bool centroids) {
   int n = std::max(c->maxnv, c->maxnf);
   if (n == 0) return;
   { MIBM_PROF(c, "update_xyz");
-    update_xyz_kernel<<<div_up(n, 128), 128, 0, c->stream>>>(
+    update_xyz_kernel<<<div_up(n, 32), 32, 0, c->stream>>>(
         c->maxnv, c->maxnf, (const int*)c->dm[MIBM_M_GHOST_VERT], (const int*)c->dm[MIBM_M_GHOST_FACE], c->drigid,
         (double*)c->dm[MIBM_M_XYZV], (const double*)c->dm[MIBM_M_TRI_BAR], (double*)c->dm[MIBM_M_VEL_TRI]); }
   ++c->launches;
   if (centroids && c->maxnf > 0) {
     MIBM_PROF(c, "centroids");
-    centroid_kernel<<<div_up(c->maxnf, 128), 128, 0, c->stream>>>(
+    centroid_kernel<<<div_up(c->maxnf, 32), 32, 0, c->stream>>>(
         c->maxnf, (const int*)c->dm[MIBM_M_VERT_OF_FACE], (const int*)c->dm[MIBM_M_GHOST_FACE],
         (const double*)c->dm[MIBM_M_XYZV], (double*)c->dm[MIBM_M_TRI_BAR]);
     ++c->launches;

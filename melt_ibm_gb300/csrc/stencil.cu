@@ -1063,8 +1063,8 @@ float stencil_time_by(Ctx* c, const StepParams* dp, int by, int reps) {
 // precision form: FP32 explicit terms and RHS into FP32 ru / rhs buffers
 // the precision form's explicit terms: u, v, w in one kernel (or, with the
 // one-pass kernel switched off, through the products as in the FP64 form),
-// then T
-void k_fused_rhs_f32(Ctx* c, const StepParams* dp, float* ru4, float* rhs4) {
+// and T on its own
+void k_rhs_uvw_f32(Ctx* c, const StepParams* dp, float* ru4, float* rhs4) {
   if (c->fused_uvw) {
     { MIBM_PROF(c, "fused_uvw_f32"); fused_uvw_launch(c, dp, ru4, rhs4); }
     ++c->launches;
@@ -1076,9 +1076,13 @@ void k_fused_rhs_f32(Ctx* c, const StepParams* dp, float* ru4, float* rhs4) {
       ++c->launches;
     }
   }
+  MIBM_LAUNCH_CHECK(c, "fused_uvw_f32");
+}
+
+void k_rhs_t_f32(Ctx* c, const StepParams* dp, float* ru, float* rhs) {
   { MIBM_PROF(c, "fused_rhs_f32");
-    if (c->fused_uvw) fused_t_launch(c, dp, ru4 + 3 * c->g.cells, rhs4 + 3 * c->g.cells);
-    else fused_rhs_launch<float>(c, dp, 3, ru4 + 3 * c->g.cells, rhs4 + 3 * c->g.cells); }
+    if (c->fused_uvw) fused_t_launch(c, dp, ru, rhs);
+    else fused_rhs_launch<float>(c, dp, 3, ru, rhs); }
   ++c->launches;
   MIBM_LAUNCH_CHECK(c, "fused_rhs_f32");
 }

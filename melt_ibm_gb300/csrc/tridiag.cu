@@ -645,8 +645,8 @@ std::vector<int> tri_chunk_candidates(Ctx* c, int dir) {
 // Constants of the geo_* kernels for (n, M, G = betadx): rho, the scale the
 // kernel applies, F and K (see the top of the file; the thresholds drop
 // relative 2^-60), then rho^(i+1) for i < M and rho^(mM) / (1 - rho^n) for
-// m < n/M.  The powers are formed in extended precision from the rounded rho,
-// so that every path round the line uses the same constant.
+// m < n/M.  The powers are formed in double-double from the rounded rho, so
+// that every path round the line uses the same constant.
 constexpr int kGeoPow = 4;                     // offsets within the slot
 constexpr int kGeoMul = kGeoPow + 32;
 constexpr int kGeoLen = kGeoMul + 32;
@@ -658,6 +658,16 @@ static double geo_scale(double betadx) {
   const double d = 1.0 - geo_rho(betadx);
   return d * d;
 }
+// an unevaluated sum of two doubles, and the product of two of them (Dekker's,
+// with the rounding error of hi * hi from one fma): the host step's tables
+// without extended precision, which is software on this machine's CPU
+struct TwoSum { double hi, lo; };
+static TwoSum dd_mul(TwoSum a, TwoSum b) {
+  const double h = a.hi * b.hi;
+  const double e = std::fma(a.hi, b.hi, -h) + (a.hi * b.lo + a.lo * b.hi);
+  const double s = h + e;
+  return TwoSum{s, e - (s - h)};
+}
 static void fill_geo(int n, int m, double betadx, double scale, double* out) {
   const int G = n / m;
   const double rho = geo_rho(betadx);
@@ -666,14 +676,11 @@ static void fill_geo(int n, int m, double betadx, double scale, double* out) {
   out[1] = scale;
   out[2] = (double)std::min((double)m, std::ceil(60.0 / bits));
   out[3] = (double)std::min((double)G, std::ceil(60.0 / (bits * m)));
-  long double p = 1.0L, rn = 1.0L;
-  for (int i = 0; i < m; ++i) { p *= (long double)rho; out[kGeoPow + i] = (double)p; }
-  for (int h = 0; h < G; ++h) rn *= p;
-  p = 1.0L / (1.0L - rn);
-  for (int h = 0; h < G; ++h) {
-    out[kGeoMul + h] = (double)p;
-    for (int i = 0; i < m; ++i) p *= (long double)rho;
-  }
+  TwoSum p{1.0, 0.0}, q{1.0, 0.0};
+  for (int i = 0; i < m; ++i) { p = dd_mul(p, TwoSum{rho, 0.0}); out[kGeoPow + i] = p.hi; }
+  for (int h = 0; h < G; ++h) { out[kGeoMul + h] = q.hi; q = dd_mul(q, p); }
+  const double wrap = 1.0 / ((1.0 - q.hi) - q.lo);
+  for (int h = 0; h < G; ++h) out[kGeoMul + h] *= wrap;
 }
 
 // fills one slot (base + the extended table of chunk m) for (n, betadx)
@@ -1307,13 +1314,23 @@ bool tri_step_fill(Ctx* c, const double betadx[3][2][3], bool f32) {
       }
     return true;
   }
-  for (int ns = 0; ns < 3; ++ns)
-    for (int f = 0; f < 2; ++f)
-      for (int d = 0; d < 3; ++d)
-        fill_slot(n[d], tri_chunk(c, d), betadx[ns][f][d], st->pinned + (size_t)((ns * 2 + f) * 3 + d) * st->len);
-  if (f32) {
-    float* hf = (float*)(st->pinned + 18 * cap);
-    for (size_t q = 0; q < 18 * (size_t)st->len; ++q) hf[q] = (float)st->pinned[q];
+  // equal systems (a Prandtl number of 1, equal spacings) get copies of one table
+  float* hf = (float*)(st->pinned + 18 * cap);
+  for (int s = 0; s < 18; ++s) {
+    const int d = s % 3, m = tri_chunk(c, d);
+    const double bd = betadx[s / 6][(s / 3) % 2][d];
+    double* out = st->pinned + (size_t)s * st->len;
+    float* outf = hf + (size_t)s * st->len;
+    int same = -1;
+    for (int o = 0; o < s && same < 0; ++o)
+      if (n[o % 3] == n[d] && tri_chunk(c, o % 3) == m && betadx[o / 6][(o / 3) % 2][o % 3] == bd) same = o;
+    if (same < 0) fill_slot(n[d], m, bd, out);
+    else memcpy(out, st->pinned + (size_t)same * st->len, sizeof(double) * (size_t)st->len);
+    if (!f32) continue;
+    if (same < 0)
+      for (int q = 0; q < st->len; ++q) outf[q] = (float)out[q];
+    else
+      memcpy(outf, hf + (size_t)same * st->len, sizeof(float) * (size_t)st->len);
   }
   return true;
 }
