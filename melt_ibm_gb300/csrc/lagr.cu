@@ -2860,11 +2860,16 @@ void lagr_loads_early(Ctx* c, const StepParams* dp) {
 // The heat flux reads the solved temperature (before the temperature forcing)
 // and the geometry, nothing of the velocity forcing: the fused step starts it
 // on the tagging's stream, idle at this point, once T is solved (called with
-// the context's stream the one that solves T).  Same conditions as above.
+// the context's stream the one that solves T).  Same conditions as above, and
+// not on large grids: there the chain hides beside the projection anyway, and
+// the flux would take the FP64 pipe from kernels the main stream waits for
+// (128^3 free body 7.44 -> 7.35 ms, 48^3 5.19 -> 3.78 ms for two and four
+// steps; HEAT256_FIGS).
+constexpr size_t kHeatEarlyCells = 4u << 20;
 void lagr_heat_early(Ctx* c) {
   c->heat_pending = false;
   if (c->I(MIBM_I_IMLSFOR) != 1 || c->maxnf == 0 || c->I(MIBM_I_IMELT) != 1) return;
-  if (!lagr_fork_enabled(c) || !c->side2) return;
+  if (!lagr_fork_enabled(c) || !c->side2 || c->g.cells > kHeatEarlyCells) return;
   if (!ensure_adjacency(c) || !ensure_lag_buffers(c)) return;
   cudaEventRecord(c->ev_hfork, c->stream);
   wait_event(c, c->side2, c->ev_hfork);
