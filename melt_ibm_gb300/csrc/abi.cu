@@ -280,7 +280,7 @@ static void step_enqueue_f64(Ctx* c) {
     const double* mean3 = lagr_particle_fused(c, dp, nullptr, ns < 2 ? c->dparams + ns + 1 : nullptr, ns + 1);
     if (c->status != MIBM_OK) return;
     k_divg(c, dp);
-    k_phcalc(c);
+    k_phcalc(c, tri_keep_order(c));
     k_updvp_prcalc(c, dp, mean3);
     if (c->status != MIBM_OK) return;
   }

@@ -409,7 +409,7 @@ void k_solve_y_f32(Ctx* c, float* rhs, const float* T, int nfield);
 // mirror: FP32 copies of the q fields written beside them (field f at mirror + f*cells), or null
 void k_solve_z_f32(Ctx* c, float* rhs, const float* T, double* const* q, int nfield, float* mirror);
 // fft.cu
-void k_phcalc(Ctx* c);
+void k_phcalc(Ctx* c, bool keep_order = false);
 void k_phcalc_f32(Ctx* c, const float* src, float* phi);
 // lagr.cu
 void lagr_find_centroid_indices(Ctx* c);

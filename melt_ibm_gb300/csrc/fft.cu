@@ -14,9 +14,10 @@
 //   X' c2r along x   two Hermitian half-rows packed as one complex line
 // Line FFTs are Stockham autosort transforms with radix-4/2/3 stages
 // (n = 2^a 3^b), twiddles e^{-2 pi i m/n} tabulated on the host in FP64 and
-// staged in shared memory.  Each pass runs the kernel of fft_fast.cuh
-// specialised for its line length when the length has one; the kernels
-// below take any length (run-time plan).  Unnormalised, FFTW sign convention
+// staged in shared memory.  The FP64 form's x and y passes run on the integer
+// pipe (fft_int.cuh); the others, and those of a step that keeps its order of
+// operations, run the kernel of fft_fast.cuh specialised for their line length
+// when the length has one, else the kernels below (any length, run-time plan).  Unnormalised, FFTW sign convention
 // (forward = e^{-i...}).  The c2r pass drops the imaginary parts of the
 // kx = 0 and kx = n1m/2 bins, as a Hermitian c2r transform does.
 #include <cmath>
@@ -230,6 +231,7 @@ __global__ void fft_z_solve(FftArgs<C> F, C* __restrict__ spec) {
 struct FftCache {
   Ctx* c = nullptr;
   double2 *twx = nullptr, *twy = nullptr, *twz = nullptr;
+  int4* itw = nullptr;      // FftArgs::itw
   float2 *ftwx = nullptr, *ftwy = nullptr, *ftwz = nullptr;
   float *fak1 = nullptr, *fak2 = nullptr, *fak3 = nullptr;
   double* eig = nullptr;    // FftArgs::eig, FP64 (built at the first FP64 solve)
@@ -360,6 +362,25 @@ static C* make_tw(Ctx* c, int n) {
   return d;
 }
 
+// (cos, -sin) of the forward twiddles to 2^-62, as signed 32-bit halves (fft_int.cuh)
+static int4* make_itw(Ctx* c, int n) {
+  std::vector<int4> h(n);
+  auto put = [](long double v, int& hi, int& lo) {
+    const long long x = (long long)std::llrint(v * 4611686018427387904.0L);
+    lo = (int)(unsigned)(x & 0xffffffffll);
+    hi = (int)((x - lo) >> 32);
+  };
+  for (int m = 0; m < n; ++m) {
+    const long double a = 2.0L * 3.141592653589793238462643383279502884L * (long double)m / (long double)n;
+    put(std::cos(a), h[m].x, h[m].y);
+    put(-std::sin(a), h[m].z, h[m].w);
+  }
+  int4* d = nullptr;
+  if (!cuda_ok(c, cudaMalloc(&d, sizeof(int4) * n), "twiddles")) return nullptr;
+  cudaMemcpy(d, h.data(), sizeof(int4) * n, cudaMemcpyHostToDevice);
+  return d;
+}
+
 static float* make_fak(Ctx* c, const double* ak, int n) {
   std::vector<double> h(n);
   cudaMemcpy(h.data(), ak, sizeof(double) * n, cudaMemcpyDeviceToHost);
@@ -378,6 +399,7 @@ static FftCache* fft_of(Ctx* c) {
   f.twx = make_tw<double2>(c, c->g.n1m);
   f.twy = make_tw<double2>(c, c->g.n2m);
   f.twz = make_tw<double2>(c, c->g.n3m);
+  f.itw = make_itw(c, c->g.n1m);
   f.ftwx = make_tw<float2>(c, c->g.n1m);
   f.ftwy = make_tw<float2>(c, c->g.n2m);
   f.ftwz = make_tw<float2>(c, c->g.n3m);
@@ -392,7 +414,7 @@ void fft_free(Ctx* c) {
   for (size_t q = 0; q < g_fft.size(); ++q)
     if (g_fft[q].c == c) {
       FftCache& f = g_fft[q];
-      cudaFree(f.twx); cudaFree(f.twy); cudaFree(f.twz);
+      cudaFree(f.twx); cudaFree(f.twy); cudaFree(f.twz); cudaFree(f.itw);
       cudaFree(f.ftwx); cudaFree(f.ftwy); cudaFree(f.ftwz);
       cudaFree(f.fak1); cudaFree(f.fak2); cudaFree(f.fak3);
       cudaFree(f.eig); cudaFree(f.feig); cudaFree(f.ztri); cudaFree(f.fztri);
@@ -406,6 +428,23 @@ void fft_free(Ctx* c) {
 bool fft_prepare(Ctx* c, bool f32) {
   FftCache* fc = fft_of(c);
   return make_eig(c, fc, f32) && (f32 || make_ztri(c, fc, false));
+}
+
+// the integer-pipe passes of the FP64 form; false: not wanted or no instance
+template <typename C, typename S>
+static bool int_x_fwd(Ctx* c, const FftArgs<C>& F, const S* src, C* spec) {
+  if constexpr (sizeof(C) == 16) return F.itw && intfft_x_fwd(c, F.itw, src, spec);
+  return false;
+}
+template <typename C>
+static bool int_x_inv(Ctx* c, const FftArgs<C>& F, const C* spec, typename Real<C>::T* dst) {
+  if constexpr (sizeof(C) == 16) return F.itw && intfft_x_inv(c, F.itw, spec, dst);
+  return false;
+}
+template <typename C>
+static bool int_y(Ctx* c, const FftArgs<C>& F, C* spec, int sign) {
+  if constexpr (sizeof(C) == 16) return F.itw && intfft_y(c, F.itw, spec, sign);
+  return false;
 }
 
 template <typename C, typename S>
@@ -425,23 +464,25 @@ static void phcalc_launch(Ctx* c, FftArgs<C> F, const S* src, typename Real<C>::
   bool f32 = sizeof(C) == sizeof(float2);
   // each pass: the kernel specialised for its line length where one exists
   { MIBM_PROF(c, f32 ? "fft_x_fwd_f32" : "fft_x_fwd");
-    if (!fastfft_x_fwd<C, S>(c, F, src, spec)) fft_x_fwd<C, S><<<gx, 256, smx, c->stream>>>(F, src, spec); }
+    if (!int_x_fwd<C, S>(c, F, src, spec) && !fastfft_x_fwd<C, S>(c, F, src, spec)) fft_x_fwd<C, S><<<gx, 256, smx, c->stream>>>(F, src, spec); }
   { MIBM_PROF(c, f32 ? "fft_y_f32" : "fft_y");
-    if (!fastfft_y<C>(c, F, spec, -1)) fft_y<C><<<gy, 256, smy, c->stream>>>(F, spec, -1); }
+    if (!int_y<C>(c, F, spec, -1) && !fastfft_y<C>(c, F, spec, -1)) fft_y<C><<<gy, 256, smy, c->stream>>>(F, spec, -1); }
   { MIBM_PROF(c, f32 ? "fft_z_solve_f32" : "fft_z_solve");
     if (!fastfft_z_solve<C>(c, F, spec)) fft_z_solve<C><<<gz, 256, smz, c->stream>>>(F, spec); }
   { MIBM_PROF(c, f32 ? "fft_y_f32" : "fft_y");
-    if (!fastfft_y<C>(c, F, spec, +1)) fft_y<C><<<gy, 256, smy, c->stream>>>(F, spec, +1); }
+    if (!int_y<C>(c, F, spec, +1) && !fastfft_y<C>(c, F, spec, +1)) fft_y<C><<<gy, 256, smy, c->stream>>>(F, spec, +1); }
   { MIBM_PROF(c, f32 ? "fft_x_inv_f32" : "fft_x_inv");
-    if (!fastfft_x_inv<C>(c, F, spec, dst)) fft_x_inv<C><<<gx, 256, smx, c->stream>>>(F, spec, dst); }
+    if (!int_x_inv<C>(c, F, spec, dst) && !fastfft_x_inv<C>(c, F, spec, dst)) fft_x_inv<C><<<gx, 256, smx, c->stream>>>(F, spec, dst); }
   c->launches += 5;
   MIBM_LAUNCH_CHECK(c, tag);
 }
 
-void k_phcalc(Ctx* c) {
+// keep_order: the FP64 passes, whose results are those of earlier builds bit
+// for bit (tri_keep_order says when the step wants that)
+void k_phcalc(Ctx* c, bool keep_order) {
   const Grid& g = c->g;
   FftCache* fc = fft_of(c);
-  if (!fc->twx || !fc->twy || !fc->twz) return;
+  if (!fc->twx || !fc->twy || !fc->twz || !fc->itw) return;
   FftArgs<double2> F;
   F.g = g;
   F.px = make_plan(g.n1m); F.py = make_plan(g.n2m); F.pz = make_plan(g.n3m);
@@ -451,6 +492,7 @@ void k_phcalc(Ctx* c) {
   if (!make_eig(c, fc, false) || !make_ztri(c, fc, false)) return;
   F.eig = fc->eig;
   F.ztri = fc->ztri; F.zt_lines = fc->zt_lines; F.zt_m = fc->zt_m;
+  F.itw = keep_order ? nullptr : fc->itw;
   phcalc_launch<double2, double>(c, F, c->df[MIBM_F_DPH], c->df[MIBM_F_DPH], "phcalc");
 }
 
@@ -471,6 +513,7 @@ void k_phcalc_f32(Ctx* c, const float* src, float* phi) {
   // FP32 transforms cost little on the FP32 pipe: the z pass stays a
   // transform (the tridiagonal lines are latency-bound and slower there)
   F.ztri = nullptr; F.zt_lines = 0; F.zt_m = 0;
+  F.itw = nullptr;
   phcalc_launch<float2, float>(c, F, src, phi, "phcalc_f32");
 }
 

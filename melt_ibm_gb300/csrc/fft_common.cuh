@@ -53,6 +53,7 @@ struct FftArgs {
   const R* ztri;
   int zt_lines;
   int zt_m;            // chunk length of the chunked z-line tables, 0: one thread per line
+  const int4* itw;     // twiddles of the integer-pipe x and y passes (n1m = n2m), nullptr: FP64 passes
 };
 
 // chunk length of the chunked z-line Poisson solve for `lines` lines of n
@@ -89,6 +90,12 @@ template <typename C>
 bool fastfft_z_solve(Ctx* c, const FftArgs<C>& F, C* spec);
 template <typename C>
 bool fastfft_x_inv(Ctx* c, const FftArgs<C>& F, const C* spec, typename Real<C>::T* dst);
+
+// the FP64 solve's x and y passes on the integer pipe (fft_int_x.cu,
+// fft_int_y.cu; tw: fft_int.cuh's twiddles); false: no instance
+bool intfft_x_fwd(Ctx* c, const int4* tw, const double* src, double2* spec);
+bool intfft_x_inv(Ctx* c, const int4* tw, const double2* spec, double* dst);
+bool intfft_y(Ctx* c, const int4* tw, double2* spec, int sign);
 
 // instances (fft_fast_f64.cu, fft_fast_f32.cu)
 template <> bool fastfft_x_fwd<double2, double>(Ctx*, const FftArgs<double2>&, const double*, double2*);
