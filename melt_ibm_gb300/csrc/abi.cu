@@ -133,7 +133,7 @@ static bool step_prepare(Ctx* c) {
   } else {
     c->q32_valid = false;
     if (!c->rhs4 && !cuda_ok(c, cudaMalloc(&c->rhs4, 4 * g.cells * sizeof(double)), "rhs4")) return false;
-    if (!c->prod && !cuda_ok(c, cudaMalloc(&c->prod, 6 * g.cells * sizeof(double)), "advection products"))
+    if (tri_keep_order(c) && !c->prod && !cuda_ok(c, cudaMalloc(&c->prod, 6 * g.cells * sizeof(double)), "advection products"))
       return false;
   }
   if (!tri_step_fill(c, bd, f32)) return false;
@@ -507,7 +507,9 @@ static int autotune(Ctx* c) {
     }
   }
   r.ms_by = -1.f;
+  r.by = c->tune_by;
   for (int by : {2, 4, 8}) {
+    if (!f32 && !tri_keep_order(c)) break;       // the one-kernel explicit terms have one block shape
     float ms = stencil_time_by(c, c->dparams, by, 5);
     if (c->status != MIBM_OK) return c->status;
     if (ms >= 0.f && (r.ms_by < 0.f || ms < r.ms_by)) { r.ms_by = ms; r.by = by; }

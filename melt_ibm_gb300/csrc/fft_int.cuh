@@ -8,7 +8,7 @@
 // line is transformed in 64-bit fixed point with one exponent per line (block
 // floating point):
 //   load    the line's largest exponent is found, every value becomes
-//           mantissa << 6 (x inverse: << 5) at that exponent, rounded;
+//           mantissa << 6 (x inverse: << 5) at that exponent;
 //   stages  radix-4/2/3 Stockham stages as in fft_fast.cuh; before each stage
 //           but the first, values are halved (rounded) as often as the stage
 //           may grow them: ceil(log2(points combined)) in all, so that
@@ -31,9 +31,12 @@
 #pragma once
 
 #include "fft_common.cuh"
+#include "fixed.cuh"
 
 namespace mibm {
 namespace intfft {
+
+using namespace fixed;
 
 struct I2 { long long x, y; };
 // (cos, -sin) 2^62 of the forward twiddle as signed halves
@@ -76,13 +79,6 @@ __device__ __forceinline__ I2 down(I2 v) { return I2{down<S>(v.x), down<S>(v.y)}
 
 __device__ __forceinline__ I2 add(I2 a, I2 b) { return I2{a.x + b.x, a.y + b.y}; }
 __device__ __forceinline__ I2 sub(I2 a, I2 b) { return I2{a.x - b.x, a.y - b.y}; }
-
-// signed halves of x: x = hi 2^32 + lo, lo in [-2^31, 2^31)
-__device__ __forceinline__ void halves(long long x, int& hi, int& lo) {
-  lo = (int)x;
-  hi = (int)(x >> 32) + (int)((unsigned)lo >> 31);
-}
-__device__ __forceinline__ long long wide(int a, int b) { return (long long)a * b; }
 
 // v w / 2^S (w, or its conjugate for INV), S = 1 or 2
 template <int S, bool INV>
@@ -181,37 +177,8 @@ __device__ __forceinline__ void run(I2* buf, const Tw* tw) {
   }
 }
 
-// biased exponent (zero and subnormal values: 0) and its maximum over values
-__device__ __forceinline__ int expo(double d) { return (int)((__double_as_longlong(d) >> 52) & 0x7ff); }
-
-// d at the exponent E of its line (1 <= E), times 2^(1075 - E + UP), rounded
-template <int UP>
-__device__ __forceinline__ long long fixed(double d, int E) {
-  const long long b = __double_as_longlong(d);
-  const int e = (int)((b >> 52) & 0x7ff);
-  long long m = (b & 0xfffffffffffffll) | (e ? 1ll << 52 : 0);
-  m <<= UP;
-  const int r = min(E - max(e, 1), 60);
-  if (r > 0) m = ((m >> (r - 1)) + 1) >> 1;
-  return b < 0 ? -m : m;
-}
-
-// f 2^(X - 1075) as a double, rounded to nearest (ties to even); E of the
-// line: NaN if it held a non-finite value
-__device__ __forceinline__ double real(long long f, int X, int E) {
-  if (E == 0x7ff) return __longlong_as_double(0x7ff8000000000000ll);
-  const unsigned long long s = (unsigned long long)f & 0x8000000000000000ull;
-  unsigned long long a = f < 0 ? 0ull - (unsigned long long)f : (unsigned long long)f;
-  if (a == 0) return 0.0;
-  const int lz = __clzll((long long)a);
-  a <<= lz;                                             // 2^63 <= a < 2^64
-  unsigned long long m = a >> 11;
-  const unsigned rest = (unsigned)a & 0x7ffu;
-  m += (rest > 0x400u) || (rest == 0x400u && (m & 1));
-  const int e = 63 - lz + X - 52;                        // biased exponent of the leading bit: 63 - lz + (X - 1075) + 1023
-  if (e < 1 || e > 2045) return scalbn((double)f, X - 1075);   // subnormal or near overflow
-  return __longlong_as_double((long long)(s | (((unsigned long long)(e - 1) << 52) + m)));
-}
+// to_double, or NaN where the line (exponent E) held a non-finite value
+__device__ __forceinline__ double real(long long f, int X, int E) { return E == 0x7ff ? quiet_nan() : to_double(f, X); }
 
 template <int N, int T>
 __device__ __forceinline__ void stage_twiddles(Tw* s, const Tw* __restrict__ tw) {
@@ -251,7 +218,7 @@ __global__ void __launch_bounds__(Shape<N>::T, 3) x_fwd(Grid g, const Tw* __rest
 #pragma unroll
     for (int p = 0; p < PER; ++p) {
       const int i = lane + 32 * p;
-      if (N % 32 == 0 || i < N) buf[i * ES + l] = I2{fixed<6>(a[p], E[q]), fixed<6>(b[p], E[q])};
+      if (N % 32 == 0 || i < N) buf[i * ES + l] = I2{from_double<6>(a[p], E[q]), from_double<6>(b[p], E[q])};
     }
   }
   __syncthreads();
@@ -308,8 +275,8 @@ __global__ void __launch_bounds__(Shape<N>::T, 3) x_inv(Grid g, const Tw* __rest
     for (int p = 0; p < PER; ++p) {
       const int kx = lane + 32 * p;
       if (kx >= H) continue;
-      const long long ax = fixed<5>(a[p].x, E[q]), ay = fixed<5>(a[p].y, E[q]);
-      const long long bx = fixed<5>(b[p].x, E[q]), by = fixed<5>(b[p].y, E[q]);
+      const long long ax = from_double<5>(a[p].x, E[q]), ay = from_double<5>(a[p].y, E[q]);
+      const long long bx = from_double<5>(b[p].x, E[q]), by = from_double<5>(b[p].y, E[q]);
       buf[kx * ES + l] = I2{ax - by, ay + bx};            // Z = Xa + i Xb
       if (kx > 0 && 2 * kx < N) buf[(N - kx) * ES + l] = I2{ax + by, bx - ay};
     }
@@ -365,7 +332,7 @@ __global__ void __launch_bounds__(Shape<N>::T, 3) y_pass(Grid g, const Tw* __res
 #pragma unroll
   for (int p = 0; p < PER; ++p) {
     const int e = e0 + p * (T / L);
-    if (N * L % T == 0 || e < N) buf[e * ES + l] = I2{fixed<6>(v[p].x, E), fixed<6>(v[p].y, E)};
+    if (N * L % T == 0 || e < N) buf[e * ES + l] = I2{from_double<6>(v[p].x, E), from_double<6>(v[p].y, E)};
   }
   __syncthreads();
   run<N, L, T, INV>(buf, tw);

@@ -2864,7 +2864,7 @@ void lagr_loads_early(Ctx* c, const StepParams* dp) {
 // not on large grids: there the chain hides beside the projection anyway, and
 // the flux would take the FP64 pipe from kernels the main stream waits for
 // (128^3 free body 7.44 -> 7.35 ms, 48^3 5.19 -> 3.78 ms for two and four
-// steps; HEAT256_FIGS).
+// steps; 256^3 FP64 81.9 -> 82.5 ms for three).
 constexpr size_t kHeatEarlyCells = 4u << 20;
 void lagr_heat_early(Ctx* c) {
   c->heat_pending = false;

@@ -14,6 +14,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "fixed.cuh"
 #include "fpconv.cuh"
 
 namespace mibm {
@@ -530,6 +531,186 @@ fused_t_f32_kernel(StencilArgs A, const StepParams* __restrict__ pp, float* __re
   ru[c0] = h;
 }
 
+// FP64 form: the explicit terms and RHS of u, v, w and T in one kernel with
+// the sums and products on the integer pipe.
+// A block takes 32 x 4 x 4 cells, one per thread: u, v, w and T of the cells
+// and one layer around them are converted once into 64-bit fixed point in
+// shared memory, u, v, w at the largest exponent of the three in the block, T
+// at its own.  Each thread forms its cell's advection terms (products of hdnl1-3
+// regrouped as above: 15 integer products; hdnlte: 6) and Laplacians from
+// there, and rounds each sum to FP64 once.  What stays FP64 is the RK
+// combination: 6 operations per velocity component, 5 for T, against 46 per cell
+// for the products kernel and the four fused_rhs kernels.  A product is kept
+// to 2^-58 of the square of the block's largest velocity, the FP64 product it
+// replaces to 2^-53 of its own value.  A cell that is not fully fluid takes
+// h_t's solid-advection branch; a block that holds a non-finite value gives NaN.
+// Layers around the cells: 2.4 values converted per value used (32 x 8 x 1
+// cells: 4).  About 1400 instructions per cell and warp, neither pipe full (FP64
+// 0.6, integer 0.4): with 64 registers two blocks share an SM.  Per substep,
+// five kernels -> this one: 128^3 330 -> 177 us, 96^3 146 -> 70, 108 x 108 x 72
+// (two spacings) 226 -> 106, 48^3 53 -> 27 us (one wave of blocks).
+struct RuSet { double* r[4]; };
+constexpr int kExX = 32, kExY = 4, kExZ = 4, kExThreads = kExX * kExY * kExZ;
+constexpr int kExHX = kExX + 2, kExHY = kExY + 2, kExHZ = kExZ + 2, kExV = kExHX * kExHY * kExHZ;
+
+// SP: 0 equal grid spacings, 1 equal in x and y, 2 any (1, 2 or 3 conversions per sum)
+template <int SP>
+__global__ void __launch_bounds__(kExThreads, 2)
+explicit_int_kernel(StencilArgs A, const StepParams* __restrict__ pp, RuSet ru, double* __restrict__ rhs4) {
+  using namespace fixed;
+  constexpr int UP = 7, kWarps = kExThreads / 32, kRows = kExHY * kExHZ, PER = (kRows + kWarps - 1) / kWarps;
+  static_assert(2 * kRows <= kExThreads, "one thread per value beyond a row's first 32");
+  __shared__ long long sq[4][kExV];
+  __shared__ int smax[2];
+  const Grid& g = A.g;
+  const int lane = threadIdx.x, warp = threadIdx.y + kExY * threadIdx.z, tid = lane + 32 * warp;
+  const int i0 = blockIdx.x * kExX, j0 = blockIdx.y * kExY, k0 = blockIdx.z * kExZ;
+  if (tid < 2) smax[tid] = 1;
+  {
+    // a warp takes whole rows of 32 values, the 2 left over of each row go to
+    // a thread each; periodic, and a cell past the grid's end repeats one inside it
+    auto wrapped = [](int x, int n) { return x < 0 ? x + n : (x < n ? x : (x < 2 * n ? x - n : x % n)); };
+    auto row_base = [&](int r) {
+      const int j = wrapped(j0 + r % kExHY - 1, g.n2m), k = wrapped(k0 + r / kExHY - 1, g.n3m);
+      return g.P * (j + g.n2m * k);
+    };
+    const int il = wrapped(i0 + lane - 1, g.n1m);
+    double raw[4][PER + 1];
+    int eu = 1, et = 1;
+#pragma unroll
+    for (int p = 0; p <= PER; ++p) {
+      const int r = p < PER ? warp + p * kWarps : tid >> 1;
+      const bool ok = p < PER ? r < kRows : tid < 2 * kRows;
+      const int c = ok ? row_base(r) + (p < PER ? il : wrapped(i0 + 31 + (tid & 1), g.n1m)) : 0;
+      raw[0][p] = ok ? A.vx[c] : 0.0;
+      raw[1][p] = ok ? A.vy[c] : 0.0;
+      raw[2][p] = ok ? A.vz[c] : 0.0;
+      raw[3][p] = ok ? A.temp[c] : 0.0;
+    }
+#pragma unroll
+    for (int p = 0; p <= PER; ++p) {
+      eu = max(eu, max(expo(raw[0][p]), max(expo(raw[1][p]), expo(raw[2][p]))));
+      et = max(et, expo(raw[3][p]));
+    }
+    eu = __reduce_max_sync(0xffffffffu, eu);
+    et = __reduce_max_sync(0xffffffffu, et);
+    __syncthreads();
+    if (lane == 0) {
+      atomicMax(&smax[0], eu);
+      atomicMax(&smax[1], et);
+    }
+    __syncthreads();
+    const int E = smax[0], ET = smax[1];
+#pragma unroll
+    for (int p = 0; p <= PER; ++p) {
+      const int r = p < PER ? warp + p * kWarps : tid >> 1;
+      if (p < PER ? r < kRows : tid < 2 * kRows) {
+        const int t = r * kExHX + (p < PER ? lane : 32 + (tid & 1));
+        sq[0][t] = from_double<UP>(raw[0][p], E);
+        sq[1][t] = from_double<UP>(raw[1][p], E);
+        sq[2][t] = from_double<UP>(raw[2][p], E);
+        sq[3][t] = from_double<UP>(raw[3][p], ET);
+      }
+    }
+  }
+  __syncthreads();
+  const int E = smax[0], ET = smax[1];
+  const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
+  if (i >= g.n1m || j >= g.n2m) return;
+  const StepParams& p = *pp;
+  // exponents of a sum of products, of a Laplacian (kept at a quarter), of a sum
+  const int XP = 2 * E - 1025, XT = E + ET - 1025;
+  {
+    const int kz = threadIdx.z, k = k0 + kz;
+    if (k >= g.n3m) return;
+    const int P = g.P, PL = (int)g.plane;
+    const idx_t c0 = i + P * (j + g.n2m * k);
+    const idx_t dip = (i + 1 == g.n1m) ? 1 - g.n1m : 1, dim = (i == 0) ? g.n1m - 1 : -1;
+    const idx_t djp = (j + 1 == g.n2m) ? -(g.n2m - 1) * P : P, djm = (j == 0) ? (g.n2m - 1) * P : -P;
+    const idx_t dkp = (k + 1 == g.n3m) ? -(g.n3m - 1) * PL : PL, dkm = (k == 0) ? (g.n3m - 1) * PL : -PL;
+    if (!MIBM_IDX_OK(c0, g.cells)) return;
+    if (E == 0x7ff || ET == 0x7ff) {
+      for (int W = 0; W < 4; ++W) rhs4[(size_t)W * g.cells + c0] = ru.r[W][c0] = quiet_nan();
+      return;
+    }
+    const int sx = 1, sy = kExHX, sz = kExHX * kExHY;
+    const int c = (threadIdx.x + 1) + sy * (threadIdx.y + 1) + sz * (kz + 1);
+    const long long* u = sq[0] + c;
+    const long long* v = sq[1] + c;
+    const long long* w = sq[2] + c;
+    const long long* T = sq[3] + c;
+    // the three differences of an advection term times their factors
+    auto adv = [&](long long x, long long y, long long z, double f1, double f2, double f3, int X) {
+      if constexpr (SP == 0) return -(f1 * to_double(x + y + z, X));
+      else if constexpr (SP == 1) return -(f1 * to_double(x + y, X) + f3 * to_double(z, X));
+      else return -(f1 * to_double(x, X) + f2 * to_double(y, X) + f3 * to_double(z, X));
+    };
+    auto lap = [&](const long long* s, double L1, double L2, double L3, int e) {
+      if constexpr (SP == 0) {
+        const long long sum = (s[sx] + s[-sx]) + (s[sy] + s[-sy]) + (s[sz] + s[-sz]);
+        return L1 * to_double((sum >> 2) - (s[0] + (s[0] >> 1)), e - UP + 2);
+      } else if constexpr (SP == 1) {
+        const long long xy = ((s[sx] + s[-sx]) >> 1) + ((s[sy] + s[-sy]) >> 1) - 2 * s[0];
+        return L1 * to_double(xy, e - UP + 1) + L3 * to_double(s[sz] + s[-sz] - 2 * s[0], e - UP);
+      } else {
+        return L1 * to_double(s[sx] + s[-sx] - 2 * s[0], e - UP) + L2 * to_double(s[sy] + s[-sy] - 2 * s[0], e - UP) +
+               L3 * to_double(s[sz] + s[-sz] - 2 * s[0], e - UP);
+      }
+    };
+    const double q1 = p.cd[kQ1], q2 = p.cd[kQ2], q3 = p.cd[kQ3];
+    const double gdt = p.cd[kGDT], rdt = p.cd[kRDT];
+    const double pc = A.pr[c0];
+    auto store = [&](int W, double h, double d) {
+      double* r = ru.r[W] + c0;
+      rhs4[(size_t)W * g.cells + c0] = gdt * h + (rdt * *r + d);
+      *r = h;
+    };
+    const double l1 = p.cd[kLV1], l2 = p.cd[kLV2], l3 = p.cd[kLV3];
+    // the products at this cell (see adv_products_kernel) that two components share
+    const long long E0 = mul_high(v[0] + v[-sx], u[0] + u[-sy]);
+    const long long F0 = mul_high(w[0] + w[-sx], u[0] + u[-sz]);
+    const long long H0 = mul_high(w[0] + w[-sy], v[0] + v[-sz]);
+    {
+      const long long x = square_high(u[sx] + u[0]) - square_high(u[0] + u[-sx]);
+      const long long y = mul_high(v[sy] + v[sy - sx], u[sy] + u[0]) - E0;
+      const long long z = mul_high(w[sz] + w[sz - sx], u[sz] + u[0]) - F0;
+      double h = adv(x, y, z, q1, q2, q3, XP);
+      if (A.forcing) h = add_forcing<double>(h, A.vofx, A.forcx, c0, p.cd[kRXLEN]);
+      store(0, h, lap(u, l1, l2, l3, E) - p.cd[kPD1] * (pc - A.pr[c0 + dim]));
+    }
+    {
+      const long long x = mul_high(v[sx] + v[0], u[sx] + u[sx - sy]) - E0;
+      const long long y = square_high(v[sy] + v[0]) - square_high(v[0] + v[-sy]);
+      const long long z = mul_high(w[sz] + w[sz - sy], v[sz] + v[0]) - H0;
+      double h = adv(x, y, z, q1, q2, q3, XP);
+      if (A.forcing) h = add_forcing<double>(h, A.vofy, A.forcy, c0, p.cd[kRYLEN]);
+      store(1, h, lap(v, l1, l2, l3, E) - p.cd[kPD2] * (pc - A.pr[c0 + djm]));
+    }
+    {
+      const long long x = mul_high(w[sx] + w[0], u[sx] + u[sx - sz]) - F0;
+      const long long y = mul_high(w[sy] + w[0], v[sy] + v[sy - sz]) - H0;
+      const long long z = square_high(w[sz] + w[0]) - square_high(w[0] + w[-sz]);
+      double h = adv(x, y, z, q1, q2, q3, XP);
+      if (p.betagz != 0.0) {
+        const double T_interp = (A.temp[c0] + A.temp[c0 + dkm]) * 0.5;
+        h = h + p.cd[kBETAGZ] * (T_interp - p.cd[kTLIQ]);
+      }
+      if (A.forcing) h = add_forcing<double>(h, A.vofz, A.forcz, c0, p.cd[kRZLEN]);
+      store(2, h, lap(w, l1, l2, l3, E) - p.cd[kPD3] * (pc - A.pr[c0 + dkm]));
+    }
+    double ht;
+    if (vof_is_one(A.vofp[c0])) {
+      const long long x = mul_high(u[sx], T[sx] + T[0]) - mul_high(u[0], T[0] + T[-sx]);
+      const long long y = mul_high(v[sy], T[sy] + T[0]) - mul_high(v[0], T[0] + T[-sy]);
+      const long long z = mul_high(w[sz], T[sz] + T[0]) - mul_high(w[0], T[0] + T[-sz]);
+      ht = adv(x, y, z, p.cd[kH1], p.cd[kH2], p.cd[kH3], XT);
+    } else {
+      ht = h_t<double>(A, i, j, k, c0, dip, dim, djp, djm, dkp, dkm, p);
+    }
+    store(3, ht, lap(T, p.cd[kLT1], p.cd[kLT2], p.cd[kLT3], ET));
+  }
+}
+
 static bool equal_spacings(const Grid& g) { return g.dx1 == g.dx2 && g.dx1 == g.dx3; }
 
 template <typename R, bool ISO>
@@ -984,6 +1165,19 @@ static void adv_products_launch(Ctx* c, R* out) {
 }
 
 void k_fused_rhs(Ctx* c, const StepParams* dp) {
+  if (!tri_keep_order(c)) {
+    { MIBM_PROF(c, "explicit_int");
+      const dim3 grid(div_up(c->g.n1m, kExX), div_up(c->g.n2m, kExY), div_up(c->g.n3m, kExZ)), block(kExX, kExY, kExZ);
+      RuSet ru;
+      for (int w = 0; w < 4; ++w) ru.r[w] = ru_of(c, w);
+      const StencilArgs a = make_args(c);
+      if (equal_spacings(c->g)) explicit_int_kernel<0><<<grid, block, 0, c->stream>>>(a, dp, ru, c->rhs4);
+      else if (c->g.dx1 == c->g.dx2) explicit_int_kernel<1><<<grid, block, 0, c->stream>>>(a, dp, ru, c->rhs4);
+      else explicit_int_kernel<2><<<grid, block, 0, c->stream>>>(a, dp, ru, c->rhs4); }
+    ++c->launches;
+    MIBM_LAUNCH_CHECK(c, "explicit_int");
+    return;
+  }
   adv_products_launch<double>(c, c->prod);
   for (int w = 0; w < 4; ++w) {
     { MIBM_PROF(c, "fused_rhs");
