@@ -137,7 +137,7 @@ static bool step_prepare(Ctx* c) {
       return false;
   }
   if (!tri_step_fill(c, bd, f32)) return false;
-  if (!fft_prepare(c, false) || (f32 && !fft_prepare(c, true))) return false;
+  if (!fft_prepare(c, false, tri_keep_order(c)) || (f32 && !fft_prepare(c, true))) return false;
   if (moving_body(c)) {
     if (!rigid_ensure(c)) return false;
     rigid_pack(c, c->hrigid_in, false);

@@ -383,7 +383,7 @@ void k_updvp_prcalc(Ctx* c, const StepParams* dp, const double* mean3);
 void k_add_field(Ctx* c, double* q, const double* r);
 double k_cfl(Ctx* c);
 void k_cfl_async(Ctx* c, double* out);
-bool fft_prepare(Ctx* c, bool f32);
+bool fft_prepare(Ctx* c, bool f32, bool keep_order = false);
 void tri_build_table(int n, double betadx, std::vector<double>& t);
 size_t tri_ext_len(int n, int m);
 void tri_build_ext_table(int n, int m, double betadx, std::vector<double>& out);

@@ -14,8 +14,8 @@
 //   X' c2r along x   two Hermitian half-rows packed as one complex line
 // Line FFTs are Stockham autosort transforms with radix-4/2/3 stages
 // (n = 2^a 3^b), twiddles e^{-2 pi i m/n} tabulated on the host in FP64 and
-// staged in shared memory.  The FP64 form's x and y passes run on the integer
-// pipe (fft_int.cuh); the others, and those of a step that keeps its order of
+// staged in shared memory.  The FP64 form's x and y passes and its z lines run on
+// the integer pipe (fft_int.cuh, fft_int_z.cu); the others, and those of a step that keeps its order of
 // operations, run the kernel of fft_fast.cuh specialised for their line length
 // when the length has one, else the kernels below (any length, run-time plan).  Unnormalised, FFTW sign convention
 // (forward = e^{-i...}).  The c2r pass drops the imaginary parts of the
@@ -232,6 +232,8 @@ struct FftCache {
   Ctx* c = nullptr;
   double2 *twx = nullptr, *twy = nullptr, *twz = nullptr;
   int4* itw = nullptr;      // FftArgs::itw
+  void* itz = nullptr;      // FftArgs::itz
+  bool itz_done = false;
   float2 *ftwx = nullptr, *ftwy = nullptr, *ftwz = nullptr;
   float *fak1 = nullptr, *fak2 = nullptr, *fak3 = nullptr;
   double* eig = nullptr;    // FftArgs::eig, FP64 (built at the first FP64 solve)
@@ -259,7 +261,7 @@ __global__ void eig_kernel(Grid g, const double* __restrict__ ak1, const double*
   }
 }
 
-// z-line tables.  After the x and y transforms, the z pass solves, for each
+// z-line tables (of the FP64 passes; fft_int_z.cu has its own).  After the x and y transforms, the z pass solves, for each
 // line (kx, ky), (D_zz - lambda) phi = r with D_zz = dx3q (phi[k+1] - 2 phi[k]
 // + phi[k-1]) periodic and lambda = ak1(kx) + ak2(ky): in Fourier space along z
 // that is the division of phcalc.f90:57 (the eigenvalues of D_zz are -ak3,
@@ -330,6 +332,19 @@ static bool make_ztri(Ctx* c, FftCache* f, bool f32) {
   }
   f->zt_lines = NT;
   f->zt_m = zm;
+  return true;
+}
+
+// the integer-pipe z lines' constants, where the scheme covers the grid
+static bool make_itz(Ctx* c, FftCache* f) {
+  if (f->itz_done) return true;
+  std::vector<char> t;
+  intfft_z_table(c->g, t);
+  if (!t.empty()) {
+    if (!cuda_ok(c, cudaMalloc(&f->itz, t.size()), "z-line tables")) return false;
+    cudaMemcpy(f->itz, t.data(), t.size(), cudaMemcpyHostToDevice);
+  }
+  f->itz_done = true;
   return true;
 }
 
@@ -414,7 +429,7 @@ void fft_free(Ctx* c) {
   for (size_t q = 0; q < g_fft.size(); ++q)
     if (g_fft[q].c == c) {
       FftCache& f = g_fft[q];
-      cudaFree(f.twx); cudaFree(f.twy); cudaFree(f.twz); cudaFree(f.itw);
+      cudaFree(f.twx); cudaFree(f.twy); cudaFree(f.twz); cudaFree(f.itw); cudaFree(f.itz);
       cudaFree(f.ftwx); cudaFree(f.ftwy); cudaFree(f.ftwz);
       cudaFree(f.fak1); cudaFree(f.fak2); cudaFree(f.fak3);
       cudaFree(f.eig); cudaFree(f.feig); cudaFree(f.ztri); cudaFree(f.fztri);
@@ -423,11 +438,16 @@ void fft_free(Ctx* c) {
     }
 }
 
-// Builds the tables the solve of the given form needs before a step is
+// Builds the tables the solve of the given form needs (keep_order: k_phcalc) before a step is
 // launched (and possibly captured into a graph).
-bool fft_prepare(Ctx* c, bool f32) {
+bool fft_prepare(Ctx* c, bool f32, bool keep_order) {
   FftCache* fc = fft_of(c);
-  return make_eig(c, fc, f32) && (f32 || make_ztri(c, fc, false));
+  if (f32) return make_eig(c, fc, true);
+  if (!keep_order) {
+    if (!make_itz(c, fc)) return false;
+    if (fc->itz) return true;
+  }
+  return make_eig(c, fc, false) && make_ztri(c, fc, false);
 }
 
 // the integer-pipe passes of the FP64 form; false: not wanted or no instance
@@ -444,6 +464,15 @@ static bool int_x_inv(Ctx* c, const FftArgs<C>& F, const C* spec, typename Real<
 template <typename C>
 static bool int_y(Ctx* c, const FftArgs<C>& F, C* spec, int sign) {
   if constexpr (sizeof(C) == 16) return F.itw && intfft_y(c, F.itw, spec, sign);
+  return false;
+}
+
+template <typename C>
+static bool int_z(Ctx* c, const FftArgs<C>& F, C* spec) {
+  if constexpr (sizeof(C) == 16) {
+    if (F.itz) intfft_z(c, F.itz, spec);
+    return F.itz != nullptr;
+  }
   return false;
 }
 
@@ -468,7 +497,7 @@ static void phcalc_launch(Ctx* c, FftArgs<C> F, const S* src, typename Real<C>::
   { MIBM_PROF(c, f32 ? "fft_y_f32" : "fft_y");
     if (!int_y<C>(c, F, spec, -1) && !fastfft_y<C>(c, F, spec, -1)) fft_y<C><<<gy, 256, smy, c->stream>>>(F, spec, -1); }
   { MIBM_PROF(c, f32 ? "fft_z_solve_f32" : "fft_z_solve");
-    if (!fastfft_z_solve<C>(c, F, spec)) fft_z_solve<C><<<gz, 256, smz, c->stream>>>(F, spec); }
+    if (!int_z<C>(c, F, spec) && !fastfft_z_solve<C>(c, F, spec)) fft_z_solve<C><<<gz, 256, smz, c->stream>>>(F, spec); }
   { MIBM_PROF(c, f32 ? "fft_y_f32" : "fft_y");
     if (!int_y<C>(c, F, spec, +1) && !fastfft_y<C>(c, F, spec, +1)) fft_y<C><<<gy, 256, smy, c->stream>>>(F, spec, +1); }
   { MIBM_PROF(c, f32 ? "fft_x_inv_f32" : "fft_x_inv");
@@ -489,10 +518,11 @@ void k_phcalc(Ctx* c, bool keep_order) {
   F.twx = fc->twx; F.twy = fc->twy; F.twz = fc->twz;
   F.ak1 = c->ak1; F.ak2 = c->ak2; F.ak3 = c->ak3;
   F.inv_nn = 1.0 / ((double)g.n1m * (double)g.n2m * (double)g.n3m);
-  if (!make_eig(c, fc, false) || !make_ztri(c, fc, false)) return;
+  if (!fft_prepare(c, false, keep_order)) return;
   F.eig = fc->eig;
   F.ztri = fc->ztri; F.zt_lines = fc->zt_lines; F.zt_m = fc->zt_m;
   F.itw = keep_order ? nullptr : fc->itw;
+  F.itz = keep_order ? nullptr : fc->itz;
   phcalc_launch<double2, double>(c, F, c->df[MIBM_F_DPH], c->df[MIBM_F_DPH], "phcalc");
 }
 
@@ -513,7 +543,7 @@ void k_phcalc_f32(Ctx* c, const float* src, float* phi) {
   // FP32 transforms cost little on the FP32 pipe: the z pass stays a
   // transform (the tridiagonal lines are latency-bound and slower there)
   F.ztri = nullptr; F.zt_lines = 0; F.zt_m = 0;
-  F.itw = nullptr;
+  F.itw = nullptr; F.itz = nullptr;
   phcalc_launch<float2, float>(c, F, src, phi, "phcalc_f32");
 }
 

@@ -3,6 +3,8 @@
 // fixed line lengths).
 #pragma once
 
+#include <vector>
+
 #include "common.cuh"
 
 namespace mibm {
@@ -54,6 +56,7 @@ struct FftArgs {
   int zt_lines;
   int zt_m;            // chunk length of the chunked z-line tables, 0: one thread per line
   const int4* itw;     // twiddles of the integer-pipe x and y passes (n1m = n2m), nullptr: FP64 passes
+  const void* itz;     // constants of the integer-pipe z lines (fft_int_z.cu), nullptr: eig and ztri
 };
 
 // chunk length of the chunked z-line Poisson solve for `lines` lines of n
@@ -96,6 +99,9 @@ bool fastfft_x_inv(Ctx* c, const FftArgs<C>& F, const C* spec, typename Real<C>:
 bool intfft_x_fwd(Ctx* c, const int4* tw, const double* src, double2* spec);
 bool intfft_x_inv(Ctx* c, const int4* tw, const double2* spec, double* dst);
 bool intfft_y(Ctx* c, const int4* tw, double2* spec, int sign);
+// its z lines (fft_int_z.cu); the table is empty where they do not cover the grid
+void intfft_z_table(const Grid& g, std::vector<char>& out);
+void intfft_z(Ctx* c, const void* tab, double2* spec);
 
 // instances (fft_fast_f64.cu, fft_fast_f32.cu)
 template <> bool fastfft_x_fwd<double2, double>(Ctx*, const FftArgs<double2>&, const double*, double2*);

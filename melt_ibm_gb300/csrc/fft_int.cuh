@@ -20,11 +20,11 @@
 // input, against outputs of about sqrt(n) times its rms: below 2^-55 of them
 // for inputs up to 16 times their rms, less than the rounding of the result.
 // The whole solve against one in extended precision, relative 2-norm of phi /
-// of its gradient, integer and FP64 passes: 32^3 noise 1.1e-15 / 4.9e-16 and
-// 1.1e-15 / 7.8e-16, 64^3 noise 3.4e-15 / 8.6e-16 and 3.4e-15 / 1.2e-15, one
-// spike 3.6e-15 / 8.4e-16 and 3.7e-15 / 1.2e-15, values over nine decades
-// 3.9e-15 / 8.9e-16 and 4.1e-15 / 1.2e-15 (phi: the z lines' error in the
-// lowest modes).  A line that holds an infinity or a NaN comes out as NaN.
+// of its gradient, with the z lines of fft_int_z.cu (the FP64 passes): 32^3 noise
+// 2.9e-16 / 3.4e-16 (1.1e-15 / 7.8e-16), 64^3 noise 2.5e-16 / 4.4e-16 (3.4e-15 /
+// 1.2e-15), one spike 2.3e-16 / 4.1e-16 (3.7e-15 / 1.2e-15), values over nine
+// decades 2.7e-16 / 4.4e-16 (4.1e-15 / 1.2e-15).  A line that holds an infinity
+// or a NaN comes out as NaN.
 // Per pass, FP64 -> integer: 128^3 x forward 61 -> 34, y 60 -> 21, x inverse 60
 // -> 29 us; 192^3 212 -> 92, 192 -> 63, 208 -> 81 us; 108 x 108 x 72 (no
 // compile-time FP64 instance) 45 -> 19, 47 -> 16, 44 -> 19 us.
