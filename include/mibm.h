@@ -436,14 +436,16 @@ int  mibm_diagnostics_get_(double* out);
 /* It runs the same periodic tridiagonal solve as solxi_ in place on       */
 /* `rhs`, a device array in the compact layout x fastest with row pitch    */
 /* `pitch` (elements), n2m rows and n3m planes, on `stream` (NULL = the   */
-/* legacy default stream).  Its only scratch, the line-factor table, is a  */
+/* legacy default stream).  Lines of 2^a 3^b cells (even) with rows on     */
+/* 16-byte boundaries and -0.24 < betadx < 1e12 need no scratch.  That of  */
+/* the others, the line-factor table, is a                                 */
 /* file-scope device array sized for lines up to 512 cells (16.4 KB, held */
 /* by every GPU that loads the library until exit); n1m > 512 (or n3m >    */
 /* 65535) returns MIBM_EINVAL without launching.  The first call on a      */
 /* device looks up that array's device address (once per device, with the */
 /* device current): make that first call before any stream capture.  Each */
-/* call writes the whole table on `stream` with a one-thread kernel and   */
-/* then solves; no host buffer is read.  All calls share the one table:    */
+/* call that needs it writes the whole table on `stream` with a one-thread */
+/* kernel and then solves; no host buffer is read.  These calls share the one table: */
 /* calls whose work can overlap on the GPU race on it.  That includes two  */
 /* calls made one after the other from the host on DIFFERENT streams: the  */
 /* second call's table write can run while the first call's solve still   */

@@ -958,9 +958,8 @@ __device__ __forceinline__ void geo_fix(const double* __restrict__ T, int F, dou
 // factors (five operations per element and shuffle scans); 128^3 35 against 60.
 __host__ __device__ constexpr int geo_cs(int m) { return m % 2 ? m : (m % 4 == 2 ? m : m + 2); }
 template <int M, bool SCALE>
-__global__ void __launch_bounds__(kGeoRowThreads) geo_x_kernel(Grid g, double* __restrict__ rhs,
-                                                               const double* __restrict__ T, int nfield,
-                                                               unsigned magic) {
+__device__ __forceinline__ void geo_x(const Grid& g, double* __restrict__ rhs, const double* __restrict__ T, int nfield,
+                                      unsigned magic) {
   extern __shared__ __align__(16) double geo_sm[];
   __shared__ double sC[kGeoRowThreads], sD[kGeoRowThreads];
   constexpr int CS = geo_cs(M), V = M % 2 ? 1 : 2;
@@ -1050,6 +1049,19 @@ __global__ void __launch_bounds__(kGeoRowThreads) geo_x_kernel(Grid g, double* _
       if (p < total && piece(p, dst, at)) *reinterpret_cast<Vec*>(dst) = *reinterpret_cast<const Vec*>(geo_sm + at);
     }
   });
+}
+template <int M, bool SCALE>
+__global__ void __launch_bounds__(kGeoRowThreads) geo_x_kernel(Grid g, double* __restrict__ rhs,
+                                                               const double* __restrict__ T, int nfield,
+                                                               unsigned magic) {
+  geo_x<M, SCALE>(g, rhs, T, nfield, magic);
+}
+// the same with the constants among the arguments
+struct GeoConst { double v[kGeoLen]; };
+template <int M>
+__global__ void __launch_bounds__(kGeoRowThreads) geo_x_arg_kernel(Grid g, double* __restrict__ rhs,
+                                                                   const __grid_constant__ GeoConst T, unsigned magic) {
+  geo_x<M, true>(g, rhs, T.v, 1, magic);
 }
 
 // y- and z-lines: block = 32 adjacent i (lanes) x G chunks (warps) of one
@@ -1574,18 +1586,22 @@ static void solve_z_launch(Ctx* c, V* rhs, const V* T, const QSet& q, int nfield
 
 // The geo_* solves; own_scale: x and y lines apply their own scale
 // (drop-in solves), else the z solve's constants hold the product of the three
+struct GeoRows { unsigned blocks, magic; size_t smem; };
+static GeoRows geo_rows(const Grid& g, int m, int nfield) {
+  const int G = g.n1m / m, R = kGeoRowThreads / G;
+  const unsigned nv = g.n1m / (m % 2 ? 1 : 2);
+  return GeoRows{(unsigned)div_up((size_t)g.n2m * g.n3m * nfield, R), (unsigned)((0x100000000ull + nv - 1) / nv),
+                 (size_t)R * G * geo_cs(m) * sizeof(double)};
+}
 static bool geo_x_launch(Ctx* c, double* rhs, const double* T, int nfield, bool own_scale) {
   const int m = geo_chunk(c, 0);
   if (!m) return false;
-  const int G = c->g.n1m / m, R = kGeoRowThreads / G;
-  const size_t sm = (size_t)R * G * geo_cs(m) * sizeof(double);
-  const unsigned blocks = div_up((size_t)c->g.n2m * c->g.n3m * nfield, R);
+  const GeoRows s = geo_rows(c->g, m, nfield);
   {
     MIBM_PROF(c, "solve_x");
-    const unsigned nv = c->g.n1m / (m % 2 ? 1 : 2), magic = (unsigned)((0x100000000ull + nv - 1) / nv);
 #define GX(M)                                                                                                 \
-  if (own_scale) geo_x_kernel<M, true><<<blocks, kGeoRowThreads, sm, c->stream>>>(c->g, rhs, T, nfield, magic); \
-  else geo_x_kernel<M, false><<<blocks, kGeoRowThreads, sm, c->stream>>>(c->g, rhs, T, nfield, magic)
+  if (own_scale) geo_x_kernel<M, true><<<s.blocks, kGeoRowThreads, s.smem, c->stream>>>(c->g, rhs, T, nfield, s.magic); \
+  else geo_x_kernel<M, false><<<s.blocks, kGeoRowThreads, s.smem, c->stream>>>(c->g, rhs, T, nfield, s.magic)
     MIBM_GEO_CASES(m, GX)
 #undef GX
   }
@@ -1737,9 +1753,11 @@ float tri_time_direction(Ctx* c, int dir, int m, bool f32, int reps) {
 // ---------------------------------------------------------------------
 // Allocation-free x-line solve (mibm_solxi_noalloc, see include/mibm.h).
 //
-// Same kernel and same factor table as the library's x-line solves, but the
-// table lives in a file-scope device array instead of memory the library
-// allocates.  Every GPU that loads the library holds this array until the
+// Lines that the geo_* kernels cover run them with the constants (formed on the
+// host in about 1 us) among the kernel's arguments: no scratch at all.  96 x 96 x
+// 64 cells: 92 -> 23 us with a device copy of the input, 60 us of it the table.
+// The others use the x-line kernel of the drop-in solves and its factor table,
+// which lives in a file-scope device array instead of memory the library allocates.  Every GPU that loads the library holds this array until the
 // process exits.  The table is written on the device by a one-thread kernel
 // on the caller's stream (tri_factors, the function build_table runs on the
 // host, bit for bit), so the call touches no host buffer.
@@ -1812,12 +1830,24 @@ extern "C" int mibm_solxi_noalloc(double* rhs, int n1m, int n2m, int n3m, int pi
   Grid g{};
   g.n1m = n1m; g.n2m = n2m; g.n3m = n3m; g.P = pitch;
   g.plane = (size_t)pitch * n2m; g.cells = g.plane * n3m;
+  cudaStream_t st = (cudaStream_t)stream;
+  // even chunks move 16 bytes at a time: rows on 16-byte boundaries
+  const size_t lines = (size_t)n2m * n3m;
+  const int m = lines <= 0x7fffffff ? geo_chunk_line(n1m, (int)lines) : 0;
+  if (m && geo_ok(betadx) && (m % 2 || ((uintptr_t)rhs % 16 == 0 && pitch % 2 == 0))) {
+    const GeoRows s = geo_rows(g, m, 1);
+    GeoConst T;
+    fill_geo(n1m, m, betadx, geo_scale(betadx), T.v);
+#define GX(M) geo_x_arg_kernel<M><<<s.blocks, kGeoRowThreads, s.smem, st>>>(g, rhs, T, s.magic)
+    MIBM_GEO_CASES(m, GX)
+#undef GX
+    return cudaGetLastError() == cudaSuccess ? MIBM_OK : MIBM_ECUDA;
+  }
   size_t sm = ((size_t)kLines * (n1m + 1) + 4 * (size_t)n1m + 4) * sizeof(double);
   if (sm > 48 * 1024 &&
       cudaFuncSetAttribute((const void*)solve_x_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
           cudaSuccess)
     return MIBM_ECUDA;
-  cudaStream_t st = (cudaStream_t)stream;
   // the line-independent factors, in stream order ahead of the solve
   tri_factors_kernel<<<1, 1, 0, st>>>(n1m, betadx, table);
   if (cudaGetLastError() != cudaSuccess) return MIBM_ECUDA;
