@@ -377,7 +377,7 @@ void k_cast_f2d(Ctx* c, size_t n, const float* a, double* b);
 void k_cast_d2f(Ctx* c, size_t n, const double* a, float* b);
 void k_divmax(Ctx* c, unsigned long long* out);
 void k_divg(Ctx* c, const StepParams* dp);
-void k_updvp(Ctx* c, const StepParams* dp, const double* mean3 = nullptr);
+void k_updvp(Ctx* c, const StepParams* dp);
 void k_prcalc(Ctx* c, const StepParams* dp);
 void k_updvp_prcalc(Ctx* c, const StepParams* dp, const double* mean3);
 void k_add_field(Ctx* c, double* q, const double* r);

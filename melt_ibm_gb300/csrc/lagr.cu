@@ -802,46 +802,72 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// per-block partial sums of up to 3 fields over the owned cells, fixed order
-__global__ void field_sum_kernel(Grid g, const double* __restrict__ a, const double* __restrict__ b,
-                                 const double* __restrict__ cc, double* __restrict__ part) {
-  int j = blockIdx.x, k = blockIdx.y;
+// Mean of the three force fields over the owned cells -> mean3[0..2], in a fixed
+// order: kFieldMeanBlocks blocks over strided rows, block sums as in seg_mean_kernel,
+// added by the last block to finish (the ticket in mean3's slot 7).  A force is
+// zero off the markers' cages, so a warp whose pieces are all zero adds nothing
+// (an FP64 addition costs it 16 clocks).
+// Bound by the reads (128^3, 50 MB): 119 -> 25 us against one block and three
+// shuffle trees per row and a second launch.
+constexpr int kFieldMeanBlocks = 152 * 4;
+__global__ void __launch_bounds__(256) field_mean_kernel(Grid g, const double* __restrict__ a,
+                                                         const double* __restrict__ b, const double* __restrict__ cc,
+                                                         double* __restrict__ part, double ncell,
+                                                         double* __restrict__ mean3) {
+  constexpr int kU = 4;
+  const unsigned FULL = 0xffffffffu;
+  __shared__ double ws[8][3];
+  __shared__ bool last;
+  const double* f[3] = {a, b, cc};
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int warps = gridDim.x * 8, rows = g.n2m * g.n3m, per = (g.n1m + 31) / 32;
   double s[3] = {0, 0, 0};
-  for (int i = threadIdx.x; i < g.n1m; i += blockDim.x) {
-    size_t c0 = cidx(g, i, j, k);
-    s[0] += a[c0]; s[1] += b[c0]; s[2] += cc[c0];
-  }
-  __shared__ double sm[3][32];
-  for (int q = 0; q < 3; ++q) {
-    double v = warp_sum(s[q]);
-    if ((threadIdx.x & 31) == 0) sm[q][threadIdx.x >> 5] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    int nw = blockDim.x >> 5;
-    for (int q = 0; q < 3; ++q) {
-      double v = (threadIdx.x < nw) ? sm[q][threadIdx.x] : 0.0;
-      v = warp_sum(v);
-      if (threadIdx.x == 0) part[3 * ((size_t)j + (size_t)g.n2m * k) + q] = v;
+  // a warp's pieces of 32 cells, kU of each field in flight
+  for (int p0 = blockIdx.x * 8 + warp; p0 < rows * per; p0 += kU * warps) {
+    double v[3][kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int p = p0 + u * warps, row = p / per, i = (p - row * per) * 32 + lane;
+      const bool ok = p < rows * per && i < g.n1m;
+      const size_t c0 = ok ? cidx(g, i, row % g.n2m, row / g.n2m) : 0;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) v[q][u] = ok ? f[q][c0] : 0.0;
     }
+    long long bits = 0;
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) bits |= __double_as_longlong(v[q][u]);
+    if (!__any_sync(FULL, bits << 1 != 0)) continue;
+#pragma unroll
+    for (int u = 0; u < kU; ++u)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) s[q] += v[q][u];
   }
-}
-
-// sum m triples in fixed order, divide by the cell count -> mean3
-__global__ void mean3_kernel(const double* __restrict__ part, int m, double ncell, double* __restrict__ out) {
-  __shared__ double sm[3][1024];
-  double s[3] = {0, 0, 0};
-  for (int t = threadIdx.x; t < m; t += blockDim.x)
-    for (int q = 0; q < 3; ++q) s[q] += part[3 * (size_t)t + q];
-  for (int q = 0; q < 3; ++q) sm[q][threadIdx.x] = s[q];
+  for (int q = 0; q < 3; ++q) {
+    const double v = warp_sum(s[q]);
+    if (lane == 0) ws[warp][q] = v;
+  }
   __syncthreads();
-  for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-    if (threadIdx.x < off)
-      for (int q = 0; q < 3; ++q) sm[q][threadIdx.x] += sm[q][threadIdx.x + off];
-    __syncthreads();
+  if (threadIdx.x < 3) {
+    double v = ws[0][threadIdx.x];
+    for (int w = 1; w < 8; ++w) v += ws[w][threadIdx.x];
+    part[3 * (size_t)blockIdx.x + threadIdx.x] = v;
   }
-  if (threadIdx.x == 0)
-    for (int q = 0; q < 3; ++q) out[q] = sm[q][0] / ncell;
+  unsigned* ticket = reinterpret_cast<unsigned*>(mean3 + 7);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (warp < 3) {
+    double v = 0.0;
+    for (int q = lane; q < (int)gridDim.x; q += 32) v += __ldcg(part + 3 * (size_t)q + warp);
+    v = warp_sum(v);
+    if (lane == 0) mean3[warp] = v / ncell;
+  }
+  if (threadIdx.x == 0) *ticket = 0u;
 }
 
 __device__ __forceinline__ void cross3(double r[3], const double x[3], const double y[3]) {
@@ -2483,14 +2509,12 @@ void lagr_mls_force(Ctx* c, const StepParams*, bool) {
 void lagr_velforce(Ctx* c) {
   if (!ensure_lag_buffers(c)) return;
   LagState* s = lag_of(c);
-  dim3 grid(c->g.n2m, c->g.n3m);
-  { MIBM_PROF(c, "field_sum");
-    field_sum_kernel<<<grid, 128, 0, c->stream>>>(c->g, c->df[MIBM_F_FORXC], c->df[MIBM_F_FORYC],
-                                                  c->df[MIBM_F_FORZC], c->red + kRedPart); }
-  double ncell = (double)c->g.n1m * (double)c->g.n2m * (double)c->g.n3m;
-  { MIBM_PROF(c, "mean3");
-    mean3_kernel<<<1, 1024, 0, c->stream>>>(c->red + kRedPart, c->g.n2m * c->g.n3m, ncell, s->mean3); }
-  c->launches += 2;
+  const double ncell = (double)c->g.n1m * (double)c->g.n2m * (double)c->g.n3m;
+  { MIBM_PROF(c, "field_mean");
+    field_mean_kernel<<<std::min(kFieldMeanBlocks, c->g.n2m * c->g.n3m), 256, 0, c->stream>>>(c->g, c->df[MIBM_F_FORXC], c->df[MIBM_F_FORYC],
+                                                               c->df[MIBM_F_FORZC], c->red + kRedPart, ncell,
+                                                               s->mean3); }
+  c->launches += 1;
   k_velforce_apply(c, s->mean3);
 }
 

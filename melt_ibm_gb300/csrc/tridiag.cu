@@ -1757,10 +1757,11 @@ float tri_time_direction(Ctx* c, int dir, int m, bool f32, int reps) {
 // host in about 1 us) among the kernel's arguments: no scratch at all.  96 x 96 x
 // 64 cells: 92 -> 23 us with a device copy of the input, 60 us of it the table.
 // The others use the x-line kernel of the drop-in solves and its factor table,
-// which lives in a file-scope device array instead of memory the library allocates.  Every GPU that loads the library holds this array until the
-// process exits.  The table is written on the device by a one-thread kernel
-// on the caller's stream (tri_factors, the function build_table runs on the
-// host, bit for bit), so the call touches no host buffer.
+// which lives in a file-scope device array instead of memory the library
+// allocates: every GPU that loads the library holds it until the process exits.
+// It is written on the device by a one-thread kernel on the caller's stream
+// (tri_factors, the function build_table runs on the host, bit for bit), so
+// that no host buffer is read.
 // ---------------------------------------------------------------------
 constexpr int kNoAllocMaxN = 512;                      // longest x-line
 constexpr int kNoAllocTable = 4 * kNoAllocMaxN + 4;    // [a|b|q|s]*n + 4 scalars
