@@ -41,6 +41,8 @@ struct LagArgs {
   int nf, nv, coff, clen;
   const double* xc; const double* xm; const double* yc; const double* ym; const double* zc; const double* zm;
   double wcon, wscl;
+  // the weights' divisors and their reciprocals: wscl/dx per direction, wcon, wcon^2
+  double wr[3], iwr[3], iwcon, wc2, iwc2, dcoef;   // dcoef: -2 / wcon^2
 };
 
 static LagArgs lag_args(Ctx* c) {
@@ -48,6 +50,12 @@ static LagArgs lag_args(Ctx* c) {
   a.g = c->g; a.nf = c->maxnf; a.nv = c->maxnv; a.coff = c->coord_off; a.clen = 3 * c->coord_off;
   a.xc = c->xc; a.xm = c->xm; a.yc = c->yc; a.ym = c->ym; a.zc = c->zc; a.zm = c->zm;
   a.wcon = c->S(MIBM_S_WCON); a.wscl = c->S(MIBM_S_WSCL);
+  a.wr[0] = a.wscl / c->g.dx1; a.wr[1] = a.wscl / c->g.dx2; a.wr[2] = a.wscl / c->g.dx3;
+  for (int d = 0; d < 3; ++d) a.iwr[d] = 1.0 / a.wr[d];
+  a.iwcon = 1.0 / a.wcon;
+  a.wc2 = a.wcon * a.wcon;
+  a.iwc2 = 1.0 / a.wc2;
+  a.dcoef = -2.0 / a.wc2;
   return a;
 }
 
@@ -70,58 +78,103 @@ __device__ __forceinline__ double coord(const LagArgs& A, int dir, int sel, int 
 // Gaussian weight and its radial derivative (geom.f90:24-53).  exp is the
 // written-out mls_exp (mls_exp.h), shared with the oracle, so that the
 // plain form's MLS construction gives the oracle's bits.
-__device__ __forceinline__ double mls_gaussian(double r, double rcoef) { return (r > 1.0) ? 0.0 : mls_exp(-sqd(r / rcoef)); }
-__device__ __forceinline__ double mls_gauss_deriv(double r, double rcoef) {
-  return (r > 1.0) ? 0.0 : -2.0 * r / sqd(rcoef) * mls_exp(-sqd(r / rcoef));
+// a / b, correctly rounded, for a constant b whose reciprocal y has been rounded
+// once: after one correction the quotient is within an ulp, from where the
+// second rounds it correctly (Markstein, Computation of elementary functions on
+// the IBM RISC System/6000, 1990).  Five FP64 operations; quotient and
+// remainder must not underflow (0 does not).
+__device__ __forceinline__ double div_const(double a, double b, double y) {
+  const double q = a * y, q1 = fma(fma(-b, q, a), y, q);
+  return fma(fma(-b, q1, a), y, q1);
 }
-
+// limit < x <= infinity for x >= 0 (false for a NaN), limit >= 0: an FP64
+// comparison issues at the FP64 rate, one of the bits does not
+__device__ __forceinline__ bool above(double x, double limit) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x),
+                           l = (unsigned long long)__double_as_longlong(limit);
+  return b > l && b <= 0x7ff0000000000000ull;
+}
+// |pos - pc| / (wscl/dx) along axis d, or 2 where it is above 4
+__device__ __forceinline__ double axis_norp(const LagArgs& A, int d, double diff) {
+  const double a = fabs(diff);
+  return above(a, 4.0 * A.wr[d]) ? 2.0 : div_const(a, A.wr[d], A.iwr[d]);
+}
+// the Gaussian weight of norp (mlsWeight.f90): 0 above 1
+__device__ __forceinline__ double mls_gaussian(const LagArgs& A, double r) {
+  return above(r, 1.0) ? 0.0 : mls_exp(-sqd(div_const(r, A.wcon, A.iwcon)));
+}
 // In-place inverse of a 4x4 column-major matrix: LU with partial pivoting
 // (dgetrf semantics, first maximal pivot) and inversion from the factors
 // (dgetri).  Returns false if a pivot is exactly zero.
-__device__ bool inv4(double* a) {
-  const int n = 4;
+__device__ __forceinline__ bool inv4(double* a) {
+  constexpr int n = 4;
   int ipiv[4];
+  double rp[4];                                   // 1 / pivot, used by both factors
+#pragma unroll
   for (int j = 0; j < n; ++j) {
     int p = j;
     double amax = fabs(a[j + n * j]);
+#pragma unroll
     for (int i = j + 1; i < n; ++i)
-      if (fabs(a[i + n * j]) > amax) { amax = fabs(a[i + n * j]); p = i; }
+      if (above(fabs(a[i + n * j]), amax)) { amax = fabs(a[i + n * j]); p = i; }
     ipiv[j] = p;
-    if (a[p + n * j] == 0.0) return false;
-    if (p != j)
-      for (int cc = 0; cc < n; ++cc) { double t = a[j + n * cc]; a[j + n * cc] = a[p + n * cc]; a[p + n * cc] = t; }
-    double r = 1.0 / a[j + n * j];
+    if (__double_as_longlong(amax) == 0) return false;
+#pragma unroll
+    for (int i = j + 1; i < n; ++i)
+#pragma unroll
+      for (int cc = 0; cc < n; ++cc) {            // rows j and p change places, in registers
+        const double t = a[j + n * cc], u = a[i + n * cc];
+        a[j + n * cc] = p == i ? u : t;
+        a[i + n * cc] = p == i ? t : u;
+      }
+    const double r = 1.0 / a[j + n * j];
+    rp[j] = r;
+#pragma unroll
     for (int i = j + 1; i < n; ++i) a[i + n * j] *= r;
+#pragma unroll
     for (int cc = j + 1; cc < n; ++cc) {
       double t = a[j + n * cc];
+#pragma unroll
       for (int i = j + 1; i < n; ++i) a[i + n * cc] -= t * a[i + n * j];
     }
   }
+#pragma unroll
   for (int j = 0; j < n; ++j) {
-    a[j + n * j] = 1.0 / a[j + n * j];
-    double ajj = -a[j + n * j];
+    a[j + n * j] = rp[j];
+    const double ajj = -rp[j];
+#pragma unroll
     for (int i = 0; i < j; ++i) {
-      double s = 0;
-      for (int k = i; k < j; ++k) s += a[i + n * k] * a[k + n * j];
+      double s = a[i + n * i] * a[i + n * j];
+#pragma unroll
+      for (int k = i + 1; k < j; ++k) s += a[i + n * k] * a[k + n * j];
       a[i + n * j] = s;
     }
+#pragma unroll
     for (int i = 0; i < j; ++i) a[i + n * j] *= ajj;
   }
-  double work[4];
-  for (int j = n - 1; j >= 0; --j) {
-    for (int i = j + 1; i < n; ++i) { work[i] = a[i + n * j]; a[i + n * j] = 0.0; }
-    if (j < n - 1)
-      for (int i = 0; i < n; ++i) {
-        double s = 0;
-        for (int k = j + 1; k < n; ++k) s += a[i + n * k] * work[k];
-        a[i + n * j] -= s;
-      }
-  }
+#pragma unroll
   for (int j = n - 2; j >= 0; --j) {
-    int jp = ipiv[j];
-    if (jp != j)
-      for (int i = 0; i < n; ++i) { double t = a[i + n * j]; a[i + n * j] = a[i + n * jp]; a[i + n * jp] = t; }
+    double work[4];
+#pragma unroll
+    for (int i = j + 1; i < n; ++i) { work[i] = a[i + n * j]; a[i + n * j] = 0.0; }
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      double s = a[i + n * (j + 1)] * work[j + 1];
+#pragma unroll
+      for (int k = j + 2; k < n; ++k) s += a[i + n * k] * work[k];
+      a[i + n * j] -= s;
+    }
   }
+#pragma unroll
+  for (int j = n - 2; j >= 0; --j)
+#pragma unroll
+    for (int c = j + 1; c < n; ++c)
+#pragma unroll
+      for (int i = 0; i < n; ++i) {               // columns j and ipiv[j] change places
+        const double t = a[i + n * j], u = a[i + n * c];
+        a[i + n * j] = ipiv[j] == c ? u : t;
+        a[i + n * c] = ipiv[j] == c ? t : u;
+      }
   return true;
 }
 
@@ -189,6 +242,38 @@ __device__ __forceinline__ CageSpec cage_spec(int comp) {
   return CageSpec{0, 1, 1, 1, 1, false};             // xm, ym, zm ; pind(1), pind(2)
 }
 
+// One z layer of the cage added to the moment sums M = sum_n w_n p_n p_n^T in the
+// reference's order (rank-one updates (w p_cc) p_r, nodes in cage order), the
+// FIRST into empty sums; TWICE for the gradient's second layer, whose values the
+// repeated layer of mls_heatFlux.f90:213 has again.  Row 0 of column cc sums
+// what row cc of column 0 does and is left to lit_symmetric.
+template <bool FIRST, bool TWICE = !FIRST>
+__device__ __forceinline__ void lit_layer(const double (&w)[9], const double (&x)[3], const double (&y)[3], double z,
+                                          double (&M)[16]) {
+#pragma unroll
+  for (int cc = 0; cc < 4; ++cc) {
+    double t[9];
+#pragma unroll
+    for (int n = 0; n < 9; ++n) t[n] = cc == 0 ? w[n] : w[n] * (cc == 1 ? x[n % 3] : cc == 2 ? y[n / 3] : z);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (r == 0 && cc > 0) continue;
+      double p[9];
+#pragma unroll
+      for (int n = 0; n < 9; ++n) p[n] = r == 0 ? t[n] : t[n] * (r == 1 ? x[n % 3] : r == 2 ? y[n / 3] : z);
+      double s = FIRST ? p[0] : M[r + 4 * cc] + p[0];
+#pragma unroll
+      for (int n = 1; n < 9; ++n) s = s + p[n];
+      if (TWICE) {
+#pragma unroll
+        for (int n = 0; n < 9; ++n) s = s + p[n];
+      }
+      M[r + 4 * cc] = s;
+    }
+  }
+}
+__device__ __forceinline__ void lit_symmetric(double (&M)[16]) { M[4] = M[1]; M[8] = M[2]; M[12] = M[3]; }
+
 // The reference's MLS shape functions at pos for the 27-point cage centred on
 // (i0, j0, k0) with per-axis staggering sx, sy, sz (mls_shape of wght1/2/3/
 // temp, mlsWeight.f90:48-412, and of wght_press, mls_structLoads.f90:271-
@@ -207,24 +292,21 @@ __device__ bool shape_lit(const LagArgs& A, const double pos[3], int i0, int j0,
     cz[q] = coord(A, 2, sz, k0 - 1 + q);
     cy[q] = coord(A, 1, sy, j0 - 1 + q);
     cx[q] = coord(A, 0, sx, i0 - 1 + q);
-    wz[q] = mls_gaussian(fabs(cz[q] - pos[2]) / (A.wscl / g.dx3), A.wcon);
-    wy[q] = mls_gaussian(fabs(cy[q] - pos[1]) / (A.wscl / g.dx2), A.wcon);
-    wx[q] = mls_gaussian(fabs(cx[q] - pos[0]) / (A.wscl / g.dx1), A.wcon);
+    wz[q] = mls_gaussian(A, axis_norp(A, 2, cz[q] - pos[2]));
+    wy[q] = mls_gaussian(A, axis_norp(A, 1, cy[q] - pos[1]));
+    wx[q] = mls_gaussian(A, axis_norp(A, 0, cx[q] - pos[0]));
   }
-  double Am[16];
-  for (int q = 0; q < 16; ++q) Am[q] = 0.0;
-  for (int kk = 0; kk < 3; ++kk)
-    for (int jj = 0; jj < 3; ++jj) {
-      double w23 = wy[jj] * wz[kk];
-      for (int ii = 0; ii < 3; ++ii) {
-        double wtx = wx[ii] * w23;
-        double pk[4] = {1.0, cx[ii], cy[jj], cz[kk]};
-        for (int cc = 0; cc < 4; ++cc) {
-          double tt = wtx * pk[cc];
-          for (int r = 0; r < 4; ++r) Am[r + 4 * cc] = Am[r + 4 * cc] + tt * pk[r];
-        }
-      }
-    }
+  double Am[16], w[9];
+  auto layer = [&](int kk) {
+    for (int n = 0; n < 9; ++n) w[n] = wx[n % 3] * (wy[n / 3] * wz[kk]);
+  };
+  layer(0);
+  lit_layer<true>(w, cx, cy, cz[0], Am);
+  layer(1);
+  lit_layer<false, false>(w, cx, cy, cz[1], Am);
+  layer(2);
+  lit_layer<false, false>(w, cx, cy, cz[2], Am);
+  lit_symmetric(Am);
   if (!inv4(Am)) return false;
   double ptxA[4];
   for (int cc = 0; cc < 4; ++cc) {
@@ -270,18 +352,45 @@ __global__ void mls_weight_kernel(LagArgs A, const double* __restrict__ tri_bar,
 // norp = |pos - pc| / (wscl/dx); W = gaussian(norp); dW = 0 at norp < eps,
 // else gauss_deriv(norp) * ((pos - pc) / |pos - pc| / (wscl/dx)).  The
 // Gaussian's exp is evaluated once for both (the same value either way).
-__device__ __forceinline__ void lit_axis_weight(const LagArgs& A, double pos, double pc, double dx, double eps,
-                                                double& W, double& dW) {
+__device__ __forceinline__ void lit_axis_weight(const LagArgs& A, int d, double pos, double pc, double& W, double& dW) {
+  const double eps = 2.220446049250313e-16;       // EPSILON(1.0d0)
   const double diff = pos - pc;
-  const double norp = fabs(diff) / (A.wscl / dx);
-  if (norp > 1.0) {
+  const double norp = axis_norp(A, d, diff);
+  if (above(norp, 1.0)) {
     W = 0.0;
     dW = 0.0;
     return;
   }
-  const double e = mls_exp(-sqd(norp / A.wcon));
+  const double e = mls_exp(-sqd(div_const(norp, A.wcon, A.iwcon)));
   W = e;
-  dW = (norp < eps) ? 0.0 : (-2.0 * norp / sqd(A.wcon) * e) * (diff / fabs(diff) / (A.wscl / dx));
+  // (pos - pc) / |pos - pc| is +-1
+  dW = __double_as_longlong(norp) < __double_as_longlong(eps)
+           ? 0.0 : (div_const(-2.0 * norp, A.wc2, A.iwc2) * e) * copysign(A.iwr[d], diff);
+}
+
+// weights of a layer's nodes: of A (D < 0), of dA_d
+__device__ __forceinline__ void lit_node_weights(int d, const double (&W0)[3], const double (&dW0)[3],
+                                                 const double (&W1)[3], const double (&dW1)[3], double W2, double dW2,
+                                                 double (&w)[9]) {
+#pragma unroll
+  for (int n = 0; n < 9; ++n) {
+    const int i = n % 3, j = n / 3;
+    w[n] = d < 0 ? W0[i] * (W1[j] * W2)
+         : d == 0 ? (dW0[i] * W1[j]) * W2 : d == 1 ? (W0[i] * dW1[j]) * W2 : (W0[i] * W1[j]) * dW2;
+  }
+}
+
+// dgam . (wt p) + gam . (dw p) of a layer's nodes
+__device__ __forceinline__ void lit_node_values(const double (&wt)[9], const double (&dw)[9], const double (&dgam)[4],
+                                                const double (&gam)[4], const double (&x)[3], const double (&y)[3],
+                                                double z, double (&v)[9]) {
+#pragma unroll
+  for (int n = 0; n < 9; ++n) {
+    const double px = x[n % 3], py = y[n / 3];
+    const double t1 = ((dgam[0] * wt[n] + dgam[1] * (wt[n] * px)) + dgam[2] * (wt[n] * py)) + dgam[3] * (wt[n] * z);
+    const double t2 = ((gam[0] * dw[n] + gam[1] * (dw[n] * px)) + gam[2] * (dw[n] * py)) + gam[3] * (dw[n] * z);
+    v[n] = t1 + t2;
+  }
 }
 
 // The reference's MLS gradient at a probe, literally (wght_gradT,
@@ -298,40 +407,34 @@ __device__ __forceinline__ void lit_axis_weight(const LagArgs& A, double pos, do
 // (wght_grad_field) in its order, so the two agree bit for bit.  B and dB are
 // not stored: each entry is a product of per-axis weight factors and a basis
 // entry, recomputed where it is used from the same factors in the same order
-// (the same bits); dA_d is accumulated in its own pass per direction.
+// (the same bits); dA_d is accumulated in its own pass per direction.  The
+// repeated layer has the middle one's coordinates and weights, so its products
+// are not formed again.
 // Returns false on a singular A.
 __device__ bool probe_grad_lit(const LagArgs& A, const double pos[3], int pi1, int pi2, int sx, int sy, int sz,
                                bool knint, const double* __restrict__ q, double grad[3]) {
   const Grid& g = A.g;
-  const double eps = 2.220446049250313e-16;       // EPSILON(1.0d0)
   const double ptx[4] = {1.0, pos[0], pos[1], pos[2]};
   const int k1 = knint ? fnint(pos[2] * g.dx3) + 1 : ffloor(pos[2] * g.dx3) + 1;
-  const int kin[3] = {k1 - 1, k1, k1};
   const int k1w = fmod_pos(k1 - 1, g.n3m) + 1;
   const int keul[3] = {k1w - 1, k1w, k1w + 1};
-  double pc[3][3], W[3][3], dW[3][3];             // [axis][point]
+  double x[3], y[3], z[2], W0[3], W1[3], W2[2], dW0[3], dW1[3], dW2[2];
   for (int r = 0; r < 3; ++r) {
-    pc[0][r] = coord(A, 0, sx, pi1 - 1 + r);
-    pc[1][r] = coord(A, 1, sy, pi2 - 1 + r);
-    pc[2][r] = coord(A, 2, sz, kin[r]);
-  }
-  const double dxa[3] = {g.dx1, g.dx2, g.dx3};
-  for (int a = 0; a < 3; ++a)
-    for (int r = 0; r < 3; ++r) lit_axis_weight(A, pos[a], pc[a][r], dxa[a], eps, W[a][r], dW[a][r]);
-  double Am[16];
-  for (int e = 0; e < 16; ++e) Am[e] = 0.0;
-  for (int nk = 0; nk < 3; ++nk)
-    for (int j = 0; j < 3; ++j) {
-      const double w23 = W[1][j] * W[2][nk];
-      for (int i = 0; i < 3; ++i) {
-        const double wtx = W[0][i] * w23;
-        const double pk[4] = {1.0, pc[0][i], pc[1][j], pc[2][nk]};
-        for (int cc = 0; cc < 4; ++cc) {
-          const double t = wtx * pk[cc];
-          for (int r = 0; r < 4; ++r) Am[r + 4 * cc] = Am[r + 4 * cc] + t * pk[r];
-        }
-      }
+    x[r] = coord(A, 0, sx, pi1 - 1 + r);
+    y[r] = coord(A, 1, sy, pi2 - 1 + r);
+    lit_axis_weight(A, 0, pos[0], x[r], W0[r], dW0[r]);
+    lit_axis_weight(A, 1, pos[1], y[r], W1[r], dW1[r]);
+    if (r < 2) {
+      z[r] = coord(A, 2, sz, k1 - 1 + r);
+      lit_axis_weight(A, 2, pos[2], z[r], W2[r], dW2[r]);
     }
+  }
+  double Am[16], wt[9], dw[9];
+  lit_node_weights(-1, W0, dW0, W1, dW1, W2[0], dW2[0], wt);
+  lit_layer<true>(wt, x, y, z[0], Am);
+  lit_node_weights(-1, W0, dW0, W1, dW1, W2[1], dW2[1], wt);
+  lit_layer<false>(wt, x, y, z[1], Am);
+  lit_symmetric(Am);
   if (!inv4(Am)) return false;
   double gam[4];
   for (int r = 0; r < 4; ++r) {                   // DGEMV('N', invA, ptx)
@@ -342,19 +445,11 @@ __device__ bool probe_grad_lit(const LagArgs& A, const double pos[3], int pi1, i
   const int kk_[3] = {wrap(keul[0] - 1, g.n3m), wrap(keul[1] - 1, g.n3m), wrap(keul[2] - 1, g.n3m)};
   for (int d = 0; d < 3; ++d) {
     double dA[16];
-    for (int e = 0; e < 16; ++e) dA[e] = 0.0;
-    for (int nk = 0; nk < 3; ++nk)
-      for (int j = 0; j < 3; ++j)
-        for (int i = 0; i < 3; ++i) {
-          const double dwd = d == 0 ? (dW[0][i] * W[1][j]) * W[2][nk]
-                           : d == 1 ? (W[0][i] * dW[1][j]) * W[2][nk]
-                                    : (W[0][i] * W[1][j]) * dW[2][nk];
-          const double pk[4] = {1.0, pc[0][i], pc[1][j], pc[2][nk]};
-          for (int cc = 0; cc < 4; ++cc) {
-            const double t = dwd * pk[cc];
-            for (int r = 0; r < 4; ++r) dA[r + 4 * cc] = dA[r + 4 * cc] + t * pk[r];
-          }
-        }
+    lit_node_weights(d, W0, dW0, W1, dW1, W2[0], dW2[0], dw);
+    lit_layer<true>(dw, x, y, z[0], dA);
+    lit_node_weights(d, W0, dW0, W1, dW1, W2[1], dW2[1], dw);
+    lit_layer<false>(dw, x, y, z[1], dA);
+    lit_symmetric(dA);
     double pk_d[4] = {0.0, 0.0, 0.0, 0.0};
     pk_d[d + 1] = 1.0;
     for (int r = 0; r < 4; ++r) {                 // pk = -dA gamma + pk
@@ -368,24 +463,17 @@ __device__ bool probe_grad_lit(const LagArgs& A, const double pos[3], int pi1, i
       for (int cc = 0; cc < 4; ++cc) t += Am[r + 4 * cc] * pk_d[cc];
       dgam[r] = t;
     }
-    double gsum = 0;
-    for (int nk = 0; nk < 3; ++nk)
-      for (int j = 0; j < 3; ++j) {
-        const int jj = fmod_pos(pi2 - 1 + j - 1, g.n2m);
-        const double w23 = W[1][j] * W[2][nk];
-        for (int i = 0; i < 3; ++i) {
-          const double wtx = W[0][i] * w23;
-          const double dwd = d == 0 ? (dW[0][i] * W[1][j]) * W[2][nk]
-                           : d == 1 ? (W[0][i] * dW[1][j]) * W[2][nk]
-                                    : (W[0][i] * W[1][j]) * dW[2][nk];
-          const double pk[4] = {1.0, pc[0][i], pc[1][j], pc[2][nk]};
-          double t1 = 0, t2 = 0;
-          for (int r = 0; r < 4; ++r) t1 += dgam[r] * (wtx * pk[r]);
-          for (int r = 0; r < 4; ++r) t2 += gam[r] * (dwd * pk[r]);
-          const double T = q[cidx(g, fmod_pos(pi1 - 1 + i - 1, g.n1m), jj, kk_[nk])];
-          gsum += (t1 + t2) * T;
-        }
+    double gsum = 0, v[9];
+    for (int nk = 0; nk < 3; ++nk) {
+      if (nk < 2) {
+        lit_node_weights(-1, W0, dW0, W1, dW1, W2[nk], dW2[nk], wt);
+        lit_node_weights(d, W0, dW0, W1, dW1, W2[nk], dW2[nk], dw);
+        lit_node_values(wt, dw, dgam, gam, x, y, z[nk], v);
       }
+#pragma unroll
+      for (int n = 0; n < 9; ++n)
+        gsum += v[n] * q[cidx(g, fmod_pos(pi1 - 1 + n % 3 - 1, g.n1m), fmod_pos(pi2 - 1 + n / 3 - 1, g.n2m), kk_[nk])];
+    }
     grad[d] = gsum;
   }
   return true;
@@ -953,9 +1041,9 @@ __global__ void mls_weight_sep_kernel(LagArgs A, const double* __restrict__ tri_
   double wx[3], wy[3], wz[3], dx[3], dy[3], dz[3];
   for (int q = 0; q < 3; ++q) {
     double cz = coord(A, 2, cs.sz, k0 - 1 + q), cy = coord(A, 1, cs.sy, j0 - 1 + q), cx = coord(A, 0, cs.sx, i0 - 1 + q);
-    wz[q] = mls_gaussian(fabs(cz - pos[2]) / (A.wscl / g.dx3), A.wcon);
-    wy[q] = mls_gaussian(fabs(cy - pos[1]) / (A.wscl / g.dx2), A.wcon);
-    wx[q] = mls_gaussian(fabs(cx - pos[0]) / (A.wscl / g.dx1), A.wcon);
+    wz[q] = mls_gaussian(A, axis_norp(A, 2, cz - pos[2]));
+    wy[q] = mls_gaussian(A, axis_norp(A, 1, cy - pos[1]));
+    wx[q] = mls_gaussian(A, axis_norp(A, 0, cx - pos[0]));
     dx[q] = cx - pos[0]; dy[q] = cy - pos[1]; dz[q] = cz - pos[2];
   }
   double X[3], Y[3], Z[3], M[16];
@@ -977,25 +1065,14 @@ __global__ void mls_weight_sep_kernel(LagArgs A, const double* __restrict__ tri_
 // The cut-off decision r > 1 uses r = |x - x_c| / (wscl/dx) rounded as the
 // reference rounds it; the rest uses precomputed reciprocals (the separable
 // construction is insensitive to last-ulp changes of the weights).
-struct AxisScale {
-  double c, inv_c, inv_wcon, dcoef;   // wscl/dx, its reciprocal, 1/wcon, -2/wcon^2
-};
-__device__ __forceinline__ AxisScale axis_scale(const LagArgs& A, double dx) {
-  AxisScale a;
-  a.c = A.wscl / dx;
-  a.inv_c = 1.0 / a.c;
-  a.inv_wcon = 1.0 / A.wcon;
-  a.dcoef = -2.0 / (A.wcon * A.wcon);
-  return a;
-}
-__device__ __forceinline__ void axis_weight(const AxisScale& a, double pos, double pc, double& w, double& dw) {
+__device__ __forceinline__ void axis_weight(const LagArgs& A, int d, double pos, double pc, double& w, double& dw) {
   const double eps = 2.220446049250313e-16;
-  double rr = pos - pc;
-  double np = fabs(rr) / a.c;
-  if (np > 1.0) { w = 0.0; dw = 0.0; return; }
-  double e = exp(-sqd(np * a.inv_wcon));
+  const double rr = pos - pc;
+  const double np = axis_norp(A, d, rr);
+  if (above(np, 1.0)) { w = 0.0; dw = 0.0; return; }
+  double e = exp(-sqd(np * A.iwcon));
   w = e;
-  dw = (np < eps) ? 0.0 : (a.dcoef * np) * e * copysign(a.inv_c, rr);
+  dw = __double_as_longlong(np) < __double_as_longlong(eps) ? 0.0 : (A.dcoef * np) * e * copysign(A.iwr[d], rr);
 }
 
 // Separable MLS gradient at a probe: the gradient of wght_gradT (mls_heatFlux
@@ -1013,12 +1090,15 @@ __device__ bool probe_grad_sep(const LagArgs& A, const double pos[3], int pi1, i
   int k1w = fmod_pos(k1 - 1, g.n3m) + 1;
   int keul[3] = {k1w - 1, k1w, k1w + 1};
   const int sel[3] = {sx, sy, sz};
-  const AxisScale sc[3] = {axis_scale(A, g.dx1), axis_scale(A, g.dx2), axis_scale(A, g.dx3)};
   double w[3][3], dw[3][3], dd[3][3];             // [axis][point]
   for (int r = 0; r < 3; ++r) {
     double pc[3] = {coord(A, 0, sel[0], pi1 - 1 + r), coord(A, 1, sel[1], pi2 - 1 + r), coord(A, 2, sel[2], kin[r])};
     for (int a = 0; a < 3; ++a) {
-      axis_weight(sc[a], pos[a], pc[a], w[a][r], dw[a][r]);
+      if (a == 2 && r == 2) {                     // the repeated layer
+        w[2][2] = w[2][1]; dw[2][2] = dw[2][1]; dd[2][2] = dd[2][1];
+        break;
+      }
+      axis_weight(A, a, pos[a], pc[a], w[a][r], dw[a][r]);
       dd[a][r] = pc[a] - pos[a];
     }
   }
@@ -1097,13 +1177,12 @@ __device__ bool probe_value_sep(const LagArgs& A, const double pos[3], int i0, i
   const Grid& g = A.g;
   int k1 = ffloor(pos[2] * g.dx3) + 1;
   int k1w = fmod_pos(k1 - 1, g.n3m) + 1;
-  const AxisScale sc[3] = {axis_scale(A, g.dx1), axis_scale(A, g.dx2), axis_scale(A, g.dx3)};
   double w[3][3], dd[3][3];
   for (int r = 0; r < 3; ++r) {
     double pc[3] = {coord(A, 0, 1, i0 - 1 + r), coord(A, 1, 1, j0 - 1 + r), coord(A, 2, 1, k1 - 1 + r)};
     for (int a = 0; a < 3; ++a) {
       double dwu;
-      axis_weight(sc[a], pos[a], pc[a], w[a][r], dwu);
+      axis_weight(A, a, pos[a], pc[a], w[a][r], dwu);
       dd[a][r] = pc[a] - pos[a];
     }
   }
@@ -1171,7 +1250,12 @@ __global__ void heat_flux_sep_kernel(LagArgs A, const double* __restrict__ temp,
 // A^-1 and gamma are published, the direction-d gradient.  Every value comes
 // from exactly the operations of probe_grad_lit in its order (the oracle's
 // bits); the split only gives the device four times the independent work per
-// probe that one thread would have.
+// probe that one thread would have.  Bound by the FP64 pipe (no contraction, so
+// a product and its sum are two instructions): the repeated layer's and the
+// symmetric sums once, divisions by constants as five operations (div_const),
+// comparisons on the bits and the probe's position formed by one warp took 20480
+// faces from 612 to 418 us, 5120 from 219 to 152; the MLS weights (mls_weight_kernel)
+// of 20480 faces went from 313 to 279 us, the precision form's from 146 to 119.
 constexpr int kHfProbes = 32;
 __global__ void __launch_bounds__(4 * kHfProbes)
 heat_flux_lit_kernel(LagArgs A, const double* __restrict__ temp, const double* __restrict__ tri_bar,
@@ -1180,17 +1264,15 @@ heat_flux_lit_kernel(LagArgs A, const double* __restrict__ temp, const double* _
                      double* __restrict__ qw_i, int* __restrict__ flag) {
   __shared__ double sW[3][3][kHfProbes], sdW[3][3][kHfProbes], spc[3][3][kHfProbes];
   __shared__ double sAi[16][kHfProbes], sgam[4][kHfProbes], sgrad[3][kHfProbes];
-  __shared__ int sok[kHfProbes];
+  __shared__ int sok[kHfProbes], scell[3][kHfProbes];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int gid = blockIdx.x * kHfProbes + lane;
   const int t = gid >> 1, side = gid & 1;
   const bool valid = t < A.nf;
   const bool live = valid && !ghost[t];
   const Grid& g = A.g;
-  const double eps = 2.220446049250313e-16;       // EPSILON(1.0d0)
   double pos[3] = {0.0, 0.0, 0.0};
-  int pi1 = 0, pi2 = 0, k1 = 0;
-  if (live) {
+  if (w == 0 && live) {
     const double n0 = tri_nor[3 * t], n1 = tri_nor[3 * t + 1], n2 = tri_nor[3 * t + 2];
     const double s = sqrt(n0 * n0 + n1 * n1 + n2 * n2);
     for (int d = 0; d < 3; ++d) {
@@ -1198,18 +1280,18 @@ heat_flux_lit_kernel(LagArgs A, const double* __restrict__ temp, const double* _
       pos[d] = side == 0 ? tri_bar[3 * t + d] + h * nd / s : tri_bar[3 * t + d] - h * nd / s;
     }
     // pind null (fused step): the probe's cage as probe_idx_kernel finds it
-    pi1 = pind ? pind[6 * t + 3 * side + 0] : ffloor(pos[0] * g.dx1) + 1;
-    pi2 = pind ? pind[6 * t + 3 * side + 1] : ffloor(pos[1] * g.dx2) + 1;
-    k1 = ffloor(pos[2] * g.dx3) + 1;
-  }
-  if (w == 0 && live) {
-    const int kin[3] = {k1 - 1, k1, k1};          // the repeated layer of mls_heatFlux.f90:213
-    const double dxa[3] = {g.dx1, g.dx2, g.dx3};
+    const int pi1 = pind ? pind[6 * t + 3 * side + 0] : ffloor(pos[0] * g.dx1) + 1;
+    const int pi2 = pind ? pind[6 * t + 3 * side + 1] : ffloor(pos[1] * g.dx2) + 1;
+    const int k1 = ffloor(pos[2] * g.dx3) + 1;
+    scell[0][lane] = pi1;
+    scell[1][lane] = pi2;
+    scell[2][lane] = k1;
     for (int r = 0; r < 3; ++r) {
-      const double pc[3] = {coord(A, 0, 1, pi1 - 1 + r), coord(A, 1, 1, pi2 - 1 + r), coord(A, 2, 1, kin[r])};
+      const double pc[3] = {coord(A, 0, 1, pi1 - 1 + r), coord(A, 1, 1, pi2 - 1 + r), coord(A, 2, 1, k1 - 1 + r)};
       for (int a = 0; a < 3; ++a) {
+        if (a == 2 && r == 2) break;              // z layers k1 - 1, k1 and k1 again
         double W, dW;
-        lit_axis_weight(A, pos[a], pc[a], dxa[a], eps, W, dW);
+        lit_axis_weight(A, a, pos[a], pc[a], W, dW);
         spc[a][r][lane] = pc[a];
         sW[a][r][lane] = W;
         sdW[a][r][lane] = dW;
@@ -1217,51 +1299,42 @@ heat_flux_lit_kernel(LagArgs A, const double* __restrict__ temp, const double* _
     }
   }
   __syncthreads();
-  double dA[16];
   const int d = w - 1;
+  double x[3], y[3];
+  for (int r = 0; r < 3; ++r) {
+    x[r] = spc[0][r][lane];
+    y[r] = spc[1][r][lane];
+  }
+  // node weights of layer nk: of A (e < 0) or dA_e
+  auto nodes = [&](int e, int nk, double (&out)[9]) {
+    const double W0[3] = {sW[0][0][lane], sW[0][1][lane], sW[0][2][lane]};
+    const double W1[3] = {sW[1][0][lane], sW[1][1][lane], sW[1][2][lane]};
+    const double dW0[3] = {sdW[0][0][lane], sdW[0][1][lane], sdW[0][2][lane]};
+    const double dW1[3] = {sdW[1][0][lane], sdW[1][1][lane], sdW[1][2][lane]};
+    lit_node_weights(e, W0, dW0, W1, dW1, sW[2][nk][lane], sdW[2][nk][lane], out);
+  };
+  double Mx[16];
+  if (live) {
+    double wn[9];
+    nodes(d, 0, wn);
+    lit_layer<true>(wn, x, y, spc[2][0][lane], Mx);
+    nodes(d, 1, wn);
+    lit_layer<false>(wn, x, y, spc[2][1][lane], Mx);
+    lit_symmetric(Mx);
+  }
   if (w == 0) {
     int ok = 0;
-    if (live) {
-      double Am[16];
-      for (int e = 0; e < 16; ++e) Am[e] = 0.0;
-      for (int nk = 0; nk < 3; ++nk)
-        for (int j = 0; j < 3; ++j) {
-          const double w23 = sW[1][j][lane] * sW[2][nk][lane];
-          for (int i = 0; i < 3; ++i) {
-            const double wtx = sW[0][i][lane] * w23;
-            const double pk[4] = {1.0, spc[0][i][lane], spc[1][j][lane], spc[2][nk][lane]};
-            for (int cc = 0; cc < 4; ++cc) {
-              const double tt = wtx * pk[cc];
-              for (int r = 0; r < 4; ++r) Am[r + 4 * cc] = Am[r + 4 * cc] + tt * pk[r];
-            }
-          }
-        }
-      if (inv4(Am)) {
-        ok = 1;
-        const double ptx[4] = {1.0, pos[0], pos[1], pos[2]};
-        for (int r = 0; r < 4; ++r) {               // DGEMV('N', invA, ptx)
-          double tt = 0;
-          for (int cc = 0; cc < 4; ++cc) tt += Am[r + 4 * cc] * ptx[cc];
-          sgam[r][lane] = tt;
-        }
-        for (int e = 0; e < 16; ++e) sAi[e][lane] = Am[e];
+    if (live && inv4(Mx)) {
+      ok = 1;
+      const double ptx[4] = {1.0, pos[0], pos[1], pos[2]};
+      for (int r = 0; r < 4; ++r) {               // DGEMV('N', invA, ptx)
+        double tt = 0;
+        for (int cc = 0; cc < 4; ++cc) tt += Mx[r + 4 * cc] * ptx[cc];
+        sgam[r][lane] = tt;
       }
+      for (int e = 0; e < 16; ++e) sAi[e][lane] = Mx[e];
     }
     sok[lane] = ok;
-  } else if (live) {
-    for (int e = 0; e < 16; ++e) dA[e] = 0.0;
-    for (int nk = 0; nk < 3; ++nk)
-      for (int j = 0; j < 3; ++j)
-        for (int i = 0; i < 3; ++i) {
-          const double dwd = d == 0 ? (sdW[0][i][lane] * sW[1][j][lane]) * sW[2][nk][lane]
-                           : d == 1 ? (sW[0][i][lane] * sdW[1][j][lane]) * sW[2][nk][lane]
-                                    : (sW[0][i][lane] * sW[1][j][lane]) * sdW[2][nk][lane];
-          const double pk[4] = {1.0, spc[0][i][lane], spc[1][j][lane], spc[2][nk][lane]};
-          for (int cc = 0; cc < 4; ++cc) {
-            const double tt = dwd * pk[cc];
-            for (int r = 0; r < 4; ++r) dA[r + 4 * cc] = dA[r + 4 * cc] + tt * pk[r];
-          }
-        }
   }
   __syncthreads();
   if (w > 0 && live && sok[lane]) {
@@ -1271,7 +1344,7 @@ heat_flux_lit_kernel(LagArgs A, const double* __restrict__ temp, const double* _
     pk_d[d + 1] = 1.0;
     for (int r = 0; r < 4; ++r) {                   // pk = -dA gamma + pk
       double tt = 0;
-      for (int cc = 0; cc < 4; ++cc) tt += dA[r + 4 * cc] * gam[cc];
+      for (int cc = 0; cc < 4; ++cc) tt += Mx[r + 4 * cc] * gam[cc];
       pk_d[r] = pk_d[r] - tt;
     }
     double dgam[4];
@@ -1280,26 +1353,20 @@ heat_flux_lit_kernel(LagArgs A, const double* __restrict__ temp, const double* _
       for (int cc = 0; cc < 4; ++cc) tt += sAi[r + 4 * cc][lane] * pk_d[cc];
       dgam[r] = tt;
     }
-    const int k1w = fmod_pos(k1 - 1, g.n3m) + 1;
-    const int kk_[3] = {wrap(k1w - 2, g.n3m), wrap(k1w - 1, g.n3m), wrap(k1w, g.n3m)};
-    double gsum = 0;
-    for (int nk = 0; nk < 3; ++nk)
-      for (int j = 0; j < 3; ++j) {
-        const int jj = fmod_pos(pi2 - 1 + j - 1, g.n2m);
-        const double w23 = sW[1][j][lane] * sW[2][nk][lane];
-        for (int i = 0; i < 3; ++i) {
-          const double wtx = sW[0][i][lane] * w23;
-          const double dwd = d == 0 ? (sdW[0][i][lane] * sW[1][j][lane]) * sW[2][nk][lane]
-                           : d == 1 ? (sW[0][i][lane] * sdW[1][j][lane]) * sW[2][nk][lane]
-                                    : (sW[0][i][lane] * sW[1][j][lane]) * sdW[2][nk][lane];
-          const double pk[4] = {1.0, spc[0][i][lane], spc[1][j][lane], spc[2][nk][lane]};
-          double t1 = 0, t2 = 0;
-          for (int r = 0; r < 4; ++r) t1 += dgam[r] * (wtx * pk[r]);
-          for (int r = 0; r < 4; ++r) t2 += gam[r] * (dwd * pk[r]);
-          const double T = temp[cidx(g, fmod_pos(pi1 - 1 + i - 1, g.n1m), jj, kk_[nk])];
-          gsum += (t1 + t2) * T;
-        }
+    const int pi1 = scell[0][lane], pi2 = scell[1][lane], k1w = fmod_pos(scell[2][lane] - 1, g.n3m) + 1;
+    double gsum = 0, v[9];
+    for (int nk = 0; nk < 3; ++nk) {
+      if (nk < 2) {
+        double wt[9], dw[9];
+        nodes(-1, nk, wt);
+        nodes(d, nk, dw);
+        lit_node_values(wt, dw, dgam, gam, x, y, spc[2][nk][lane], v);
       }
+      const int kk = wrap(k1w - 2 + nk, g.n3m);
+#pragma unroll
+      for (int n = 0; n < 9; ++n)
+        gsum += v[n] * temp[cidx(g, fmod_pos(pi1 - 1 + n % 3 - 1, g.n1m), fmod_pos(pi2 - 1 + n / 3 - 1, g.n2m), kk)];
+    }
     sgrad[d][lane] = gsum;
   }
   __syncthreads();
@@ -1326,7 +1393,7 @@ heat_flux_lit_kernel(LagArgs A, const double* __restrict__ temp, const double* _
 // inversion is done by all four lanes alike.  The chain of FP64 instructions
 // of a block is a third of the other kernel's and there are four times the
 // blocks, at a quarter more FP64 instructions in all: faster until the SMs are
-// full (1280 faces 102 -> 79 us, 5120 faces 219 -> 216, 20480 faces 612 -> 789).
+// full (1280 faces 72 -> 60 us, 5120 faces 152 -> 163, 20480 faces 418 -> 582).
 constexpr int kHf4Probes = 8;
 constexpr int kHf4Faces = 4096;
 __global__ void __launch_bounds__(128)
@@ -1365,13 +1432,12 @@ heat_flux_lit4_kernel(LagArgs A, const double* __restrict__ temp, const double* 
     pi2 = pind ? pind[6 * t + 3 * side + 1] : ffloor(pos[1] * g.dx2) + 1;
     k1 = ffloor(pos[2] * g.dx3) + 1;
   }
-  if (live && 4 * w + c < 9) {                    // one axis weight per lane
+  if (live && 4 * w + c < 8) {                    // one axis weight per lane
     const int a = (4 * w + c) % 3, r = (4 * w + c) / 3;
     const double pc = a == 0 ? coord(A, 0, 1, pi1 - 1 + r)
-                             : (a == 1 ? coord(A, 1, 1, pi2 - 1 + r)
-                                       : coord(A, 2, 1, r == 0 ? k1 - 1 : k1));   // the repeated layer of mls_heatFlux.f90:213
+                             : (a == 1 ? coord(A, 1, 1, pi2 - 1 + r) : coord(A, 2, 1, k1 - 1 + r));
     double W, dW;
-    lit_axis_weight(A, pos[a], pc, a == 0 ? g.dx1 : (a == 1 ? g.dx2 : g.dx3), eps, W, dW);
+    lit_axis_weight(A, a, pos[a], pc, W, dW);
     spc[a][r][pr] = pc;
     sW[a][r][pr] = W;
     sdW[a][r][pr] = dW;
@@ -1385,19 +1451,30 @@ heat_flux_lit4_kernel(LagArgs A, const double* __restrict__ temp, const double* 
          : d == 1 ? (sW[0][i][pr] * sdW[1][j][pr]) * sW[2][nk][pr]
                   : (sW[0][i][pr] * sW[1][j][pr]) * sdW[2][nk][pr];
   };
-  double col[4] = {0.0, 0.0, 0.0, 0.0};           // column c
+  double col[4] = {0.0, 0.0, 0.0, 0.0};           // column c; layer 1 counts twice (lit_layer)
   if (live) {
-    for (int nk = 0; nk < 3; ++nk)
-      for (int j = 0; j < 3; ++j)
-        for (int i = 0; i < 3; ++i) {
-          const double wn = w == 0 ? wt_of(i, j, nk) : dw_of(i, j, nk);
-          const double px = spc[0][i][pr], py = spc[1][j][pr], pz = spc[2][nk][pr];
-          const double tt = wn * (c == 0 ? 1.0 : (c == 1 ? px : (c == 2 ? py : pz)));
-          col[0] = col[0] + tt;
-          col[1] = col[1] + tt * px;
-          col[2] = col[2] + tt * py;
-          col[3] = col[3] + tt * pz;
-        }
+#pragma unroll
+    for (int nk = 0; nk < 2; ++nk) {
+      const double pz = spc[2][nk][pr];
+      double p[4][9];
+#pragma unroll
+      for (int n = 0; n < 9; ++n) {
+        const int i = n % 3, j = n / 3;
+        const double wn = w == 0 ? wt_of(i, j, nk) : dw_of(i, j, nk);
+        const double px = spc[0][i][pr], py = spc[1][j][pr];
+        const double tt = wn * (c == 0 ? 1.0 : (c == 1 ? px : (c == 2 ? py : pz)));
+        p[0][n] = tt;
+        p[1][n] = tt * px;
+        p[2][n] = tt * py;
+        p[3][n] = tt * pz;
+      }
+#pragma unroll
+      for (int rep = 0; rep <= nk; ++rep)
+#pragma unroll
+        for (int n = 0; n < 9; ++n)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) col[r] = col[r] + p[r][n];
+    }
   }
   if (w == 0) {
     double Am[16];
@@ -1438,20 +1515,33 @@ heat_flux_lit4_kernel(LagArgs A, const double* __restrict__ temp, const double* 
     for (int r = 0; r < 4; ++r) dgam[r] = __shfl_sync(FULL, dg, (lane & ~3) + r);
     const int k1w = fmod_pos(k1 - 1, g.n3m) + 1;
     double gsum = 0;
-    for (int m = 0; m < 7; ++m) {                  // nodes 4m .. 4m+3 in cage order, one per lane
+    double nv[5];                                  // nodes 4m .. 4m+3 of layers 0 and 1, one per lane
+#pragma unroll
+    for (int m = 0; m < 5; ++m) {
       const int nd = 4 * m + c;
-      double val = 0.0;
-      if (go && nd < 27) {
+      nv[m] = 0.0;
+      if (go && nd < 18) {
         const int i = nd % 3, j = (nd / 3) % 3, nk = nd / 9;
         const double wtx = wt_of(i, j, nk), dwd = dw_of(i, j, nk);
-        const double pk[4] = {1.0, spc[0][i][pr], spc[1][j][pr], spc[2][nk][pr]};
-        double t1 = 0, t2 = 0;
-        for (int r = 0; r < 4; ++r) t1 += dgam[r] * (wtx * pk[r]);
-        for (int r = 0; r < 4; ++r) t2 += gam[r] * (dwd * pk[r]);
-        const double T = temp[cidx(g, fmod_pos(pi1 - 1 + i - 1, g.n1m), fmod_pos(pi2 - 1 + j - 1, g.n2m),
-                                   wrap(k1w - 2 + nk, g.n3m))];
-        val = (t1 + t2) * T;
+        const double px = spc[0][i][pr], py = spc[1][j][pr], pz = spc[2][nk][pr];
+        const double t1 = ((dgam[0] * wtx + dgam[1] * (wtx * px)) + dgam[2] * (wtx * py)) + dgam[3] * (wtx * pz);
+        const double t2 = ((gam[0] * dwd + gam[1] * (dwd * px)) + gam[2] * (dwd * py)) + gam[3] * (dwd * pz);
+        nv[m] = t1 + t2;
       }
+    }
+#pragma unroll
+    for (int m = 0; m < 7; ++m) {                  // all 27 in cage order
+      const int nd = 4 * m + c;
+      double val = m < 5 ? nv[m] : 0.0;
+      if (m >= 4) {                                // node nd - 9: lane c - 1 of group m - 2, lane 3 of m - 3 for c = 0
+        const double a = __shfl_sync(FULL, nv[m - 2], (lane & ~3) + ((c + 3) & 3));
+        const double b = __shfl_sync(FULL, nv[m - 3], (lane & ~3) + 3);
+        if (nd >= 18) val = c == 0 ? b : a;
+      }
+      if (go && nd < 27)
+        val *= temp[cidx(g, fmod_pos(pi1 - 1 + nd % 3 - 1, g.n1m), fmod_pos(pi2 - 1 + (nd / 3) % 3 - 1, g.n2m),
+                         wrap(k1w - 2 + nd / 9, g.n3m))];
+#pragma unroll
       for (int q = 0; q < 4; ++q) {
         const double v = __shfl_sync(FULL, val, (lane & ~3) + q);
         if (4 * m + q < 27) gsum += v;

@@ -68,16 +68,7 @@ MIBM_HD double mexp_pow2(int n) {
   return d;
 }
 
-MIBM_HD double mls_exp(double x) {
-  const double kInvLn2 = 0x1.71547652b82fep+0;      // 1/ln2 rounded
-  const double kLn2Hi = 0x1.62e42ffp-1;             // ln2 to 29 significant bits
-  const double kLn2Lo = -0x1.718432a1b0e26p-35;     // ln2 - kLn2Hi rounded
-  if (x != x) return x;
-  if (x > 709.782712893384) return mexp_mul(mexp_pow2(1023), 2.0);   // overflows to +inf
-  if (x < -745.2) return 0.0;
-  const double nd = mexp_rint(mexp_mul(x, kInvLn2));
-  const int n = (int)nd;
-  const double r = mexp_add(mexp_add(x, -mexp_mul(nd, kLn2Hi)), -mexp_mul(nd, kLn2Lo));
+MIBM_HD double mexp_poly(double r) {
   // q(r) = 1/2! + r/3! + ... + r^11/13!
   double q = 1.6059043836821613e-10;                // 1/13!
   q = mexp_add(mexp_mul(q, r), 2.08767569878681e-09);      // 1/12!
@@ -91,7 +82,31 @@ MIBM_HD double mls_exp(double x) {
   q = mexp_add(mexp_mul(q, r), 0.041666666666666664);      // 1/4!
   q = mexp_add(mexp_mul(q, r), 0.16666666666666666);       // 1/3!
   q = mexp_add(mexp_mul(q, r), 0.5);                       // 1/2!
-  const double p = mexp_add(1.0, mexp_add(r, mexp_mul(mexp_mul(r, r), q)));
+  return q;
+}
+
+MIBM_HD double mls_exp(double x) {
+  const double kInvLn2 = 0x1.71547652b82fep+0;      // 1/ln2 rounded
+  const double kLn2Hi = 0x1.62e42ffp-1;             // ln2 to 29 significant bits
+  const double kLn2Lo = -0x1.718432a1b0e26p-35;     // ln2 - kLn2Hi rounded
+#if defined(__CUDA_ARCH__)
+  // -708 < x < 708: the same operations without FP64 comparisons (of the bits
+  // instead), with rint and its integer from one addition of 1.5 2^52 and the
+  // scaling in the exponent, where it is exact
+  if ((__double2hiint(x) & 0x7fffffff) < 0x40862000) {
+    const double t = mexp_add(mexp_mul(x, kInvLn2), 0x1.8p52), nd = mexp_add(t, -0x1.8p52);
+    const double r = mexp_add(mexp_add(x, -mexp_mul(nd, kLn2Hi)), -mexp_mul(nd, kLn2Lo));
+    const double p = mexp_add(1.0, mexp_add(r, mexp_mul(mexp_mul(r, r), mexp_poly(r))));
+    return __longlong_as_double(__double_as_longlong(p) + ((long long)__double2loint(t) << 52));
+  }
+#endif
+  if (x != x) return x;
+  if (x > 709.782712893384) return mexp_mul(mexp_pow2(1023), 2.0);   // overflows to +inf
+  if (x < -745.2) return 0.0;
+  const double nd = mexp_rint(mexp_mul(x, kInvLn2));
+  const int n = (int)nd;
+  const double r = mexp_add(mexp_add(x, -mexp_mul(nd, kLn2Hi)), -mexp_mul(nd, kLn2Lo));
+  const double p = mexp_add(1.0, mexp_add(r, mexp_mul(mexp_mul(r, r), mexp_poly(r))));
   if (n >= -1022) return mexp_mul(p, mexp_pow2(n));
   // subnormal results: two exact-until-the-last scalings
   return mexp_mul(mexp_mul(p, mexp_pow2(n + 600)), mexp_pow2(-600));
