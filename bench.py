@@ -56,6 +56,7 @@ from melt_ibm_gb300.workloads import WORKLOAD_TEXT, WORKLOADS  # noqa: E402
 # compulsory field reads + writes of that kernel, in passes of N^3 doubles).
 ALGO_PASSES = {
     "fused_rhs": 7.0,      # x/y/z/T average: reads u,v,w(,T),p,ru ; writes rhs, ru
+    "explicit_int": 20.0,  # all four: reads u,v,w,T,p, three VOF fields and ru of each; writes rhs, ru of each
     # one launch for u, v, w (3 fields), one for T: mean of 3x and 1x the field passes
     "solve_x": 4.0, "solve_y": 4.0, "solve_z": 8.0,
     "fft_x_fwd": 1.0 + 1.125, "fft_y": 2.25, "fft_z_solve": 2.25, "fft_x_inv": 1.125 + 1.0,
@@ -106,8 +107,8 @@ def step_bytes_per_cell(form: str, forcing: bool, tagging: bool, nproj: int = 2)
 # workload; a workload without its own figure scales the nearest one by the
 # cell count (the traffic is per-cell).
 NCU_TRAFFIC = {
-    "melt256_c2": {"fused_rhs": {"bytes_per_launch": 1.2905e9, "measured_at": "256^3 (melt256_c2)"}},
-    "melt128_c1": {"fused_rhs": {"bytes_per_launch": 139.6e6, "measured_at": "128^3 (melt128_c1)"}},
+    "melt256_c2": {"fused_rhs": {"bytes_per_launch": 1.2909e9, "measured_at": "256^3 (melt256_c2)"}},
+    "melt128_c1": {"explicit_int": {"bytes_per_launch": 369.5e6, "measured_at": "128^3 (melt128_c1)"}},
 }
 
 # FP64 warp instructions of one step (ncu sm__inst_executed_pipe_fp64.sum
@@ -115,8 +116,8 @@ NCU_TRAFFIC = {
 # FP64 form is bounded by the FP64 issue rate (one warp instruction per 16
 # clocks per SM on this part): this count over that rate is the step's FP64
 # floor.
-FP64_CENSUS = {"melt256_c2": {"warp_instructions_per_step": 404.58e6, "clocks_per_instruction_per_sm": 16},
-               "melt128_c1": {"warp_instructions_per_step": 51.88e6, "clocks_per_instruction_per_sm": 16}}
+FP64_CENSUS = {"melt256_c2": {"warp_instructions_per_step": 388.00e6, "clocks_per_instruction_per_sm": 16},
+               "melt128_c1": {"warp_instructions_per_step": 28.08e6, "clocks_per_instruction_per_sm": 16}}
 
 FIELDS = {"u": abi.MIBM_F_VX, "v": abi.MIBM_F_VY, "w": abi.MIBM_F_VZ, "T": abi.MIBM_F_TEMP, "p": abi.MIBM_F_PR}
 FIELD_MASK = sum(1 << f for f in FIELDS.values())
