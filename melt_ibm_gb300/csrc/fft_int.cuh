@@ -38,10 +38,6 @@ namespace intfft {
 
 using namespace fixed;
 
-struct I2 { long long x, y; };
-// (cos, -sin) 2^62 of the forward twiddle as signed halves
-struct Tw { int ch, cl, sh, sl; };
-
 __host__ __device__ constexpr int nstages(int n) {
   int s = 0;
   while (n % 4 == 0) { n /= 4; ++s; }
@@ -79,23 +75,6 @@ __device__ __forceinline__ I2 down(I2 v) { return I2{down<S>(v.x), down<S>(v.y)}
 
 __device__ __forceinline__ I2 add(I2 a, I2 b) { return I2{a.x + b.x, a.y + b.y}; }
 __device__ __forceinline__ I2 sub(I2 a, I2 b) { return I2{a.x - b.x, a.y - b.y}; }
-
-// v w / 2^S (w, or its conjugate for INV), S = 1 or 2
-template <int S, bool INV>
-__device__ __forceinline__ I2 twiddle(I2 v, Tw w) {
-  int xh, xl, yh, yl;
-  halves(v.x, xh, xl);
-  halves(v.y, yh, yl);
-  // forward: (x c - y s, x s + y c); inverse: (x c + y s, y c - x s)
-  const int ah = INV ? yh : -yh, al = INV ? yl : -yl;
-  const int bh = INV ? -xh : xh, bl = INV ? -xl : xl;
-  constexpr long long half = 1ll << (29 + S);
-  const long long mr = wide(xh, w.ch) + wide(ah, w.sh);
-  const long long mi = wide(yh, w.ch) + wide(bh, w.sh);
-  const long long lr = half + wide(xh, w.cl) + wide(xl, w.ch) + wide(ah, w.sl) + wide(al, w.sh);
-  const long long li = half + wide(yh, w.cl) + wide(yl, w.ch) + wide(bh, w.sl) + wide(bl, w.sh);
-  return I2{(mr << (2 - S)) + (lr >> (30 + S)), (mi << (2 - S)) + (li >> (30 + S))};
-}
 
 // x sqrt(3)/2
 __device__ __forceinline__ long long times_s3(long long x) {

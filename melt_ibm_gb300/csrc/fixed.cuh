@@ -2,12 +2,52 @@
 // kernels that do their arithmetic on the integer pipe (fft_int.cuh, the
 // explicit terms of stencil.cu): an FP64 instruction costs as much issue as
 // some 32 integer ones on this part.
+//
+// The products of halves also build for the host (without CUDA), so that a
+// CPU test can check them against exact arithmetic.
 #pragma once
 
+#if defined(__CUDACC__)
 #include <cuda_runtime.h>
+#define FIXED_FN __host__ __device__ __forceinline__
+#else
+#define FIXED_FN inline
+#endif
 
 namespace mibm {
 namespace fixed {
+
+// signed halves of x: x = hi 2^32 + lo, lo in [-2^31, 2^31).  -lo does not
+// always fit a half: products are subtracted, halves never negated.
+FIXED_FN void halves(long long x, int& hi, int& lo) {
+  lo = (int)x;
+  hi = (int)(x >> 32) + (int)((unsigned)lo >> 31);
+}
+FIXED_FN long long wide(int a, int b) { return (long long)a * b; }
+
+struct I2 { long long x, y; };
+// (cos, -sin) 2^62 of the forward twiddle as signed halves
+struct Tw { int ch, cl, sh, sl; };
+
+// v w / 2^S (w, or its conjugate for INV), S = 1 or 2; a component is
+// within half a unit plus the two products of low halves left out, 2^-S each
+template <int S, bool INV>
+FIXED_FN I2 twiddle(I2 v, Tw w) {
+  int xh, xl, yh, yl;
+  halves(v.x, xh, xl);
+  halves(v.y, yh, yl);
+  constexpr long long half = 1ll << (29 + S);
+  // forward: (x c - y s, y c + x s); inverse: (x c + y s, y c - x s)
+  const long long pr = wide(yh, w.sh), pi = wide(xh, w.sh);
+  const long long qr = wide(yh, w.sl) + wide(yl, w.sh), qi = wide(xh, w.sl) + wide(xl, w.sh);
+  const long long mr = INV ? wide(xh, w.ch) + pr : wide(xh, w.ch) - pr;
+  const long long mi = INV ? wide(yh, w.ch) - pi : wide(yh, w.ch) + pi;
+  const long long lr = half + wide(xh, w.cl) + wide(xl, w.ch) + (INV ? qr : -qr);
+  const long long li = half + wide(yh, w.cl) + wide(yl, w.ch) + (INV ? -qi : qi);
+  return I2{mr * (1ll << (2 - S)) + (lr >> (30 + S)), mi * (1ll << (2 - S)) + (li >> (30 + S))};
+}
+
+#if defined(__CUDACC__)
 
 // biased exponent field (zero and subnormal values: 0)
 __device__ __forceinline__ int expo(double d) { return (int)((__double_as_longlong(d) >> 52) & 0x7ff); }
@@ -51,13 +91,6 @@ __device__ __forceinline__ double to_double(long long f, int X) {
 
 __device__ __forceinline__ double quiet_nan() { return __longlong_as_double(0x7ff8000000000000ll); }
 
-// signed halves of x: x = hi 2^32 + lo, lo in [-2^31, 2^31)
-__device__ __forceinline__ void halves(long long x, int& hi, int& lo) {
-  lo = (int)x;
-  hi = (int)(x >> 32) + (int)((unsigned)lo >> 31);
-}
-__device__ __forceinline__ long long wide(int a, int b) { return (long long)a * b; }
-
 // a b / 2^64 without lo*lo, rounded down: within one unit (|a|, |b| < 2^62)
 __device__ __forceinline__ long long mul_high(long long a, long long b) {
   int ah, al, bh, bl;
@@ -70,6 +103,7 @@ __device__ __forceinline__ long long square_high(long long a) {
   halves(a, ah, al);
   return wide(ah, ah) + (wide(ah, al) >> 31);
 }
+#endif
 
 }  // namespace fixed
 }  // namespace mibm
