@@ -972,12 +972,12 @@ __device__ __forceinline__ void geo_x(const Grid& g, double* __restrict__ rhs, c
   };
   const int rows = min(R, lines - row0), total = rows * nv;
   // the block's rows as one run of V-wide pieces, eight of a thread in flight;
-  // piece / nv as a multiply by magic = 2^32 / nv rounded up (exact below 2^16)
+  // piece / nv as a multiply by magic = 2^32 / nv rounded up (exact below 2^16; 2^32 itself, for lines of 2, does not fit)
   auto move = [&](auto body) {
     for (int p0 = threadIdx.x; p0 < total; p0 += 8 * kGeoRowThreads) body(p0);
   };
   auto piece = [&](int p, double*& at_g, int& at_s) {
-    const int r = (int)__umulhi((unsigned)p, magic), e = (p - r * nv) * V;
+    const int r = M == 2 && nv == 1 ? p : (int)__umulhi((unsigned)p, magic), e = (p - r * nv) * V;
     at_g = row_ptr(r) + e;
     at_s = r * RS + (e / M) * CS + e % M;
     return MIBM_IDX_OK((size_t)(at_g - rhs) % g.cells + V - 1, g.cells);
