@@ -2112,13 +2112,16 @@ __global__ void sdf_reset_kernel(Grid g, unsigned long long* __restrict__ sdf_bi
 // cell; the exact pass skips a face whose lower bound exceeds that minimum:
 // such a face is strictly farther than the nearest one, so the minimum, the
 // set of faces tied at it and hence the earliest-face winner are unchanged.
-// The bounds are evaluated in FP32 from FP32 copies of the coordinates
-// (|x| < 13, rounding error < 1e-6 per coordinate; vertices within 1e-6 of the
-// plane; < 4e-6 on a bound), and kBandMargin covers that error on both sides.
+// The bounds are evaluated in FP32 from FP32 copies of the coordinates, whose
+// rounding grows with the coordinate: with X the largest one of the pair, both
+// copies together put P - c off by 2 sqrt(3) 2^-24 X, the arithmetic by some 8
+// 2^-24 |P - c| more, and a vertex may be 1e-6 off the plane.  The margin of
+// either side is kBandMargin, which covers that up to X = 13 (a box of 2 pi),
+// or kBandRel X if that is more.
 // Without a plane (BandFace) h = r = 0 and rho = |P - c|; that bound alone let
 // the exact pass evaluate so many pairs that its three passes took 64 us each
 // with 20480 faces at 256^3 (now 22) and 20 us with 5120 at 128^3 (now 11).
-constexpr float kBandMargin = 8e-6f;
+constexpr float kBandMargin = 8e-6f, kBandRel = 6.2e-7f;
 
 __global__ void cm32_kernel(LagArgs A, float* __restrict__ cm32) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2135,15 +2138,18 @@ __global__ void band_prep_kernel(TagArgs T, BandFace* __restrict__ band_face, in
   band_prep_one(f, T.L.nv, T.vof, T.x, pos, T.L.g, band_face, face_cell);
 }
 
-// the bound of cell (ii, jj, kk) from face F with in-plane radius rad
+// the bound of cell (ii, jj, kk) from face F with in-plane radius rad, and its margin
 __device__ __forceinline__ float band_bound(const float* __restrict__ cm32, int clen, int coff, int ii, int jj, int kk,
-                                            const BandFace& F, float rad) {
-  const float vx = cm32[min(max(ii + coff, 0), clen - 1)] - F.c.x;
-  const float vy = cm32[clen + min(max(jj + coff, 0), clen - 1)] - F.c.y;
-  const float vz = cm32[2 * clen + min(max(kk + coff, 0), clen - 1)] - F.c.z;
+                                            const BandFace& F, float rad, float& margin) {
+  const float gx = cm32[min(max(ii + coff, 0), clen - 1)];
+  const float gy = cm32[clen + min(max(jj + coff, 0), clen - 1)];
+  const float gz = cm32[2 * clen + min(max(kk + coff, 0), clen - 1)];
+  const float vx = gx - F.c.x, vy = gy - F.c.y, vz = gz - F.c.z;
   const float h = F.n.x * vx + F.n.y * vy + F.n.z * vz;
   const float px = vx - h * F.n.x, py = vy - h * F.n.y, pz = vz - h * F.n.z;
   const float a = fmaxf(sqrtf(px * px + py * py + pz * pz) - rad, 0.f);
+  const float X = fmaxf(fmaxf(fmaxf(fabsf(gx), fabsf(gy)), fmaxf(fabsf(gz), fabsf(F.c.x))), fmaxf(fabsf(F.c.y), fabsf(F.c.z)));
+  margin = fmaxf(kBandMargin, kBandRel * X);
   return sqrtf(h * h + a * a);
 }
 
@@ -2163,8 +2169,9 @@ __global__ void band_select_kernel(TagArgs T, const BandFace* __restrict__ band_
     int ii = b.x - 2 + q % 5, jj = b.y - 2 + (q / 5) % 5, kk = b.z - 2 + q / 25;
     int im = fmod_pos(ii - 1, g.n1m), jm = fmod_pos(jj - 1, g.n1m), km = fmod_pos(kk - 1, g.n3m);
     const BandFace F = band_face[f];
-    const float lb = band_bound(cm32, A.clen, A.coff, ii, jj, kk, F, F.c.w) - kBandMargin;
-    keep = !(lb > __uint_as_float(band_ub[cidx(g, im, jm, km)]));
+    float margin;
+    const float lb = band_bound(cm32, A.clen, A.coff, ii, jj, kk, F, F.c.w, margin);
+    keep = !(lb - margin > __uint_as_float(band_ub[cidx(g, im, jm, km)]));
   }
   unsigned m = __ballot_sync(0xffffffffu, keep);
   if (!m) return;
@@ -2187,8 +2194,9 @@ __global__ void band_ub_kernel(TagArgs T, const BandFace* __restrict__ band_face
   int ii = b.x - 2 + q % 5, jj = b.y - 2 + (q / 5) % 5, kk = b.z - 2 + q / 25;
   int im = fmod_pos(ii - 1, g.n1m), jm = fmod_pos(jj - 1, g.n1m), km = fmod_pos(kk - 1, g.n3m);
   const BandFace F = band_face[f];
-  const float ub = band_bound(cm32, A.clen, A.coff, ii, jj, kk, F, F.n.w) + kBandMargin;
-  atomicMin(&band_ub[cidx(g, im, jm, km)], __float_as_uint(ub));
+  float margin;
+  const float ub = band_bound(cm32, A.clen, A.coff, ii, jj, kk, F, F.n.w, margin);
+  atomicMin(&band_ub[cidx(g, im, jm, km)], __float_as_uint(ub + margin));
 }
 
 // one thread per (triangle, band cell) of the compact list of
