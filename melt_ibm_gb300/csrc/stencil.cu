@@ -543,7 +543,8 @@ fused_t_f32_kernel(StencilArgs A, const StepParams* __restrict__ pp, float* __re
 // for the products kernel and the four fused_rhs kernels.  A product is kept
 // to 2^-58 of the square of the block's largest velocity, the FP64 product it
 // replaces to 2^-53 of its own value.  A cell that is not fully fluid takes
-// h_t's solid-advection branch; a block that holds a non-finite value gives NaN.
+// h_t's solid-advection branch; a block that holds a non-finite velocity gives
+// NaN, one that holds a non-finite T gives it for T alone.
 // Layers around the cells: 2.4 values converted per value used (32 x 8 x 1
 // cells: 4).  About 1400 instructions per cell and warp, neither pipe full (FP64
 // 0.6, integer 0.4): with 64 registers two blocks share an SM.  Per substep,
@@ -629,7 +630,7 @@ explicit_int_kernel(StencilArgs A, const StepParams* __restrict__ pp, RuSet ru, 
     const idx_t djp = (j + 1 == g.n2m) ? -(g.n2m - 1) * P : P, djm = (j == 0) ? (g.n2m - 1) * P : -P;
     const idx_t dkp = (k + 1 == g.n3m) ? -(g.n3m - 1) * PL : PL, dkm = (k == 0) ? (g.n3m - 1) * PL : -PL;
     if (!MIBM_IDX_OK(c0, g.cells)) return;
-    if (E == 0x7ff || ET == 0x7ff) {
+    if (E == 0x7ff) {
       for (int W = 0; W < 4; ++W) rhs4[(size_t)W * g.cells + c0] = ru.r[W][c0] = quiet_nan();
       return;
     }
@@ -697,6 +698,10 @@ explicit_int_kernel(StencilArgs A, const StepParams* __restrict__ pp, RuSet ru, 
       }
       if (A.forcing) h = add_forcing<double>(h, A.vofz, A.forcz, c0, p.cd[kRZLEN]);
       store(2, h, lap(w, l1, l2, l3, E) - p.cd[kPD3] * (pc - A.pr[c0 + dkm]));
+    }
+    if (ET == 0x7ff) {
+      rhs4[3 * g.cells + c0] = ru.r[3][c0] = quiet_nan();
+      return;
     }
     double ht;
     if (vof_is_one(A.vofp[c0])) {
