@@ -535,21 +535,32 @@ fused_t_f32_kernel(StencilArgs A, const StepParams* __restrict__ pp, float* __re
 // the sums and products on the integer pipe.
 // A block takes 32 x 4 x 4 cells, one per thread: u, v, w and T of the cells
 // and one layer around them are converted once into 64-bit fixed point in
-// shared memory, u, v, w at the largest exponent of the three in the block, T
-// at its own.  Each thread forms its cell's advection terms (products of hdnl1-3
-// regrouped as above: 15 integer products; hdnlte: 6) and Laplacians from
-// there, and rounds each sum to FP64 once.  What stays FP64 is the RK
-// combination: 6 operations per velocity component, 5 for T, against 46 per cell
-// for the products kernel and the four fused_rhs kernels.  A product is kept
-// to 2^-58 of the square of the block's largest velocity, the FP64 product it
-// replaces to 2^-53 of its own value.  A cell that is not fully fluid takes
-// h_t's solid-advection branch; a block that holds a non-finite velocity gives
-// NaN, one that holds a non-finite T gives it for T alone.
+// shared memory, each at its own largest exponent in the block.  Each thread
+// forms its cell's advection terms (products of hdnl1-3 regrouped as above: 15
+// integer products; hdnlte: 6) and Laplacians from there, and rounds each sum
+// to FP64 once.  What stays FP64 is the RK combination: 6 operations per
+// velocity component, 5 for T, against 46 per cell for the products kernel and
+// the four fused_rhs kernels.
+// The products of a carried component with the three velocities are summed at
+// the exponent of its largest value times the largest velocity of the block
+// and kept to 2^-58 of that product; the FP64 products they replace are kept to
+// 2^-53 of their own value.  So a small component beside a large one keeps its
+// digits, and cells 2^5 and more below their block's largest value have fewer
+// than in FP64: there the step's own rounding is larger, since the projection
+// takes gradients from all components and leaves about 2^-53 of the largest
+// velocity.  Advection terms against extended precision, relative 2-norm, FP64
+// kernels / this one: smooth flow at 48^3 8e-16 / 7e-17, noise 3e-16 / 7e-17,
+// v and w 1e-4 and 1e-8 of u 7e-16, 1e-15 / 7e-17, 7e-17 (at one exponent for
+// the three: 4e-13, 7e-9).
+// A cell that is not fully fluid takes h_t's solid-advection branch; a block
+// that holds a non-finite velocity gives NaN, one that holds a non-finite T
+// gives it for T alone.
 // Layers around the cells: 2.4 values converted per value used (32 x 8 x 1
 // cells: 4).  About 1400 instructions per cell and warp, neither pipe full (FP64
 // 0.6, integer 0.4): with 64 registers two blocks share an SM.  Per substep,
-// five kernels -> this one: 128^3 330 -> 177 us, 96^3 146 -> 70, 108 x 108 x 72
-// (two spacings) 226 -> 106, 48^3 53 -> 27 us (one wave of blocks).
+// five kernels -> this one: 128^3 330 -> 183 us (one exponent for u, v and w:
+// 178), 96^3 146 -> 71, 108 x 108 x 72 (two spacings) 226 -> 107, 48^3 53 -> 27
+// us (one wave of blocks).
 struct RuSet { double* r[4]; };
 constexpr int kExX = 32, kExY = 4, kExZ = 4, kExThreads = kExX * kExY * kExZ;
 constexpr int kExHX = kExX + 2, kExHY = kExY + 2, kExHZ = kExZ + 2, kExV = kExHX * kExHY * kExHZ;
@@ -559,14 +570,14 @@ template <int SP>
 __global__ void __launch_bounds__(kExThreads, 2)
 explicit_int_kernel(StencilArgs A, const StepParams* __restrict__ pp, RuSet ru, double* __restrict__ rhs4) {
   using namespace fixed;
-  constexpr int UP = 7, kWarps = kExThreads / 32, kRows = kExHY * kExHZ, PER = (kRows + kWarps - 1) / kWarps;
+  constexpr int UP = 8, kWarps = kExThreads / 32, kRows = kExHY * kExHZ, PER = (kRows + kWarps - 1) / kWarps;
   static_assert(2 * kRows <= kExThreads, "one thread per value beyond a row's first 32");
   __shared__ long long sq[4][kExV];
-  __shared__ int smax[2];
+  __shared__ int smax[4];
   const Grid& g = A.g;
   const int lane = threadIdx.x, warp = threadIdx.y + kExY * threadIdx.z, tid = lane + 32 * warp;
   const int i0 = blockIdx.x * kExX, j0 = blockIdx.y * kExY, k0 = blockIdx.z * kExZ;
-  if (tid < 2) smax[tid] = 1;
+  if (tid < 4) smax[tid] = 1;
   {
     // a warp takes whole rows of 32 values, the 2 left over of each row go to
     // a thread each; periodic, and a cell past the grid's end repeats one inside it
@@ -577,7 +588,7 @@ explicit_int_kernel(StencilArgs A, const StepParams* __restrict__ pp, RuSet ru, 
     };
     const int il = wrapped(i0 + lane - 1, g.n1m);
     double raw[4][PER + 1];
-    int eu = 1, et = 1;
+    int e[4] = {1, 1, 1, 1};
 #pragma unroll
     for (int p = 0; p <= PER; ++p) {
       const int r = p < PER ? warp + p * kWarps : tid >> 1;
@@ -589,38 +600,33 @@ explicit_int_kernel(StencilArgs A, const StepParams* __restrict__ pp, RuSet ru, 
       raw[3][p] = ok ? A.temp[c] : 0.0;
     }
 #pragma unroll
-    for (int p = 0; p <= PER; ++p) {
-      eu = max(eu, max(expo(raw[0][p]), max(expo(raw[1][p]), expo(raw[2][p]))));
-      et = max(et, expo(raw[3][p]));
-    }
-    eu = __reduce_max_sync(0xffffffffu, eu);
-    et = __reduce_max_sync(0xffffffffu, et);
+    for (int p = 0; p <= PER; ++p)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) e[q] = max(e[q], expo(raw[q][p]));
     __syncthreads();
-    if (lane == 0) {
-      atomicMax(&smax[0], eu);
-      atomicMax(&smax[1], et);
-    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) e[q] = __reduce_max_sync(0xffffffffu, e[q]);
+    if (lane < 4) atomicMax(&smax[lane], lane < 2 ? (lane ? e[1] : e[0]) : (lane == 2 ? e[2] : e[3]));
     __syncthreads();
-    const int E = smax[0], ET = smax[1];
+    const int E[4] = {smax[0], smax[1], smax[2], smax[3]};
 #pragma unroll
     for (int p = 0; p <= PER; ++p) {
       const int r = p < PER ? warp + p * kWarps : tid >> 1;
       if (p < PER ? r < kRows : tid < 2 * kRows) {
         const int t = r * kExHX + (p < PER ? lane : 32 + (tid & 1));
-        sq[0][t] = from_double<UP>(raw[0][p], E);
-        sq[1][t] = from_double<UP>(raw[1][p], E);
-        sq[2][t] = from_double<UP>(raw[2][p], E);
-        sq[3][t] = from_double<UP>(raw[3][p], ET);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sq[q][t] = from_double<UP>(raw[q][p], E[q]);
       }
     }
   }
   __syncthreads();
-  const int E = smax[0], ET = smax[1];
+  const int EU = smax[0], EV = smax[1], EW = smax[2], ET = smax[3], E = max(EU, max(EV, EW));
   const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
   if (i >= g.n1m || j >= g.n2m) return;
   const StepParams& p = *pp;
-  // exponents of a sum of products, of a Laplacian (kept at a quarter), of a sum
-  const int XP = 2 * E - 1025, XT = E + ET - 1025;
+  // products with u, v, w come to the exponent of those with the largest of them
+  const int su = min(E - EU, 63), sv = min(E - EV, 63), sw = min(E - EW, 63);
+  const bool shifted = (su | sv | sw) != 0;              // of the whole block
   {
     const int kz = threadIdx.z, k = k0 + kz;
     if (k >= g.n3m) return;
@@ -640,22 +646,29 @@ explicit_int_kernel(StencilArgs A, const StepParams* __restrict__ pp, RuSet ru, 
     const long long* v = sq[1] + c;
     const long long* w = sq[2] + c;
     const long long* T = sq[3] + c;
-    // the three differences of an advection term times their factors
+    // the three differences of an advection term (their products with u, v and
+    // w) of a component with exponent X times their factors
     auto adv = [&](long long x, long long y, long long z, double f1, double f2, double f3, int X) {
-      if constexpr (SP == 0) return -(f1 * to_double(x + y + z, X));
-      else if constexpr (SP == 1) return -(f1 * to_double(x + y, X) + f3 * to_double(z, X));
-      else return -(f1 * to_double(x, X) + f2 * to_double(y, X) + f3 * to_double(z, X));
+      if (SP < 2 && shifted) {
+        x >>= su;
+        y >>= sv;
+        if (SP == 0) z >>= sw;
+      }
+      constexpr int S = 2 * UP + 1011;                     // two scales 2^(1075 + UP), less the 64 bits of mul_high
+      if constexpr (SP == 0) return -(f1 * to_double(x + y + z, X + E - S));
+      else if constexpr (SP == 1)
+        return -(f1 * to_double(x + y, X + E - S) + f3 * to_double(z, X + EW - S));
+      else return -(f1 * to_double(x, X + EU - S) + f2 * to_double(y, X + EV - S) + f3 * to_double(z, X + EW - S));
     };
     auto lap = [&](const long long* s, double L1, double L2, double L3, int e) {
-      if constexpr (SP == 0) {
-        const long long sum = (s[sx] + s[-sx]) + (s[sy] + s[-sy]) + (s[sz] + s[-sz]);
-        return L1 * to_double((sum >> 2) - (s[0] + (s[0] >> 1)), e - UP + 2);
+      const long long x = s[sx] + s[-sx], y = s[sy] + s[-sy], z = s[sz] + s[-sz];      // below 2^62
+      if constexpr (SP == 0) {                             // at a quarter
+        return L1 * to_double(((x + y) >> 2) + (z >> 2) - (s[0] + (s[0] >> 1)), e - UP + 2);
       } else if constexpr (SP == 1) {
-        const long long xy = ((s[sx] + s[-sx]) >> 1) + ((s[sy] + s[-sy]) >> 1) - 2 * s[0];
-        return L1 * to_double(xy, e - UP + 1) + L3 * to_double(s[sz] + s[-sz] - 2 * s[0], e - UP);
+        return L1 * to_double((x >> 1) + (y >> 1) - 2 * s[0], e - UP + 1) + L3 * to_double(z - 2 * s[0], e - UP);
       } else {
-        return L1 * to_double(s[sx] + s[-sx] - 2 * s[0], e - UP) + L2 * to_double(s[sy] + s[-sy] - 2 * s[0], e - UP) +
-               L3 * to_double(s[sz] + s[-sz] - 2 * s[0], e - UP);
+        return L1 * to_double(x - 2 * s[0], e - UP) + L2 * to_double(y - 2 * s[0], e - UP) +
+               L3 * to_double(z - 2 * s[0], e - UP);
       }
     };
     const double q1 = p.cd[kQ1], q2 = p.cd[kQ2], q3 = p.cd[kQ3];
@@ -675,29 +688,29 @@ explicit_int_kernel(StencilArgs A, const StepParams* __restrict__ pp, RuSet ru, 
       const long long x = square_high(u[sx] + u[0]) - square_high(u[0] + u[-sx]);
       const long long y = mul_high(v[sy] + v[sy - sx], u[sy] + u[0]) - E0;
       const long long z = mul_high(w[sz] + w[sz - sx], u[sz] + u[0]) - F0;
-      double h = adv(x, y, z, q1, q2, q3, XP);
+      double h = adv(x, y, z, q1, q2, q3, EU);
       if (A.forcing) h = add_forcing<double>(h, A.vofx, A.forcx, c0, p.cd[kRXLEN]);
-      store(0, h, lap(u, l1, l2, l3, E) - p.cd[kPD1] * (pc - A.pr[c0 + dim]));
+      store(0, h, lap(u, l1, l2, l3, EU) - p.cd[kPD1] * (pc - A.pr[c0 + dim]));
     }
     {
       const long long x = mul_high(v[sx] + v[0], u[sx] + u[sx - sy]) - E0;
       const long long y = square_high(v[sy] + v[0]) - square_high(v[0] + v[-sy]);
       const long long z = mul_high(w[sz] + w[sz - sy], v[sz] + v[0]) - H0;
-      double h = adv(x, y, z, q1, q2, q3, XP);
+      double h = adv(x, y, z, q1, q2, q3, EV);
       if (A.forcing) h = add_forcing<double>(h, A.vofy, A.forcy, c0, p.cd[kRYLEN]);
-      store(1, h, lap(v, l1, l2, l3, E) - p.cd[kPD2] * (pc - A.pr[c0 + djm]));
+      store(1, h, lap(v, l1, l2, l3, EV) - p.cd[kPD2] * (pc - A.pr[c0 + djm]));
     }
     {
       const long long x = mul_high(w[sx] + w[0], u[sx] + u[sx - sz]) - F0;
       const long long y = mul_high(w[sy] + w[0], v[sy] + v[sy - sz]) - H0;
       const long long z = square_high(w[sz] + w[0]) - square_high(w[0] + w[-sz]);
-      double h = adv(x, y, z, q1, q2, q3, XP);
+      double h = adv(x, y, z, q1, q2, q3, EW);
       if (p.betagz != 0.0) {
         const double T_interp = (A.temp[c0] + A.temp[c0 + dkm]) * 0.5;
         h = h + p.cd[kBETAGZ] * (T_interp - p.cd[kTLIQ]);
       }
       if (A.forcing) h = add_forcing<double>(h, A.vofz, A.forcz, c0, p.cd[kRZLEN]);
-      store(2, h, lap(w, l1, l2, l3, E) - p.cd[kPD3] * (pc - A.pr[c0 + dkm]));
+      store(2, h, lap(w, l1, l2, l3, EW) - p.cd[kPD3] * (pc - A.pr[c0 + dkm]));
     }
     if (ET == 0x7ff) {
       rhs4[3 * g.cells + c0] = ru.r[3][c0] = quiet_nan();
@@ -708,7 +721,7 @@ explicit_int_kernel(StencilArgs A, const StepParams* __restrict__ pp, RuSet ru, 
       const long long x = mul_high(u[sx], T[sx] + T[0]) - mul_high(u[0], T[0] + T[-sx]);
       const long long y = mul_high(v[sy], T[sy] + T[0]) - mul_high(v[0], T[0] + T[-sy]);
       const long long z = mul_high(w[sz], T[sz] + T[0]) - mul_high(w[0], T[0] + T[-sz]);
-      ht = adv(x, y, z, p.cd[kH1], p.cd[kH2], p.cd[kH3], XT);
+      ht = adv(x, y, z, p.cd[kH1], p.cd[kH2], p.cd[kH3], ET);
     } else {
       ht = h_t<double>(A, i, j, k, c0, dip, dim, djp, djm, dkp, dkm, p);
     }
