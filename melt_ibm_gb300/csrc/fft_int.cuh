@@ -19,15 +19,18 @@
 // last place kept.  The unit at the end is n 2^-61 of the line's largest
 // input, against outputs of about sqrt(n) times its rms: below 2^-55 of them
 // for inputs up to 16 times their rms, less than the rounding of the result.
+// One line against extended precision, before that rounding, relative 2-norm (FP64
+// stages): noise 1e-17 .. 6e-17 (2e-16); a spike, the worst input for one
+// scale per line, 5e-17 at 128, 1.4e-16 at 192, 2.2e-16 at 512 (6e-17 .. 1.2e-16).
 // The whole solve against one in extended precision, relative 2-norm of phi /
 // of its gradient, with the z lines of fft_int_z.cu (the FP64 passes): 32^3 noise
 // 2.9e-16 / 3.4e-16 (1.1e-15 / 7.8e-16), 64^3 noise 2.5e-16 / 4.4e-16 (3.4e-15 /
 // 1.2e-15), one spike 2.3e-16 / 4.1e-16 (3.7e-15 / 1.2e-15), values over nine
 // decades 2.7e-16 / 4.4e-16 (4.1e-15 / 1.2e-15).  A line that holds an infinity
 // or a NaN comes out as NaN.
-// Per pass, FP64 -> integer: 128^3 x forward 61 -> 34, y 60 -> 21, x inverse 60
-// -> 29 us; 192^3 212 -> 92, 192 -> 63, 208 -> 81 us; 108 x 108 x 72 (no
-// compile-time FP64 instance) 45 -> 19, 47 -> 16, 44 -> 19 us.
+// Per pass, FP64 -> integer: 128^3 x forward 61 -> 20, y 60 -> 20, x inverse 60
+// -> 20 us; 192^3 212 -> 58, 192 -> 57, 208 -> 56 us; 108 x 108 x 72 (no
+// compile-time FP64 instance) 45 -> 15, 47 -> 15, 44 -> 15 us.
 #pragma once
 
 #include "fft_common.cuh"

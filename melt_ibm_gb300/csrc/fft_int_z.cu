@@ -14,13 +14,22 @@
 // the end values of the K chunks before it (weights rho^{mM} / (1 - rho^n),
 // 2^-60 dropped), and adds the entry's decay to its cells.  Per line the host
 // gives the bits that a sweep may grow values by: they start as far up as the
-// first sweep allows and are shifted down, rounded, before the second.
+// first sweep allows.  Before the second they are shifted down, rounded, from
+// what the first has made of them: a line that oscillates in z has not grown and is
+// left where it is.
 // The zero line (lambda = 0, mean set to 0) is two running sums, exact in
 // 128-bit integers, in a block of its own beside the others.
-// Error: fft_int.cuh.  The table's wavenumbers are those of the half-angle formula,
-// which alone takes 64^3 noise from 5.1e-15 to 2.5e-16 (phi, relative 2-norm).
-// Per solve, FP64 -> this: 48^3 25 -> 9.3 us,
-// 96^3 39 -> 14.4, 128^3 49 -> 24, 192^3 145 -> 56, 108 x 108 x 72 63 -> 14.
+// Error (see also fft_int.cuh; phi, relative 2-norm, 8 x 8 lines of 16 to 512 cells
+// times cos x, FP64 lines / these): noise, a spike or the lowest mode in z 1e-15 ..
+// 1e-12 / 1e-16 .. 4e-16; modes from n/8 up, alone, on the average 0.2 to 0.6
+// of the FP64 lines' in cubic and taller boxes (256 cells, n/2 - 1: 6e-14 / 7e-15),
+// up to 5 times them in boxes 0.4 as tall as wide, where 1/e is 100 and more.
+// The alternating mode and n/4 by themselves come out of the FP64 lines to a few
+// 1e-15 at some lengths (216, 288, 432), where all their roundings cancel; here to
+// 2e-14 (216) .. 1e-13 (288).  The table's wavenumbers are those of the half-angle
+// formula, which alone takes 64^3 noise from 5.1e-15 to 2.5e-16.
+// Per solve, FP64 -> this: 48^3 25 -> 8.8 us,
+// 96^3 39 -> 14.4, 128^3 49 -> 25, 192^3 145 -> 58, 108 x 108 x 72 63 -> 15.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -36,11 +45,11 @@ using namespace fixed;
 constexpr int kMaxChunks = 32, kMaxLine = 512;
 
 // a line's constants, times 2^62 as signed halves: rho, rho^M and 1/(1 -
-// rho^n) - 1; guard bits of the load (may be negative), halvings between the
-// sweeps, K; and the final factor
+// rho^n) - 1; guard bits of the load (may be negative), bits that a sweep may
+// grow values by, K; and the final factor
 struct alignas(16) ZLine {
   int rh, rl, mh, ml;
-  int wh, wl, up, down;
+  int wh, wl, up, grow;
   int K, pad;
   double scale;
 };
@@ -110,7 +119,7 @@ __device__ __noinline__ void zero_line(int n, size_t st, double2* __restrict__ s
 template <int M, int T>
 __global__ void __launch_bounds__(T, T <= 512 ? 2 : 1) z_lines(Grid g, const ZLine* __restrict__ tab, double2* __restrict__ spec) {
   __shared__ __align__(16) long long sC[kMaxChunks][32], sD[kMaxChunks][32];
-  __shared__ int sE[32];
+  __shared__ int sE[32], sB[32];
   static_assert(sizeof(sC) >= kMaxLine * sizeof(__int128), "the zero line's sums fit");
   const size_t st = 2 * (size_t)g.HP * g.n2m;
   if (blockIdx.x == 0) {
@@ -123,7 +132,10 @@ __global__ void __launch_bounds__(T, T <= 512 ? 2 : 1) z_lines(Grid g, const ZLi
   const int kx = act ? l % H : 1, ky = act ? l / H : 0;
   const ZLine Z = tab[kx + H * min(ky, g.n2m - ky)];
   double* __restrict__ rp = (double*)(spec + kx + (size_t)g.HP * ky) + (lane & 1) + (size_t)(w * M) * st;
-  if (w == 0) sE[lane] = 1;
+  if (w == 0) {
+    sE[lane] = 1;
+    sB[lane] = 0;
+  }
   long long r[M];
   int E = 1;
   {
@@ -157,18 +169,26 @@ __global__ void __launch_bounds__(T, T <= 512 ? 2 : 1) z_lines(Grid g, const ZLi
   sC[w][lane] = r[M - 1];
   __syncthreads();
   long long t = entry(sC, -1);
-  const long long half = (1ll << Z.down) >> 1;
+  int top = 0;
 #pragma unroll
   for (int i = 0; i < M; ++i) {
     t = frac(t, Z.rh, Z.rl);
-    r[i] = (r[i] + t + half) >> Z.down;
+    r[i] += t;
+    top |= (int)(r[i] >> 32) ^ (int)(r[i] >> 63);
   }
+  // down to where the second sweep's growth just fits
+  atomicMax(&sB[lane], 64 - __clz(top));
+  __syncthreads();
+  const int down = max(sB[lane] + Z.grow - 61, 0);
+  const long long half = (1ll << down) >> 1;
+#pragma unroll
+  for (int i = 0; i < M; ++i) r[i] = (r[i] + half) >> down;
 #pragma unroll
   for (int i = M - 2; i >= 0; --i) r[i] += frac(r[i + 1], Z.rh, Z.rl);
   sD[w][lane] = r[0];
   __syncthreads();
   t = entry(sD, 1);
-  const int X = E - Z.up + Z.down;
+  const int X = E - Z.up + down;
 #pragma unroll
   for (int i = M - 1; i >= 0; --i) {
     t = frac(t, Z.rh, Z.rl);
@@ -240,7 +260,7 @@ void intfft_z_table(const Grid& g, std::vector<char>& out) {
       // a sweep grows values by at most (1 + w) / e
       const int bits = (int)std::ceil(std::log2((1.0 + std::ldexp((double)w, -62)) / e) + 0.01);
       z.up = 8 - bits;                                      // below 2^61 after the first sweep
-      z.down = bits;                                        // and after the second
+      z.grow = bits;
       const double drop = 60.0 / (-std::log2(std::max(std::ldexp((double)rm, -62), 1e-300)));
       z.K = (int)std::min((double)(n / M), std::ceil(drop));
       z.scale = -nfac / lambda * e * e;
