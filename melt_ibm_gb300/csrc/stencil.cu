@@ -988,8 +988,9 @@ __global__ void divmax_kernel(StencilArgs A, unsigned long long* __restrict__ ou
   if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(v));
 }
 
-// p + phi - al beta lap(phi); ISO as updvp_prcalc_kernel: 3 FP64 operations
-// instead of 8 (192^3: 109 -> 68 us)
+// p + phi - al beta lap(phi); ISO: the six neighbours summed on the integer
+// pipe where that is at least as good as in FP64 (sum6_guarded; not next to
+// zeros of phi), 3 FP64 operations instead of 8 (192^3: 109 -> 87 us; 66 without the guard)
 template <bool ISO>
 __global__ void prcalc_kernel(StencilArgs A, const StepParams* __restrict__ pp, const double* __restrict__ dph,
                               double* __restrict__ pr) {
@@ -1000,8 +1001,8 @@ __global__ void prcalc_kernel(StencilArgs A, const StepParams* __restrict__ pp, 
   const double d = dph[c0];
   const double pip = dph[c0 + dip], pjp = dph[c0 + djp], pkp = dph[c0 + dkp];
   const double pim = dph[c0 + dim], pjm = dph[c0 + djm], pkm = dph[c0 + dkm];
-  double t;
-  if constexpr (ISO) t = pp->cd[kPB1] * sum6_f64(pip, pim, pjp, pjm, pkp, pkm);
+  double t, sum;
+  if (ISO && sum6_guarded(pip, pim, pjp, pjm, pkp, pkm, sum)) t = pp->cd[kPB1] * sum;
   else t = pp->cd[kPB1] * (pip + pim) + pp->cd[kPB2] * (pjp + pjm) + pp->cd[kPB3] * (pkp + pkm);
   pr[c0] = (pr[c0] + pp->cd[kPBC] * d) - t;
 }
