@@ -436,9 +436,9 @@ int  mibm_diagnostics_get_(double* out);
 /* It runs the same periodic tridiagonal solve as solxi_ in place on       */
 /* `rhs`, a device array in the compact layout x fastest with row pitch    */
 /* `pitch` (elements), n2m rows and n3m planes, on `stream` (NULL = the   */
-/* legacy default stream).  Lines of 2^a 3^b cells (even) with rows on     */
-/* 16-byte boundaries and -0.24 < betadx < 1e12 need no scratch.  That of  */
-/* the others, the line-factor table, is a                                 */
+/* legacy default stream).  Lines of an even number 2^a 3^b of cells, rows */
+/* on 16-byte boundaries and -0.24 < betadx < 1e12 need no scratch.  That  */
+/* of the others, the line-factor table, is a                             */
 /* file-scope device array sized for lines up to 512 cells (16.4 KB, held */
 /* by every GPU that loads the library until exit); n1m > 512 (or n3m >    */
 /* 65535) returns MIBM_EINVAL without launching.  The first call on a      */

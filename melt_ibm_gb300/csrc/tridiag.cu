@@ -586,10 +586,11 @@ int tri_chunk(Ctx* c, int dir) {
 // averaged: 192^3 24: 87 / 115, 16: 91 / 118, 32: 95 / 121; 256^3 32: 201 / 246,
 // 16: 202 / 262; 96^3 24: 17 / 21, 16: 18.4 / 22; within 5% at 48-64).
 // x: 16 (256^3 196, 32: 221; 128^3 35, 8: 42, 32: 44), but 8 or 6 where 16 leaves
-// fewer than 100 blocks for a field (48^3 10.8 against 12.9); odd ones last,
-// they load 8 bytes at a time.
+// fewer than 100 blocks for a field (48^3 10.8 against 12.9); odd ones late,
+// they load 8 bytes at a time; 18 for 486 cells, the one even 2^a 3^b length up to 512
+// without another.
 static int geo_chunk_line(int n, int lines) {
-  static const int pref[] = {16, 12, 8, 6, 4, 2, 3};
+  static const int pref[] = {16, 12, 8, 6, 4, 2, 3, 18};
   int found = 0;
   for (int m : pref) {
     if (n % m != 0 || n / m > 32) continue;
