@@ -3304,7 +3304,10 @@ const double* lagr_particle_fused(Ctx* c, const StepParams* dp, float* m32, Step
   const bool next_here = fork && next_prologue >= 0 && c->side3;     // the next substep's geometry work follows
   const bool tag_next = next_here && c->side2 && !c->I(MIBM_I_STATIONARY) && ensure_band(c);
   bool imelt = c->I(MIBM_I_IMELT) == 1;
-  if (imelt && !c->heat_pending) heat_flux_launch(c, true);
+  if (imelt && !c->heat_pending) {
+    if (!fork) lagr_find_probe_indices(c);   // no next substep's cage indices follow: the host finds the probes in pind
+    heat_flux_launch(c, true);
+  }
   // the temperature forcing (after the heat flux, which reads the unforced
   // temperature) and the reset of the narrow band need nothing of what
   // follows here: they go to the tagging's stream, off the chain to the next
