@@ -366,7 +366,6 @@ static uint64_t step_key(Ctx* c) {
   }
   mix((uint64_t)c->precision); mix((uint64_t)c->nproj); mix(c->lag_gen); mix(c->q32 ? 1 : 0);
   mix(c->tune_gen); mix(c->diag_on ? 1 : 0); mix(c->tri_geo ? 1 : 0);
-  mix(c->linear ? 1 : 0);
   return h;
 }
 
@@ -376,20 +375,22 @@ static bool graphs_allowed(Ctx* c) {
   return c->use_graph && c->steps_done >= 1 && !c->profiling && !lagr_remesh_active(c);
 }
 
-static void drop_graph(Ctx* c) {
-  if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
-  if (c->graph) cudaGraphDestroy(c->graph);
-  c->graph_exec = nullptr;
-  c->graph = nullptr;
+static void drop_graphs(Ctx* c) {
+  for (Ctx::StepGraph& s : c->graphs) {
+    if (s.exec) cudaGraphExecDestroy(s.exec);
+    if (s.graph) cudaGraphDestroy(s.graph);
+    s = Ctx::StepGraph{};
+  }
   c->graph_key = 0;
 }
 
-// Capture step_enqueue into a graph; false (and graphs off for this
+// Capture step_enqueue into the graph of the context's form (both graphs are
+// dropped when the key has changed); false (and graphs off for this
 // context) if the capture or the instantiation fails.  A linear step (a member
 // of a large batch) has its side streams stand for the main one, so that the
 // forks and joins vanish and the graph is one chain.
 static bool capture_step(Ctx* c, uint64_t key) {
-  drop_graph(c);
+  if (key != c->graph_key) drop_graphs(c);
   cudaStream_t* const sides[4] = {&c->side, &c->side2, &c->side3, &c->tsolve};
   cudaStream_t own[4];
   for (int q = 0; q < 4; ++q) {
@@ -430,11 +431,16 @@ static bool capture_step(Ctx* c, uint64_t key) {
     c->use_graph = false;
     return false;
   }
-  c->graph = gr;
-  c->graph_exec = ex;
+  c->step_graph() = Ctx::StepGraph{gr, ex, kernels};
   c->graph_key = key;
-  c->graph_kernels = kernels;
   return true;
+}
+
+// the context's step as a graph of its form: captured where there is none yet
+static bool have_graph(Ctx* c) {
+  if (!graphs_allowed(c)) return false;
+  const uint64_t key = step_key(c);
+  return (c->step_graph().exec && key == c->graph_key) || capture_step(c, key);
 }
 
 // tsch.f90:18-97 on the device.  From the second call on, the device part
@@ -444,14 +450,9 @@ static void tschem(Ctx* c) {
   if (!step_prepare(c)) return;
   step_head(c);
   if (c->status != MIBM_OK) return;
-  bool graph = graphs_allowed(c);
-  if (graph) {
-    uint64_t key = step_key(c);
-    if (!c->graph_exec || key != c->graph_key) graph = capture_step(c, key);
-  }
-  if (graph) {
-    if (!cuda_ok(c, cudaGraphLaunch(c->graph_exec, c->stream), "step graph")) return;
-    c->launches += c->graph_kernels;
+  if (have_graph(c)) {
+    if (!cuda_ok(c, cudaGraphLaunch(c->step_graph().exec, c->stream), "step graph")) return;
+    c->launches += c->step_graph().kernels;
   } else {
     step_enqueue(c);
   }
@@ -564,6 +565,25 @@ static void batch_drop_graph(Batch* b) {
   b->built_from.clear();
 }
 
+// Whether a case's step runs as one chain beside its batch's other members.
+// The device runs a process's streams (and a graph's branches) on eight
+// hardware queues; work that shares one waits in line.  A step graph has four
+// branches most of the time, so with members enough each case runs as one chain
+// and the cases alone overlap, unless it has so much of the batch's work that
+// its own chain would be what the others wait for.  Precision form: from five
+// members, up to half of the cells; FP64 form, whose branches also share the
+// FP64 pipe out better: from eight, up to an eighth.  ms per batch step, all
+// branching / all chains (/ chains but the largest), precision form: 3 x 48^3
+// 1.08 / 1.17, 4 x 1.30 / 1.30, 5 x 1.64 / 1.43, 8 x 2.44 / 1.77; 5 x 64^3 1.97 /
+// 1.79, 5 x 96^3 3.32 / 3.15, 5 x 128^3 5.73 / 5.57, 6 x 192^3 18.7 / 18.6; 4 x
+// 64^3 and 192^3 4.92 / 4.86 / 4.54, 8 x 64^3 and 192^3 6.25 / 5.97 / 5.55, 3 x 64^3
+// and 3 x 128^3 4.48 / 4.25 / 4.56.  FP64 form: 4 x 48^3 1.24 / 1.49, 5 x 1.50 /
+// 1.64, 8 x 2.19 / 2.02; 8 x 64^3 2.75 / 2.59, 5 x 96^3 4.17 / 4.44; 4 x 64^3, 3 x
+// 96^3 and 2 x 128^3 6.80 / 7.51 / 6.87; 8 x 64^3 and 192^3 12.6 / 13.4 / 12.6.
+static bool step_as_chain(const Ctx* c, size_t members, size_t cells) {
+  return c->precision == 1 ? members >= 5 && 2 * c->g.cells <= cells : members >= 8 && 8 * c->g.cells <= cells;
+}
+
 // One batch step.  A case that fails (non-finite field, allocation or CUDA
 // error in its own work) is left out of the rest of the step with its status
 // kept in its context; the other cases complete the step exactly as they
@@ -610,17 +630,11 @@ static int batch_step(Batch* b, int ntime) {
     }
   }
   drop_failed(cs);
-  // (B) forcing (gcurv.f90:164-170) and the host part of each step.  The device
-  // runs a process's streams (and a graph's branches) on eight hardware
-  // queues; work that shares one waits in line.  A step graph has four
-  // branches most of the time, so from kLinearCases members up each case runs
-  // as one chain and the cases alone overlap (us per case and step of n 48^3
-  // cases as chains / as branching graphs, precision form: n = 3 391 / 375, 4
-  // 334 / 343, 5 293 / 349, 8 226 / 318; FP64 form: 4 484 / 468, 5 424 / 453, 8
-  // 331 / 419).
-  constexpr size_t kLinearCases = 5;
+  // (B) forcing (gcurv.f90:164-170) and the host part of each step
+  size_t cells = 0;
+  for (Ctx* c : cs) cells += c->g.cells;
   for (Ctx* c : cs) {
-    c->linear = cs.size() >= kLinearCases;
+    c->linear = step_as_chain(c, cs.size(), cells);
     if (c->I(MIBM_I_FORCING) == 1) {
       int which = c->I(MIBM_I_WHICH_HIT);
       if (which == 1) k_hit_random_force(c);
@@ -635,24 +649,20 @@ static int batch_step(Batch* b, int ntime) {
   // (C) device work: step graphs (captured where missing or stale)
   bool all_graphs = b->launch == 0;
   for (Ctx* c : cs) {
-    bool graph = graphs_allowed(c);
-    if (graph) {
-      uint64_t key = step_key(c);
-      if (!c->graph_exec || key != c->graph_key) graph = capture_step(c, key);
-    }
+    const bool graph = have_graph(c);
     all_graphs = all_graphs && graph && c->status == MIBM_OK;
   }
   drop_failed(cs);
   if (cs.empty()) return first_bad;
   if (all_graphs) {
     std::vector<cudaGraphExec_t> now;
-    for (Ctx* c : cs) now.push_back(c->graph_exec);
+    for (Ctx* c : cs) now.push_back(c->step_graph().exec);
     if (!b->exec || now != b->built_from) {
       batch_drop_graph(b);
       bool ok = cudaGraphCreate(&b->graph, 0) == cudaSuccess;
       for (size_t q = 0; ok && q < cs.size(); ++q) {
         cudaGraphNode_t node;
-        ok = cudaGraphAddChildGraphNode(&node, b->graph, nullptr, 0, cs[q]->graph) == cudaSuccess;
+        ok = cudaGraphAddChildGraphNode(&node, b->graph, nullptr, 0, cs[q]->step_graph().graph) == cudaSuccess;
       }
       ok = ok && cudaGraphInstantiate(&b->exec, b->graph, cudaGraphInstantiateFlagUseNodePriority) == cudaSuccess;
       if (!ok) { cudaGetLastError(); batch_drop_graph(b); all_graphs = false; }
@@ -663,12 +673,13 @@ static int batch_step(Batch* b, int ntime) {
     for (Ctx* c : cs)   // forcing and buffer work enqueued on the case streams comes first
       if (!cuda_ok(c, cudaStreamSynchronize(c->stream), "batch")) return c->status;
     if (!cuda_ok(cs[0], cudaGraphLaunch(b->exec, b->stream), "batch graph")) return cs[0]->status;
-    for (Ctx* c : cs) c->launches += c->graph_kernels;
+    for (Ctx* c : cs) c->launches += c->step_graph().kernels;
     if (!cuda_ok(cs[0], cudaStreamSynchronize(b->stream), "batch graph")) return cs[0]->status;
   } else {
     for (Ctx* c : cs) {
-      if (c->graph_exec && graphs_allowed(c)) {
-        if (cuda_ok(c, cudaGraphLaunch(c->graph_exec, c->stream), "step graph")) c->launches += c->graph_kernels;
+      if (c->step_graph().exec && graphs_allowed(c)) {
+        if (cuda_ok(c, cudaGraphLaunch(c->step_graph().exec, c->stream), "step graph"))
+          c->launches += c->step_graph().kernels;
       } else {
         step_enqueue(c);
       }
@@ -1004,7 +1015,7 @@ int mibm_autotune_load_(const char* path) {
 void mibm_set_graphs_(const int* on) {
   Ctx* c = current(); if (!ready(c)) return;
   c->use_graph = *on != 0;
-  if (!c->use_graph) drop_graph(c);
+  if (!c->use_graph) drop_graphs(c);
 }
 
 // The host's remesher (see include/mibm.h); fn = NULL removes it.

@@ -191,19 +191,25 @@ struct Ctx {
   float* q32 = nullptr;
   bool q32_valid = false;
   unsigned long long* divmax = nullptr;   // device max|div u| (IEEE bits)
-  // captured step graph (tschem_ from its second call): replayed while the
-  // key of everything a step reads by value from the host is unchanged
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t graph_exec = nullptr;
+  // captured step graphs (tschem_ from its second call): [0] with the side
+  // streams' branches, [1] one chain (a member of a large batch); replayed
+  // while the key of everything a step reads by value from the host is
+  // unchanged.  Both are kept: the form follows the batch's other members.
+  struct StepGraph {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    uint64_t kernels = 0;                 // kernel launches recorded in it
+  };
+  StepGraph graphs[2];
+  StepGraph& step_graph() { return graphs[linear ? 1 : 0]; }
   bool use_graph = true;
-  uint64_t graph_key = 0;
-  uint64_t graph_kernels = 0;             // kernel launches recorded in the graph
+  uint64_t graph_key = 0;                 // of both graphs
   uint64_t steps_done = 0;
   uint64_t lag_gen = 0;                   // bumped when the Lagrangian launch sequence changes
   bool profiling = false;                 // per-kernel event profiling on (no graphs then)
   // shapes chosen by the autotuner (tune.cu); -1 / 8 = the default rules
   int tune_m[3] = {-1, -1, -1};           // line-solve chunk length per direction
-  bool linear = false;                    // member of a large batch: the step graph is one chain
+  bool linear = false;                    // this step as one chain (step_as_chain)
   bool one_stream = false;                // capturing that chain: the side streams stand for the main one
   bool tri_geo = false;                   // FP64 step: every line solve takes the geo_* kernels (tridiag.cu)
   int tune_by = 2;                        // block height of the explicit-term kernels (32 x 2 threads: the

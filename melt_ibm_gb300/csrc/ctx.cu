@@ -319,8 +319,10 @@ void release(Ctx* c) {
   cudaSetDevice(c->device);
   unpin_host(c);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
-  if (c->graph) cudaGraphDestroy(c->graph);
+  for (Ctx::StepGraph& s : c->graphs) {
+    if (s.exec) cudaGraphExecDestroy(s.exec);
+    if (s.graph) cudaGraphDestroy(s.graph);
+  }
   for (int i = 0; i < MIBM_NFIELDS; ++i) cudaFree(c->df[i]);
   for (int i = 0; i < MIBM_NMESH; ++i) cudaFree(c->dm[i]);
   cudaFree(c->pad_vx); cudaFree(c->pad_vy); cudaFree(c->stage); cudaFree(c->spec); cudaFree(c->mesh_stage);
