@@ -586,10 +586,14 @@ __global__ void plan_check_kernel(int nf, const int* __restrict__ pind, const in
   if (diff) atomicOr(dirty, 1);
 }
 
-// key of entry e, or -1 for a ghost face
+// The kernels over entries take them slot by slot: thread p has the entry of
+// triangle p % nf, so that a warp's entries are those of neighbouring triangles at one
+// cage slot and many of them share a cell (plan_slot).
+// key and number of entry p, key -1 for a ghost face
 __device__ __forceinline__ int plan_key(const Grid& g, int nf, const int* __restrict__ pind,
-                                        const int* __restrict__ ghost, int e) {
-  const int per = 27 * nf, comp = e / per, r = e - comp * per, t = r / 27, sl = r - 27 * t;
+                                        const int* __restrict__ ghost, int p, int& e) {
+  const int q = p / nf, t = p - q * nf, comp = q / 27, sl = q - 27 * comp;
+  e = 27 * (comp * nf + t) + sl;
   if (ghost[t]) return -1;
   int i0, j0, k0;
   cage_center(comp, pind + 6 * t, i0, j0, k0);
@@ -600,10 +604,11 @@ __global__ void __launch_bounds__(256) plan_mark_kernel(Grid g, int nf, const in
                                                         const int* __restrict__ ghost, const int* __restrict__ dirty,
                                                         unsigned* __restrict__ bitmap) {
   if (!*dirty) return;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 108 * nf) return;
-  const int key = plan_key(g, nf, pind, ghost, e);
-  if (key < 0) return;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  int e, key = -1;
+  if (p < 108 * nf) key = plan_key(g, nf, pind, ghost, p, e);
+  const unsigned same = __match_any_sync(0xffffffffu, key);
+  if (key < 0 || (threadIdx.x & 31) != __ffs(same) - 1) return;
   const unsigned bit = 1u << (key & 31);
   if (!(bitmap[key >> 5] & bit)) atomicOr(bitmap + (key >> 5), bit);   // a stale 0 only repeats the atomic
 }
@@ -682,30 +687,39 @@ __global__ void __launch_bounds__(256) plan_runs_kernel(const unsigned* __restri
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
     nruns[0] = base + total;
     nruns[1] = 0;                        // the storage cursor
+    nruns[2] = 0;                        // long runs
   }
 }
 
-// a slot of its run for every entry
+// a slot of its run for every entry: one atomic for the entries of a warp that
+// share a run (a body of 20480 faces within a few cells has runs of as many entries: 240 -> SLOTFIG us)
 __global__ void __launch_bounds__(256) plan_slot_kernel(Grid g, int nf, const int* __restrict__ pind,
                                                         const int* __restrict__ ghost, const int* __restrict__ dirty,
                                                         const unsigned* __restrict__ bitmap,
                                                         const int* __restrict__ wpre, int* __restrict__ run_cnt,
                                                         int2* __restrict__ slot) {
   if (!*dirty) return;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 108 * nf) return;
-  const int key = plan_key(g, nf, pind, ghost, e);
-  int2 s = make_int2(-1, 0);
-  if (key >= 0) {
-    s.x = wpre[key >> 5] + __popc(bitmap[key >> 5] & ((1u << (key & 31)) - 1u));
-    s.y = atomicAdd(run_cnt + s.x, 1);
+  const unsigned FULL = 0xffffffffu;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  int e, run = -1;
+  if (p < 108 * nf) {
+    const int key = plan_key(g, nf, pind, ghost, p, e);
+    if (key >= 0) run = wpre[key >> 5] + __popc(bitmap[key >> 5] & ((1u << (key & 31)) - 1u));
   }
-  slot[e] = s;
+  const unsigned same = __match_any_sync(FULL, run);
+  const int first = __ffs(same) - 1;
+  int at = 0;
+  if (run >= 0 && lane == first) at = atomicAdd(run_cnt + run, __popc(same));
+  at = __shfl_sync(FULL, at, first) + __popc(same & ((1u << lane) - 1u));
+  if (p < 108 * nf) slot[p] = make_int2(run, at);
 }
 
-// storage for every run: a warp of runs takes its total from the cursor
+// storage for every run: a warp of runs takes its total from the cursor; runs
+// of more than kLongRun entries are listed
+constexpr int kLongRun = 128;
 __global__ void __launch_bounds__(256) plan_store_kernel(const int* __restrict__ dirty, const int* __restrict__ run_cnt,
-                                                         int* __restrict__ run_off, int* __restrict__ nruns) {
+                                                         int* __restrict__ run_off, int* __restrict__ nruns,
+                                                         int* __restrict__ long_run) {
   if (!*dirty) return;
   const unsigned FULL = 0xffffffffu;
   const int n = nruns[0], lane = threadIdx.x & 31;
@@ -720,6 +734,7 @@ __global__ void __launch_bounds__(256) plan_store_kernel(const int* __restrict__
     if (lane == 31) base = atomicAdd(nruns + 1, x);
     base = __shfl_sync(FULL, base, 31);
     if (h < n) run_off[h] = base + x - v;
+    if (h < n && v > kLongRun) long_run[atomicAdd(nruns + 2, 1)] = h;
   }
 }
 
@@ -729,13 +744,52 @@ __global__ void __launch_bounds__(256) plan_place_kernel(int nf, const int* __re
                                                          const int2* __restrict__ slot, const int* __restrict__ run_off,
                                                          int* __restrict__ entry, int* __restrict__ saved) {
   if (!*dirty) return;
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 108 * nf) return;
-  const int2 s = slot[e];
-  if (s.x >= 0) entry[run_off[s.x] + s.y] = e;
-  if (e < nf) {
-    for (int q = 0; q < 6; ++q) saved[7 * (size_t)e + q] = pind[6 * e + q];
-    saved[7 * (size_t)e + 6] = ghost[e];
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= 108 * nf) return;
+  const int2 s = slot[p];
+  const int q = p / nf, t = p - q * nf;                   // plan_key's order
+  if (s.x >= 0) entry[run_off[s.x] + s.y] = 27 * (q / 27 * nf + t) + q % 27;
+  if (p < nf) {
+    for (int d = 0; d < 6; ++d) saved[7 * (size_t)p + d] = pind[6 * p + d];
+    saved[7 * (size_t)p + 6] = ghost[p];
+  }
+}
+
+// A long run into triangle order, by a block: a triangle has one entry of a run
+// (its 27 cage cells differ), so a bitmap of the triangles, by tiles, gives every entry its
+// rank.  All threads of the block call.
+constexpr int kSortWords = 256;
+__device__ void plan_sort_long(int nf, int len, const int* __restrict__ entry, int* __restrict__ src) {
+  __shared__ unsigned bits[kSortWords];
+  __shared__ int before[kSortWords], wsum[8];
+  constexpr int kPer = kSortWords / 256, kTile = 32 * kSortWords;
+  const int t = threadIdx.x, per = 27 * nf, base = entry[0] / per * per;          // of the run's component
+  int done = 0;
+  for (int t0 = 0; t0 < nf; t0 += kTile) {
+    for (int w = t; w < kSortWords; w += 256) bits[w] = 0u;
+    __syncthreads();
+    for (int i = t; i < len; i += 256) {
+      const unsigned f = (unsigned)((entry[i] - base) / 27 - t0);
+      if (f < (unsigned)kTile) atomicOr(bits + f / 32, 1u << (f & 31));
+    }
+    __syncthreads();
+    int n = 0, total;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) n += __popc(bits[kPer * t + q]);
+    int at = block_scan(n, wsum, total) + done;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      before[kPer * t + q] = at;
+      at += __popc(bits[kPer * t + q]);
+    }
+    __syncthreads();
+    for (int i = t; i < len; i += 256) {
+      const int e = entry[i];
+      const unsigned f = (unsigned)((e - base) / 27 - t0);
+      if (f < (unsigned)kTile) src[before[f / 32] + __popc(bits[f / 32] & ((1u << (f & 31)) - 1u))] = e;
+    }
+    done += total;
+    __syncthreads();
   }
 }
 
@@ -743,10 +797,13 @@ __global__ void __launch_bounds__(256) plan_place_kernel(int nf, const int* __re
 // entry is the number of smaller ones), and its word of the bitmap back to zero
 // for the next build.  A run has about ten entries, so half of a whole warp would idle:
 // 20480 faces 58 -> 50 us (32 runs loaded at once by a warp: 118, too few warps).
-__global__ void __launch_bounds__(256) plan_order_kernel(const int* __restrict__ dirty, const int* __restrict__ nruns,
+// Ranks cost the square of the length: the long runs of a fine mesh on a coarse grid, or
+// of a body that has melted to a few cells, go to whole blocks (LONGFIG).
+__global__ void __launch_bounds__(256) plan_order_kernel(int nf, const int* __restrict__ dirty, const int* __restrict__ nruns,
                                                          const int* __restrict__ run_key,
                                                          const int* __restrict__ run_off,
                                                          const int* __restrict__ run_cnt,
+                                                         const int* __restrict__ long_run,
                                                          const int* __restrict__ entry, int* __restrict__ src,
                                                          unsigned* __restrict__ bitmap) {
   if (!*dirty) return;
@@ -757,7 +814,7 @@ __global__ void __launch_bounds__(256) plan_order_kernel(const int* __restrict__
   for (int h0 = (blockIdx.x * 256 + (threadIdx.x & ~31)) / W; h0 < n; h0 += step) {
     const int h = h0 + ((threadIdx.x & 31) / W);
     const bool act = h < n;
-    const int o = act ? run_off[h] : 0, len = act ? run_cnt[h] : 0;
+    const int o = act ? run_off[h] : 0, all = act ? run_cnt[h] : 0, len = all > kLongRun ? 0 : all;
     const int longest = max(len, __shfl_xor_sync(FULL, len, W));
     if (act && lane == 0) bitmap[run_key[h] >> 5] = 0u;
     for (int i0 = 0; i0 < longest; i0 += W) {
@@ -770,6 +827,10 @@ __global__ void __launch_bounds__(256) plan_order_kernel(const int* __restrict__
       }
       if (i0 + lane < len) src[o + rank] = v;
     }
+  }
+  for (int q = blockIdx.x; q < nruns[2]; q += gridDim.x) {
+    const int h = long_run[q], o = run_off[h];
+    plan_sort_long(nf, run_cnt[h], entry + o, src + o);
   }
 }
 
@@ -2405,7 +2466,8 @@ struct LagState {
   int plan_words = 0;
   int2* slot = nullptr;                          // per entry: its run and its slot in it
   int *run_key = nullptr, *run_cnt = nullptr, *run_off = nullptr;
-  int* nruns = nullptr;                          // [0] runs, [1] storage cursor
+  int* nruns = nullptr;                          // [0] runs, [1] storage cursor, [2] long runs
+  int* long_run = nullptr;                       // the long runs, in no order
   int *entry = nullptr, *src = nullptr;          // entries by run, then in triangle order
   int* saved = nullptr;                          // 7 ints per face: pind(1:6), ghost
   int* dirty = nullptr;
@@ -2512,7 +2574,8 @@ static bool ensure_lag_buffers(Ctx* c) {
               cuda_ok(c, cudaMalloc(&s->run_key, sizeof(int) * runs), "plan") &&
               cuda_ok(c, cudaMalloc(&s->run_cnt, sizeof(int) * runs), "plan") &&
               cuda_ok(c, cudaMalloc(&s->run_off, sizeof(int) * runs), "plan") &&
-              cuda_ok(c, cudaMalloc(&s->nruns, sizeof(int) * 2), "plan") &&
+              cuda_ok(c, cudaMalloc(&s->nruns, sizeof(int) * 3), "plan") &&
+              cuda_ok(c, cudaMalloc(&s->long_run, sizeof(int) * (n / kLongRun + 1)), "plan") &&
               cuda_ok(c, cudaMalloc(&s->entry, sizeof(int) * n), "plan") &&
               cuda_ok(c, cudaMalloc(&s->src, sizeof(int) * n), "plan") &&
               cuda_ok(c, cudaMalloc(&s->saved, sizeof(int) * 7 * (size_t)std::max(1, c->maxnf)), "plan") &&
@@ -2521,7 +2584,7 @@ static bool ensure_lag_buffers(Ctx* c) {
     if (!ok) return false;
     cudaMemsetAsync(s->bitmap, 0, sizeof(unsigned) * (size_t)s->plan_words, c->stream);
     cudaMemsetAsync(s->saved, 0xff, sizeof(int) * 7 * (size_t)std::max(1, c->maxnf), c->stream);
-    cudaMemsetAsync(s->nruns, 0, sizeof(int) * 2, c->stream);
+    cudaMemsetAsync(s->nruns, 0, sizeof(int) * 3, c->stream);
     cudaMemsetAsync(s->dirty, 0, sizeof(int), c->stream);
   }
   return true;
@@ -2579,12 +2642,13 @@ static void update_plan(Ctx* c, const StepParams* dp, bool checked) {
     plan_slot_kernel<<<eb, 256, 0, c->stream>>>(c->g, nf, pind, ghost, s->dirty, s->bitmap, s->wpre, s->run_cnt,
                                                 s->slot); }
   { MIBM_PROF(c, "plan_store");
-    plan_store_kernel<<<std::min<unsigned>(eb, 304), 256, 0, c->stream>>>(s->dirty, s->run_cnt, s->run_off, s->nruns); }
+    plan_store_kernel<<<std::min<unsigned>(eb, 304), 256, 0, c->stream>>>(s->dirty, s->run_cnt, s->run_off, s->nruns,
+                                                                              s->long_run); }
   { MIBM_PROF(c, "plan_place");
     plan_place_kernel<<<eb, 256, 0, c->stream>>>(nf, pind, ghost, s->dirty, s->slot, s->run_off, s->entry, s->saved); }
   { MIBM_PROF(c, "plan_order");
     plan_order_kernel<<<std::min<unsigned>(eb, kScatterBlocks), 256, 0, c->stream>>>(
-        s->dirty, s->nruns, s->run_key, s->run_off, s->run_cnt, s->entry, s->src, s->bitmap); }
+        nf, s->dirty, s->nruns, s->run_key, s->run_off, s->run_cnt, s->long_run, s->entry, s->src, s->bitmap); }
   cudaMemsetAsync(s->dirty, 0, sizeof(int), c->stream);
   c->launches += 7;
   MIBM_LAUNCH_CHECK(c, "scatter plan");
@@ -3450,7 +3514,7 @@ void lagr_free(Ctx* c) {
       cudaFree(s->band_ub); cudaFree(s->band_face); cudaFree(s->face_cell); cudaFree(s->cm32);
       cudaFree(s->band_list); cudaFree(s->band_count);
       cudaFree(s->bitmap); cudaFree(s->wpre); cudaFree(s->tsum); cudaFree(s->slot);
-      cudaFree(s->run_key); cudaFree(s->run_cnt); cudaFree(s->run_off); cudaFree(s->nruns);
+      cudaFree(s->run_key); cudaFree(s->run_cnt); cudaFree(s->run_off); cudaFree(s->nruns); cudaFree(s->long_run);
       cudaFree(s->entry); cudaFree(s->src);
       cudaFree(s->saved); cudaFree(s->dirty); cudaFree(s->segval);
       delete s;
