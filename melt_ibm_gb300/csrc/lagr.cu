@@ -561,14 +561,15 @@ __global__ void force_coef_kernel(Grid g, int nf, ForceArgs F, double tmelt, dou
 // (ghost faces have no entries).  A run is the entries of one key, in triangle
 // order; runs are numbered in key order.  The keys touched are marked in a
 // bitmap of 4*cells bits; a scan of its population counts numbers the runs in
-// key order; each entry then takes a slot of its run with one atomic, runs
-// take storage from a cursor, and a warp per run puts its few tens of entries
-// into triangle order by rank.  The slots and the storage depend on the order
+// key order; entries then take slots of their runs with atomics, runs take
+// storage from a cursor, and half a warp per run puts its few tens of entries
+// into triangle order by rank (a block where there are more).  The slots and the storage depend on the order
 // of the atomics, the finished runs do not.  Eight launches, each a few
 // microseconds: this chain is on the step's critical path at small and
 // moderate grids.  A radix sort of all entries by key in its place took 3 or 4
 // passes of five launches and five more for the run heads (serial kernel time
-// of the plan, 5120 faces on 128^3: 170 -> 95 us per substep).
+// of the plan, 5120 faces on 128^3: 170 -> 95 us per substep; 20480 faces, radius
+// 0.3 on 16^3 / 0.4 on 64^3: 166 -> 155 / 216 -> 114 us).
 // The plan depends only on the cage centres (pind) and the ghost flags;
 // `plan_check` compares them with the values the plan was built from and
 // every kernel of the rebuild returns at once when nothing changed, so a
@@ -692,7 +693,7 @@ __global__ void __launch_bounds__(256) plan_runs_kernel(const unsigned* __restri
 }
 
 // a slot of its run for every entry: one atomic for the entries of a warp that
-// share a run (a body of 20480 faces within a few cells has runs of as many entries: 240 -> SLOTFIG us)
+// share a run (a body of 20480 faces within a few cells has runs of as many entries: 240 -> 35 us)
 __global__ void __launch_bounds__(256) plan_slot_kernel(Grid g, int nf, const int* __restrict__ pind,
                                                         const int* __restrict__ ghost, const int* __restrict__ dirty,
                                                         const unsigned* __restrict__ bitmap,
@@ -757,7 +758,8 @@ __global__ void __launch_bounds__(256) plan_place_kernel(int nf, const int* __re
 
 // A long run into triangle order, by a block: a triangle has one entry of a run
 // (its 27 cage cells differ), so a bitmap of the triangles, by tiles, gives every entry its
-// rank.  All threads of the block call.
+// rank.  All threads of the block call.  Tiles of 8192 triangles: with 32768 the
+// kernel's 8 KB of shared memory cost the 48^3 step 1%.
 constexpr int kSortWords = 256;
 __device__ void plan_sort_long(int nf, int len, const int* __restrict__ entry, int* __restrict__ src) {
   __shared__ unsigned bits[kSortWords];
@@ -798,7 +800,8 @@ __device__ void plan_sort_long(int nf, int len, const int* __restrict__ entry, i
 // for the next build.  A run has about ten entries, so half of a whole warp would idle:
 // 20480 faces 58 -> 50 us (32 runs loaded at once by a warp: 118, too few warps).
 // Ranks cost the square of the length: the long runs of a fine mesh on a coarse grid, or
-// of a body that has melted to a few cells, go to whole blocks (LONGFIG).
+// of a body that has melted to a few cells, go to whole blocks (20480 faces, radius 0.3 on
+// 16^3: 271 ms -> 51 us, 0.4 on 64^3 1003 -> 35 us, 0.5 on 128^3 94 -> 78 us).
 __global__ void __launch_bounds__(256) plan_order_kernel(int nf, const int* __restrict__ dirty, const int* __restrict__ nruns,
                                                          const int* __restrict__ run_key,
                                                          const int* __restrict__ run_off,
