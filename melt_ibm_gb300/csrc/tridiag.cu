@@ -616,12 +616,16 @@ static int geo_chunk(Ctx* c, int dir) {
 
 // Whether the FP64 step of context c keeps the Thomas sweep's order of
 // operations.  The literal MLS of a body that melts without moving turns a
-// last-bit difference of a vertex coordinate into about 1e-8 of the heat flux
-// on fine grids (the condition number of its moment matrix grows as (n/L)^2),
-// and the front integrates it: after 9 steps from identical inputs another
-// order of the line solves alone moves the pressure at single cells by 1e-9
-// (96^3), 6e-9 (144^3), 1e-8 (192^3) and 1.5e-7 (256^3) of its rms.  Fine grids
-// therefore keep it, so that their runs reproduce those of earlier builds.
+// last-bit difference of a vertex coordinate into 1e-9 to 1e-7 of the heat flux
+// (the condition number of its moment matrix grows as the square of the
+// body's position in cells, whatever the box's length: one unit in the last place of
+// the probes' centroids moves a tenth of the fluxes by more than 3e-9 at 48^3, 1.2e-8 at 96^3,
+// 3.4e-8 at 144^3 and 4.5e-8 at 192^3, the same to 10% in boxes of 1, 2 pi, 20 and
+// 100 length units), and the front integrates it: after 9 steps from identical
+// inputs another order of the line solves alone moves the pressure at single cells
+// by 1e-9 (96^3), 6e-9 (144^3), 1e-8 (192^3) and 1.5e-7 (256^3) of its rms.  There
+// is no step in that: the line is drawn below 1e-8, between 144 and 192 cells.  Finer
+// grids keep the order, so that their runs reproduce those of earlier builds.
 constexpr int kOrderCells = 160;
 bool tri_keep_order(Ctx* c) {
   return c->I(MIBM_I_IMLSFOR) == 1 && c->I(MIBM_I_IMELT) == 1 && c->I(MIBM_I_IMLSSTR) != 1 && c->maxnf > 0 &&
