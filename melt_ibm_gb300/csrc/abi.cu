@@ -9,6 +9,7 @@
 //   * the four RHS fields are separate buffers, so all explicit terms are
 //     formed from the substep's initial fields exactly as tsch.f90:49-57
 //     orders them (every invtr only advances its own component).
+#include <atomic>
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
@@ -431,7 +432,8 @@ static bool capture_step(Ctx* c, uint64_t key) {
     c->use_graph = false;
     return false;
   }
-  c->step_graph() = Ctx::StepGraph{gr, ex, kernels};
+  static std::atomic<uint64_t> captures{0};
+  c->step_graph() = Ctx::StepGraph{gr, ex, kernels, ++captures};
   c->graph_key = key;
   return true;
 }
@@ -545,7 +547,7 @@ struct Batch {
   cudaStream_t stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  std::vector<cudaGraphExec_t> built_from;   // the case graphs the batch graph holds
+  std::vector<uint64_t> built_from;          // the case graphs the batch graph holds, by serial
 };
 static std::mutex g_batch_mu;
 static std::map<int, Batch*> g_batch;
@@ -655,8 +657,8 @@ static int batch_step(Batch* b, int ntime) {
   drop_failed(cs);
   if (cs.empty()) return first_bad;
   if (all_graphs) {
-    std::vector<cudaGraphExec_t> now;
-    for (Ctx* c : cs) now.push_back(c->step_graph().exec);
+    std::vector<uint64_t> now;
+    for (Ctx* c : cs) now.push_back(c->step_graph().serial);
     if (!b->exec || now != b->built_from) {
       batch_drop_graph(b);
       bool ok = cudaGraphCreate(&b->graph, 0) == cudaSuccess;

@@ -199,6 +199,7 @@ struct Ctx {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     uint64_t kernels = 0;                 // kernel launches recorded in it
+    uint64_t serial = 0;                  // of the capture: handles come back after a graph is dropped
   };
   StepGraph graphs[2];
   StepGraph& step_graph() { return graphs[linear ? 1 : 0]; }
